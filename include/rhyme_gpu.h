@@ -393,7 +393,9 @@ int rhyme_gpu_rate_probe(int kind, int iters, double* ops_per_second, double* ms
  * Instrumentation (no reference counterpart): checks the integer forms of
  * the FP64 <-> FP32 conversions of the mixed state update against the
  * hardware conversions on n pseudo-random values from `seed` (doubles of
- * every exponent, FP32 rounding ties and range limits, FP32 values).
+ * every exponent, FP32 rounding ties and range limits, FP32 values), and
+ * the integer forms of the FP64 division, square root and comparisons of
+ * the FP64 kernels against the hardware operations on as many operands.
  * *mismatches: the number that differ (0 expected).
  */
 int rhyme_gpu_check_conversions(long long n, unsigned long long seed, unsigned long long* mismatches);

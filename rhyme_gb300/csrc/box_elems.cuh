@@ -200,7 +200,7 @@ __device__ __forceinline__ void flux_elem(const Gas<double>& G, const Rp<double>
     l[c] = ur[(long long)c * F + o];
     r[c] = ul[(long long)c * F + o + sa];
   }
-  interface_flux<D, AX, double, true>(G, rp, l, r, f);
+  interface_flux<D, AX>(G, rp, l, r, f);
 #pragma unroll
   for (int c = 0; c < D + 2; ++c) fr[(long long)c * F + o] = f[c];
 }
@@ -262,7 +262,8 @@ __device__ __forceinline__ double signal_speed_elem(const Gas<double>& G, const 
   double ss = 0.0;
 #pragma unroll
   for (int a = 0; a < D; ++a) ss = ss + u[1 + a] * u[1 + a];
-  const double v = sqrt(ss) / u[0] + sound_speed<D>(G, u);
+  const Inv<double> i0 = m_inv(u[0]);
+  const double v = m_div(m_sqrt(ss), i0) + sound_speed<D>(G, u, i0);
   if (!(u[0] > 0.0) || !isfinite(v)) bad = 1;
   return v;
 }

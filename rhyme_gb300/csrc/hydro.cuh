@@ -18,6 +18,7 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "fp64_int.h"
 #include "libm_pow.h"
 
 namespace rgpu {
@@ -27,7 +28,7 @@ namespace rgpu {
 // pow that the compiled reference calls for every real `**`, so the FP64 path
 // returns the reference's bits even in flows that amplify a one-ulp
 // difference.
-__device__ __forceinline__ double m_sqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ double m_sqrt(double x) { return sqrt_rn(x); }
 __device__ __forceinline__ float m_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double m_pow(double x, double y) { return libm_pow::pow(x, y); }
 // Float powers as 2^(y log2 x) with CUDA's log2f and exp2f: the rounding of
@@ -47,6 +48,35 @@ __device__ __forceinline__ void m_pow2(float x, float y1, float y2, float& r1, f
 __device__ __forceinline__ double m_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float m_abs(float x) { return fabsf(x); }
 
+// Divisions, comparisons and powers of two: FP64 through the integer forms
+// of fp64_int.h (the same bits; a division or a comparison on the FP64 pipe
+// costs 550 or 64 cycles a warp), FP32 as written. Inv is a divisor used
+// several times.
+template <typename T> struct Inv;
+template <> struct Inv<float> { float b; };
+template <> struct Inv<double> { Divisor d; };
+__host__ __device__ __forceinline__ Inv<float> m_inv(float b) { return {b}; }
+__host__ __device__ __forceinline__ Inv<double> m_inv(double b) { return {divisor(b)}; }
+__device__ __forceinline__ float m_div(float a, const Inv<float>& i) { return a / i.b; }
+__device__ __forceinline__ double m_div(double a, const Inv<double>& i) { return div_by(a, i.d); }
+template <typename T> __device__ __forceinline__ T m_div(T a, T b) { return m_div(a, m_inv(b)); }
+// a / (2 b): the significand of 2 b is that of b
+__device__ __forceinline__ double div_half(double a, const Inv<double>& i) {
+  Divisor d = i.d;
+  d.b = f64_scale<1>(d.b);
+  return div_by(a, d);
+}
+__device__ __forceinline__ bool m_gt(float a, float b) { return a > b; }
+__device__ __forceinline__ bool m_gt(double a, double b) { return f64_gt(a, b); }
+__device__ __forceinline__ bool m_neg(float a) { return a < 0.f; }
+__device__ __forceinline__ bool m_neg(double a) { return f64_negative(a); }
+__device__ __forceinline__ float m_half(float a) { return 0.5f * a; }
+__device__ __forceinline__ double m_half(double a) { return f64_scale<-1>(a); }
+__device__ __forceinline__ float m_twice(float a) { return 2.f * a; }
+__device__ __forceinline__ double m_twice(double a) { return f64_scale<1>(a); }
+__device__ __forceinline__ bool m_tiny(float a) { return fabsf(a) < FLT_MIN; }
+__device__ __forceinline__ bool m_tiny(double a) { return f64_tiny(a); }
+
 template <typename T> struct Limits;
 template <> struct Limits<double> {
   __device__ static constexpr double tiny() { return DBL_MIN; }
@@ -56,8 +86,8 @@ template <> struct Limits<float> {
 };
 
 // Fortran MAX/MIN of two reals (same ternary as the CPU oracle).
-template <typename T> __device__ __forceinline__ T fmax_ref(T a, T b) { return (b > a) ? b : a; }
-template <typename T> __device__ __forceinline__ T fmin_ref(T a, T b) { return (b < a) ? b : a; }
+template <typename T> __device__ __forceinline__ T fmax_ref(T a, T b) { return m_gt(b, a) ? b : a; }
+template <typename T> __device__ __forceinline__ T fmin_ref(T a, T b) { return m_gt(a, b) ? b : a; }
 
 // Ideal-gas constants (rhyme_riemann_problem_init.f90:20-27,
 // rhyme_irs_init.f90:21-27) plus the literal quotients the reference
@@ -66,6 +96,7 @@ template <typename T>
 struct Gas {
   T g, gm1, gp1, gm1_gp1, gm1_2g, gp1_2g, g_inv, kb_amu;
   T two_gp1, two_gm1, inv_gm1_2g, gm1_half, half_gm1, g_kb_amu;
+  Inv<T> by_gm1, by_gp1, by_kb_amu;  // divisors
 };
 
 // Run parameters used inside kernels.
@@ -83,19 +114,19 @@ struct Limiter {
 
 // ---- EOS: rhyme_hydro_base / rhyme_ideal_gas ------------------------------
 
-// rhyme_hydro_base_specific_kinetic_energy.f90:9
+// rhyme_hydro_base_specific_kinetic_energy.f90:9; i0: the density as a divisor
 template <int D, typename T>
 __device__ __forceinline__ T sp_kin_e(const T* u) {
   T s = T(0);
 #pragma unroll
   for (int a = 0; a < D; ++a) s = s + u[1 + a] * u[1 + a];
-  return (T(0.5) * s) / (u[0] * u[0]);
+  return m_div(m_half(s), u[0] * u[0]);
 }
 
 // rhyme_hydro_base_specific_internal_energy.f90:9
 template <int D, typename T>
-__device__ __forceinline__ T sp_int_e(const T* u) {
-  return u[D + 1] / u[0] - sp_kin_e<D>(u);
+__device__ __forceinline__ T sp_int_e(const T* u, const Inv<T>& i0) {
+  return m_div(u[D + 1], i0) - sp_kin_e<D>(u);
 }
 
 // The FP32 forms of the mixed sweeps (pressure, sound speed, flux) are the
@@ -108,28 +139,36 @@ __device__ __forceinline__ T sp_int_e(const T* u) {
 
 // rhyme_ideal_gas_pressure.f90:9
 template <int D, typename T>
-__device__ __forceinline__ T pressure(const Gas<T>& G, const T* u) {
+__device__ __forceinline__ T pressure(const Gas<T>& G, const T* u, const Inv<T>& i0) {
   if constexpr (sizeof(T) == sizeof(float)) {
     T s = T(0);
 #pragma unroll
     for (int a = 0; a < D; ++a) s = s + u[1 + a] * u[1 + a];
     return (u[D + 1] - T(0.5) * s / u[0]) * G.gm1;
   }
-  return u[0] * sp_int_e<D>(u) * G.gm1;
+  return u[0] * sp_int_e<D>(u, i0) * G.gm1;
+}
+template <int D, typename T>
+__device__ __forceinline__ T pressure(const Gas<T>& G, const T* u) {
+  return pressure<D>(G, u, m_inv(u[0]));
 }
 
 // rhyme_ideal_gas_temperature_per_mu.f90:9-10, _speed_of_sound.f90:9
 template <int D, typename T>
-__device__ __forceinline__ T sound_speed(const Gas<T>& G, const T* u) {
+__device__ __forceinline__ T sound_speed(const Gas<T>& G, const T* u, const Inv<T>& i0) {
   if constexpr (sizeof(T) == sizeof(float)) return m_sqrt(G.g * pressure<D>(G, u) / u[0]);
-  T t_mu = sp_int_e<D>(u) * G.gm1 / G.kb_amu;
+  T t_mu = m_div(sp_int_e<D>(u, i0) * G.gm1, G.by_kb_amu);
   return m_sqrt(G.g_kb_amu * t_mu);
+}
+template <int D, typename T>
+__device__ __forceinline__ T sound_speed(const Gas<T>& G, const T* u) {
+  return sound_speed<D>(G, u, m_inv(u[0]));
 }
 
 // rhyme_ideal_gas_flux.f90:12-23 along axis AX
 template <int D, int AX, typename T>
 __device__ __forceinline__ void flux(const Gas<T>& G, const T* u, T* f) {
-  if (m_abs(u[0]) < Limits<T>::tiny()) {
+  if (m_tiny(u[0])) {
 #pragma unroll
     for (int c = 0; c < D + 2; ++c) f[c] = T(0);
     return;
@@ -148,12 +187,13 @@ __device__ __forceinline__ void flux(const Gas<T>& G, const T* u, T* f) {
     f[D + 1] = vn * (u[D + 1] + p);
     return;
   }
-  T p = pressure<D>(G, u);
+  const Inv<T> i0 = m_inv(u[0]);
+  T p = pressure<D>(G, u, i0);
   f[0] = u[1 + AX];
 #pragma unroll
-  for (int a = 0; a < D; ++a) f[1 + a] = u[1 + a] * f[0] / u[0];
+  for (int a = 0; a < D; ++a) f[1 + a] = m_div(u[1 + a] * f[0], i0);
   f[1 + AX] = f[1 + AX] + p;
-  f[D + 1] = f[0] / u[0] * (u[D + 1] + p);
+  f[D + 1] = m_div(f[0], i0) * (u[D + 1] + p);
 }
 
 // rhyme_ideal_gas_primitive_vars_to_conserved.f90:9-11
@@ -166,7 +206,7 @@ __device__ __forceinline__ void prim_vars_to_cons(const Gas<T>& G, T rho, const 
     u[1 + a] = rho * v[a];
     s = s + v[a] * v[a];
   }
-  u[D + 1] = T(0.5) * rho * s + p / G.gm1;
+  u[D + 1] = m_half(rho) * s + m_div(p, G.by_gm1);
 }
 
 // ---- slope limiter: rhyme_slope_limiter*.f90 -------------------------------
@@ -177,10 +217,49 @@ __device__ __forceinline__ T xi_r(T w, T r) {
   return T(2) / (T(1) - w + (T(1) + w) * r);
 }
 
+// The FP64 limiter: the operations of limited_slope below, through the
+// integer forms. With w = 0 (the default) they reduce, with the same
+// results, to fewer: 0.5 d_L + 0.5 d_R is half of the rounded sum, xi_r is
+// 2/(1+r), and of two quotients with the same divisor the smaller one is
+// known from the numerators (rounding is monotonic), so van Leer, minmod
+// and superbee need one division after r.
+__device__ __forceinline__ double limited_slope_f64(int type, double w, double ul, double u, double ur) {
+  const double d_L = u - ul, d_R = ur - u;
+  const double r = f64_tiny(d_R) ? 0.0 : div_rn(d_L, d_R);
+  if (!f64_above(r, 0.0)) return 0.0;
+  double d;
+  if (w == 0.0) {
+    d = d_L + d_R;
+    // half the sum, exactly, well above the subnormal range
+    d = ((f64_hi(d) & 0x7fffffffu) - 0x08000000u < 0x7fe00000u - 0x08000000u) ? f64_scale<-1>(d) : 0.5 * d_L + 0.5 * d_R;
+    const bool big = f64_above(r, 1.0);
+    if (f64_hi(r) < 0x7ff00000u) {
+      if (type == 1) return div_rn(big ? 2.0 : f64_scale<1>(r), 1.0 + r) * d;
+      if (type == 2) return (big ? div_rn(2.0, 1.0 + r) : r) * d;
+      if (type == 4) {
+        if (big) return div_rn(2.0, 1.0 + r) * d;
+        return f64_above(r, 0.5) ? d : f64_scale<1>(r) * d;
+      }
+      const double xi = div_rn(2.0, 1.0 + r);
+      return fmin_ref(div_rn(r * (1.0 + r), 1.0 + r * r), xi) * d;
+    }
+  } else {
+    const double h = 0.5 * (1.0 + w);
+    d = h * d_L + h * d_R;
+  }
+  const double xi = div_rn(2.0, 1.0 - w + (1.0 + w) * r);
+  if (type == 1) return fmin_ref(div_rn(f64_scale<1>(r), 1.0 + r), xi) * d;
+  if (type == 2) return (f64_above(r, 1.0) ? fmin_ref(1.0, xi) : r) * d;
+  if (type == 3) return fmin_ref(div_rn(r * (1.0 + r), 1.0 + r * r), xi) * d;
+  if (f64_above(r, 1.0)) return fmin_ref(fmin_ref(r, xi), 2.0) * d;
+  return f64_above(r, 0.5) ? d : f64_scale<1>(r) * d;
+}
+
 // r (rhyme_slope_limiter.f90:62-82) and delta of the four limiters
 // (van Leer :13-27, minmod :13-29, van Albada :13-27, superbee :13-31).
 template <typename T>
 __device__ __forceinline__ T limited_slope(int type, T w, T ul, T u, T ur) {
+  if constexpr (sizeof(T) == sizeof(double)) return limited_slope_f64(type, w, ul, u, ur);
   T d_L = u - ul;
   T d_R = ur - u;
   T d = T(0.5) * (T(1) + w) * d_L + T(0.5) * (T(1) + w) * d_R;
@@ -217,8 +296,8 @@ __device__ __forceinline__ void half_step(const Gas<T>& G, const T* u, const T* 
   T fl[D + 2], fr[D + 2];
 #pragma unroll
   for (int c = 0; c < D + 2; ++c) {
-    l[c] = u[c] - T(0.5) * delta[c];
-    r[c] = u[c] + T(0.5) * delta[c];
+    l[c] = u[c] - m_half(delta[c]);
+    r[c] = u[c] + m_half(delta[c]);
   }
   flux<D, AX>(G, l, fl);
   flux<D, AX>(G, r, fr);
@@ -240,114 +319,112 @@ __device__ __forceinline__ void face_states(const Gas<T>& G, int lim, T w, const
   half_step<D, AX>(G, u0, delta, hdtdx, l, r);
 }
 
-// ---- exact Riemann solver: rhyme_irs_*, rhyme_riemann_problem_* -----------
+// ---- exact Riemann solver (FP64): rhyme_irs_*, rhyme_riemann_problem_* -----
+//
+// Every operation is the reference's, in its order; what is arranged for the
+// GPU is which lanes of a warp run together. Left and right states differ in
+// signs and roles only, so where one lane needs a wave of its left side and
+// another lane the same kind of wave of its right side, both run it in one
+// pass on the side each has picked (a selection of registers is a few
+// integer instructions, a pass of the rarefaction's two powers 57 FP64
+// ones). Divisors used more than once (a side's density, pressure and sound
+// speed) are kept with their reciprocal (Inv).
 
-// Loop-invariant terms of rhyme_irs_nonlinear_wave_function.f90:15-23 for one
-// side (Ak, Bk, 2cs/gm1, 1/(rho cs)): the reference recomputes them every
-// Newton iteration with the same operations, so computing them once gives the
-// same values. With LAZY (double only) the pair a branch needs is formed on
-// its first use (a side usually stays a shock or a rarefaction through the
-// iteration, and FP64 divisions are scarce on GB300): the plain FP64 flux
-// kernels take it (2-D slab 117 -> 126 M cell-updates/s); the FP64 fix-up of
-// the mixed form does not (its kernel would spill, and the mixed batch and
-// the server's latency suffered); float forms all four up front.
-template <typename T>
+// One side's loop-invariant terms of
+// rhyme_irs_nonlinear_wave_function.f90:15-23 (Ak, Bk, 2cs/gm1, 1/(rho cs)):
+// the reference recomputes them every Newton iteration with the same
+// operations, so computing them once gives the same values.
 struct WaveSide {
-  T rho, p, cs, Ak, Bk, c2g, irc;
-  bool shock_ready, fan_ready;
+  double p, Ak, Bk, c2g, irc;
+  Inv<double> ip;
 };
 
-template <typename T>
-__device__ __forceinline__ void wave_shock_terms(const Gas<T>& G, WaveSide<T>& w) {
-  w.Ak = T(2) / (G.gp1 * w.rho);
-  w.Bk = G.gm1 * w.p / G.gp1;
-  w.shock_ready = true;
-}
-
-template <typename T>
-__device__ __forceinline__ void wave_fan_terms(const Gas<T>& G, WaveSide<T>& w) {
-  w.c2g = T(2) * w.cs / G.gm1;
-  w.irc = T(1) / (w.rho * w.cs);
-  w.fan_ready = true;
-}
-
-template <typename T, bool LAZY>
-__device__ __forceinline__ WaveSide<T> wave_side(const Gas<T>& G, T s_rho, T s_p, T s_cs) {
-  WaveSide<T> w;
-  w.rho = s_rho;
+__device__ __forceinline__ WaveSide wave_side(const Gas<double>& G, double s_rho, double s_p, double s_cs) {
+  WaveSide w;
   w.p = s_p;
-  w.cs = s_cs;
-  w.shock_ready = w.fan_ready = false;
-  if constexpr (!LAZY) {
-    wave_shock_terms(G, w);
-    wave_fan_terms(G, w);
-  }
+  w.ip = m_inv(s_p);
+  w.Ak = m_div(2.0, G.gp1 * s_rho);
+  w.Bk = m_div(G.gm1 * s_p, G.by_gp1);
+  w.c2g = m_div(m_twice(s_cs), G.by_gm1);
+  w.irc = m_div(1.0, s_rho * s_cs);
   return w;
 }
 
-// rhyme_irs_nonlinear_wave_function.f90:13-24
-template <typename T, bool LAZY>
-__device__ __forceinline__ void nonlinear_wave(const Gas<T>& G, WaveSide<T>& w, T p, T& f, T& fprime) {
-  if (p > w.p) {
-    if constexpr (LAZY) {
-      if (!w.shock_ready) wave_shock_terms(G, w);
+// rhyme_irs_nonlinear_wave_function.f90:13-24 of both sides at p.
+__device__ __forceinline__ void nonlinear_waves(const Gas<double>& G, const WaveSide& L, const WaveSide& R, double p,
+                                                double& l_f, double& l_fp, double& r_f, double& r_fp) {
+  const bool l_shock = m_gt(p, L.p), r_shock = m_gt(p, R.p);
+  // rarefactions, then shocks: first the left side of a lane if it is of the
+  // kind, else the right one; then the right side where both are
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool l = pass == 0 && !l_shock;
+    if (l || (!r_shock && (pass == 0 || !l_shock))) {
+      double y, z;
+      const Inv<double> ip = l ? L.ip : R.ip;
+      m_pow2(m_div(p, ip), G.gm1_2g, -G.gp1_2g, y, z);
+      const double f = (l ? L.c2g : R.c2g) * (y - 1.0);
+      const double fp = (l ? L.irc : R.irc) * z;
+      l_f = l ? f : l_f;
+      l_fp = l ? fp : l_fp;
+      r_f = l ? r_f : f;
+      r_fp = l ? r_fp : fp;
     }
-    const T bp = w.Bk + p;
-    const T factor = m_sqrt(w.Ak / bp);
-    f = (p - w.p) * factor;
-    fprime = factor * (T(1) - (p - w.p) / (T(2) * bp));
-  } else if constexpr (sizeof(T) == sizeof(float)) {
-    // (p/p_k)^e - 1 as expm1(e log1p((p - p_k)/p_k)): the same quantity
-    // without the cancellation of the literal form when p is close to p_k
-    // (a float power near 1 carries an ulp of 1, a large relative error of
-    // the difference); p - p_k is exact there.
-    const float t = log1pf((p - w.p) / w.p);
-    f = w.c2g * expm1f(G.gm1_2g * t);
-    fprime = w.irc * expf(-G.gp1_2g * t);
-  } else {
-    if constexpr (LAZY) {
-      if (!w.fan_ready) wave_fan_terms(G, w);
+  }
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool l = pass == 0 && l_shock;
+    if (l || (r_shock && (pass == 0 || l_shock))) {
+      const double pk = l ? L.p : R.p;
+      const double bp = (l ? L.Bk : R.Bk) + p;
+      const Inv<double> ibp = m_inv(bp);
+      const double dp = p - pk;
+      const double factor = m_sqrt(m_div(l ? L.Ak : R.Ak, ibp));
+      const double f = dp * factor;
+      // (p - pk)/(2 bp): half of the quotient by bp
+      const double fp = factor * (1.0 - div_half(dp, ibp));
+      l_f = l ? f : l_f;
+      l_fp = l ? fp : l_fp;
+      r_f = l ? r_f : f;
+      r_fp = l ? r_fp : fp;
     }
-    T y, z;
-    m_pow2(p / w.p, G.gm1_2g, -G.gp1_2g, y, z);
-    f = w.c2g * (y - T(1));
-    fprime = w.irc * z;
   }
 }
 
 // Guess 0 of rhyme_irs_guess_p_star.f90:14-38 (the adaptive PVRS /
 // two-rarefaction / two-shock choice), not yet floored.
-template <typename T>
-__device__ __forceinline__ T guess_p_star_adaptive(const Gas<T>& G, T l_rho, T vl, T l_p, T l_cs, T r_rho, T vr,
-                                                   T r_p, T r_cs) {
-  T p;
-  const T q_user = T(2);
-  T cup = T(0.25) * (l_rho + r_rho) * (l_cs + r_cs);
-  T ppv = fmax_ref(T(0.5) * (l_p + r_p) + T(0.5) * (vl - vr) * cup, T(0));
-  T p_min = fmin_ref(l_p, r_p);
-  T p_max = fmax_ref(l_p, r_p);
-  T q_max = p_max / p_min;
-  if (q_max <= q_user && (p_min < ppv && ppv < p_max)) {
-    p = ppv;  // PVRS
-  } else if (ppv < p_min) {  // two-rarefaction
-    T pq = m_pow(l_p / r_p, G.gm1_2g);
-    T um = (pq * vl / l_cs + vr / r_cs + G.two_gm1 * (pq - T(1))) / (pq / l_cs + T(1) / r_cs);
-    T ptl = T(1) + G.half_gm1 * (vl - um) / l_cs;
-    T ptr = T(1) + G.half_gm1 * (um - vr) / r_cs;
-    p = T(0.5) * (l_p * m_pow(ptl, G.inv_gm1_2g) + r_p * m_pow(ptr, G.inv_gm1_2g));
-  } else {  // two-shock
-    T gel = m_sqrt((G.two_gp1 / l_rho) / (G.gm1_gp1 * l_p + ppv));
-    T ger = m_sqrt((G.two_gp1 / r_rho) / (G.gm1_gp1 * r_p + ppv));
-    p = (gel * l_p + ger * r_p - (vr - vl)) / (gel + ger);
+__device__ __forceinline__ double guess_p_star_adaptive(const Gas<double>& G, double l_rho, double vl, double l_p,
+                                                        double l_cs, double r_rho, double vr, double r_p,
+                                                        double r_cs) {
+  const double cup = 0.25 * (l_rho + r_rho) * (l_cs + r_cs);
+  const double ppv = fmax_ref(0.5 * (l_p + r_p) + 0.5 * (vl - vr) * cup, 0.0);
+  const double p_min = fmin_ref(l_p, r_p);
+  const double p_max = fmax_ref(l_p, r_p);
+  // q_max = p_max/p_min <= q_user = 2: for normal numbers the quotient
+  // rounds to at most 2 exactly where p_max <= 2 p_min
+  const bool near2 = (!m_tiny(p_min) && f64_hi(p_min) < 0x7fe00000u && f64_hi(p_max) < 0x7ff00000u)
+                         ? !m_gt(p_max, m_twice(p_min))
+                         : p_max / p_min <= 2.0;
+  if (near2 && (m_gt(ppv, p_min) && m_gt(p_max, ppv))) return ppv;  // PVRS
+  if (m_gt(p_min, ppv)) {                                          // two-rarefaction
+    const Inv<double> icl = m_inv(l_cs), icr = m_inv(r_cs);
+    const double pq = m_pow(m_div(l_p, r_p), G.gm1_2g);
+    const double um = m_div(m_div(pq * vl, icl) + m_div(vr, icr) + G.two_gm1 * (pq - 1.0),
+                            m_div(pq, icl) + m_div(1.0, icr));
+    const double ptl = 1.0 + m_div(G.half_gm1 * (vl - um), icl);
+    const double ptr = 1.0 + m_div(G.half_gm1 * (um - vr), icr);
+    return 0.5 * (l_p * m_pow(ptl, G.inv_gm1_2g) + r_p * m_pow(ptr, G.inv_gm1_2g));
   }
-  return p;
+  // two-shock
+  const double gel = m_sqrt(m_div(m_div(G.two_gp1, l_rho), G.gm1_gp1 * l_p + ppv));
+  const double ger = m_sqrt(m_div(m_div(G.two_gp1, r_rho), G.gm1_gp1 * r_p + ppv));
+  return m_div(gel * l_p + ger * r_p - (vr - vl), gel + ger);
 }
 
 // Guess number k (0..5) of rhyme_irs_guess_p_star.f90:14-71, floored at tiny.
-template <typename T>
-__device__ __noinline__ T guess_p_star(const Gas<T>& G, int k, T l_rho, T vl, T l_p, T l_cs, T r_rho,
-                                       T vr, T r_p, T r_cs) {
-  T p;
+static __device__ __noinline__ double guess_p_star(const Gas<double>& G, int k, double l_rho, double vl, double l_p,
+                                            double l_cs, double r_rho, double vr, double r_p, double r_cs) {
+  double p;
   if (k == 0) {
     p = guess_p_star_adaptive(G, l_rho, vl, l_p, l_cs, r_rho, vr, r_p, r_cs);
   } else if (k == 1) {  // Ramses
@@ -358,235 +435,152 @@ __device__ __noinline__ T guess_p_star(const Gas<T>& G, int k, T l_rho, T vl, T 
                   (m_pow(l_cs / l_p, G.gm1_2g) + m_pow(r_cs / r_p, G.gm1_2g)),
               G.inv_gm1_2g);
   } else if (k == 3) {  // two-shock approximation; g_K at :74-80
-    T l_g = m_sqrt((T(2) / (G.gp1 * l_rho)) / (l_p + G.gm1_gp1 * l_p));
-    T r_g = m_sqrt((T(2) / (G.gp1 * r_rho)) / (r_p + G.gm1_gp1 * r_p));
+    double l_g = m_sqrt((2.0 / (G.gp1 * l_rho)) / (l_p + G.gm1_gp1 * l_p));
+    double r_g = m_sqrt((2.0 / (G.gp1 * r_rho)) / (r_p + G.gm1_gp1 * r_p));
     p = (l_g * l_p + r_g * r_p - (vr - vl)) / (l_g + r_g);
   } else if (k == 4) {  // p_PV
-    p = T(0.5) * (l_p + r_p) - T(0.125) * (vr - vl) * (l_rho + r_rho) * (l_cs + r_cs);
+    p = 0.5 * (l_p + r_p) - 0.125 * (vr - vl) * (l_rho + r_rho) * (l_cs + r_cs);
   } else {  // arithmetic mean
-    p = T(0.5) * (l_p + r_p);
+    p = 0.5 * (l_p + r_p);
   }
-  return fmax_ref(p, Limits<T>::tiny());
+  return fmax_ref(p, Limits<double>::tiny());
 }
 
 // rhyme_irs_exec.f90:19-44 with lazily evaluated guesses. l_f / r_f are the
 // wave functions at the last iterate before the final update.
-template <typename T, bool LAZY>
-__device__ __forceinline__ T irs_exec(const Gas<T>& G, T tol, int n_iter, T l_rho, T vl, T l_p, T l_cs,
-                                      T& l_f, T r_rho, T vr, T r_p, T r_cs, T& r_f) {
-  T p_star = T(0), p_prev, l_fp, r_fp;
-  WaveSide<T> WL = wave_side<T, LAZY>(G, l_rho, l_p, l_cs);
-  WaveSide<T> WR = wave_side<T, LAZY>(G, r_rho, r_p, r_cs);
+__device__ __forceinline__ double irs_exec(const Gas<double>& G, double tol, int n_iter, const WaveSide& WL,
+                                           const WaveSide& WR, double l_rho, double vl, double l_cs, double& l_f,
+                                           double r_rho, double vr, double r_cs, double& r_f) {
+  double p_star = 0.0, p_prev, l_fp, r_fp;
+  const double du = vr - vl;
   for (int gid = 0; gid < 6; ++gid) {
-    p_star = guess_p_star(G, gid, l_rho, vl, l_p, l_cs, r_rho, vr, r_p, r_cs);
+    p_star = guess_p_star(G, gid, l_rho, vl, WL.p, l_cs, r_rho, vr, WR.p, r_cs);
     p_prev = p_star;
     for (int i = 1; i <= n_iter; ++i) {
-      nonlinear_wave<T, LAZY>(G, WL, p_star, l_f, l_fp);
-      nonlinear_wave<T, LAZY>(G, WR, p_star, r_f, r_fp);
-      p_star = p_prev - (l_f + r_f + (vr - vl)) / (l_fp + r_fp);
-      if (p_star < T(0)) break;
-      if (T(2) * m_abs(p_star - p_prev) / (p_star + p_prev) < tol) break;
+      nonlinear_waves(G, WL, WR, p_star, l_f, l_fp, r_f, r_fp);
+      p_star = p_prev - m_div(l_f + r_f + du, l_fp + r_fp);
+      if (m_neg(p_star)) break;
+      if (m_gt(tol, m_div(m_twice(m_abs(p_star - p_prev)), p_star + p_prev))) break;
       p_prev = p_star;
     }
-    if (p_star > T(0)) break;
+    if (f64_above(p_star, 0.0)) break;
   }
-  if (p_star < T(0)) p_star = T(0);
+  if (m_neg(p_star)) p_star = 0.0;
   return p_star;
 }
 
-// rp_side_t (rhyme_riemann_problem.f90:53-56)
-template <int D, typename T>
+// rp_side_t (rhyme_riemann_problem.f90:53-56), with the pressure as a divisor
+template <int D>
 struct Side {
-  T rho, v[D], p, cs;
+  double rho, v[D], p, cs;
+  Inv<double> ip;
 };
-
-// Sampled star-region summary (rhyme_riemann_problem.f90:33-51).
-template <typename T>
-struct Star {
-  T u, p;
-  bool l_shock, r_shock;
-  T l_rho, l_speed, l_cs, l_speedH, l_speedT;  // speed = shock speed
-  T r_rho, r_speed, r_cs, r_speedH, r_speedT;
-  T l_f, r_f;
-};
-
-// rhyme_riemann_problem_star.f90:12-65, split so that only the side the
-// sampling reads is formed: p* and u* (:12-38), then the left (:40, 43-53)
-// or the right (:41, 55-65) star state, each with the reference's
-// operations.
-template <int D, int AX, typename T, bool LAZY>
-__device__ __forceinline__ void rp_star_pu(const Gas<T>& G, const Rp<T>& rp, const Side<D, T>& L,
-                                           const Side<D, T>& R, Star<T>& s) {
-  s.p = irs_exec<T, LAZY>(G, rp.tol, rp.n_iter, L.rho, L.v[AX], L.p, L.cs, s.l_f, R.rho, R.v[AX], R.p, R.cs,
-                          s.r_f);
-  if (s.p < rp.vac_p) s.p = rp.vac_p;
-  s.u = T(0.5) * ((R.v[AX] + L.v[AX]) + (s.r_f - s.l_f));
-}
-
-template <int D, int AX, typename T>
-__device__ __forceinline__ void rp_star_left(const Gas<T>& G, const Side<D, T>& L, Star<T>& s) {
-  T ps_pl = s.p / L.p;
-  if (s.p > L.p) {
-    s.l_shock = true;
-    s.l_rho = L.rho * (G.gm1_gp1 + ps_pl) / (G.gm1_gp1 * ps_pl + T(1));
-    s.l_speed = L.v[AX] - L.cs * m_sqrt(G.gp1_2g * ps_pl + G.gm1_2g);
-  } else {
-    s.l_shock = false;
-    T pg, pa;
-    m_pow2(ps_pl, G.g_inv, G.gm1_2g, pg, pa);
-    s.l_rho = L.rho * pg;
-    s.l_cs = L.cs * pa;
-    s.l_speedH = L.v[AX] - L.cs;
-    s.l_speedT = s.u - s.l_cs;
-  }
-}
-
-template <int D, int AX, typename T>
-__device__ __forceinline__ void rp_star_right(const Gas<T>& G, const Side<D, T>& R, Star<T>& s) {
-  T ps_pr = s.p / R.p;
-  if (s.p > R.p) {
-    s.r_shock = true;
-    s.r_rho = R.rho * (G.gm1_gp1 + ps_pr) / (G.gm1_gp1 * ps_pr + T(1));
-    s.r_speed = R.v[AX] + R.cs * m_sqrt(G.gp1_2g * ps_pr + G.gm1_2g);
-  } else {
-    s.r_shock = false;
-    T pg, pa;
-    m_pow2(ps_pr, G.g_inv, G.gm1_2g, pg, pa);
-    s.r_rho = R.rho * pg;
-    s.r_cs = R.cs * pa;
-    s.r_speedH = R.v[AX] + R.cs;
-    s.r_speedT = s.u + s.r_cs;
-  }
-}
 
 // rhyme_riemann_problem_w_kfan.f90:14-31
-template <int D, int AX, typename T>
-__device__ __forceinline__ void w_kfan_body(const Gas<T>& G, const Side<D, T>& s, T dxdt, bool is_right, T* u) {
-  T cs = is_right ? -s.cs : s.cs;
-  const T base = G.two_gp1 + G.gm1_gp1 / cs * (s.v[AX] - dxdt);
-  T prho, pp;
+template <int D, int AX>
+__device__ __noinline__ void w_kfan(const Gas<double>& G, const Side<D>& s, double dxdt, bool is_right, double* u) {
+  double cs = is_right ? -s.cs : s.cs;
+  const double base = G.two_gp1 + m_div(G.gm1_gp1, cs) * (s.v[AX] - dxdt);
+  double prho, pp;
   m_pow2(base, G.two_gm1, G.inv_gm1_2g, prho, pp);
-  T rho = s.rho * prho;
-  T v[D];
+  double rho = s.rho * prho;
+  double v[D];
 #pragma unroll
   for (int a = 0; a < D; ++a) v[a] = s.v[a];
   v[AX] = G.two_gp1 * (cs + G.half_gm1 * s.v[AX] + dxdt);
-  T p = s.p * pp;
+  double p = s.p * pp;
   prim_vars_to_cons<D>(G, rho, v, p, u);
 }
 
-template <int D, int AX, typename T>
-__device__ __noinline__ void w_kfan_call(const Gas<T>& G, const Side<D, T>& s, T dxdt, bool is_right, T* u) {
-  w_kfan_body<D, AX>(G, s, dxdt, is_right, u);
-}
-
-// The double form is a call (its powers are long and rarely sampled); the
-// float form is inlined: a call would keep the caller's state vector in
-// local memory (its address escapes), a load and store per component on
-// every interface of the FP32 sweeps.
-template <int D, int AX, typename T>
-__device__ __forceinline__ void w_kfan(const Gas<T>& G, const Side<D, T>& s, T dxdt, bool is_right, T* u) {
-  if constexpr (sizeof(T) == sizeof(float)) w_kfan_body<D, AX>(G, s, dxdt, is_right, u);
-  else w_kfan_call<D, AX>(G, s, dxdt, is_right, u);
-}
-
-// rhyme_riemann_problem_w_star{L,R}_{sho,fan}.f90:12-15
-template <int D, int AX, typename T>
-__device__ __forceinline__ void w_star(const Gas<T>& G, const Side<D, T>& side, const Star<T>& s, T rho,
-                                       T* u) {
-  T v[D];
-#pragma unroll
-  for (int a = 0; a < D; ++a) v[a] = side.v[a];
-  v[AX] = s.u;
-  prim_vars_to_cons<D>(G, rho, v, s.p, u);
-}
-
-// rhyme_riemann_problem_sampling.f90:13-47 at x/t = dxdt
-// (the reference forms both sides' star states, and both sides' velocities
-// across AX, first; only the side read here gets them, from its conserved
-// state q, which leaves every value read unchanged)
-template <int D, int AX, typename T>
-__device__ __forceinline__ void side_transverse(Side<D, T>& S, const T* q) {
-#pragma unroll
-  for (int a = 0; a < D; ++a)
-    if (a != AX) S.v[a] = q[1 + a] / q[0];
-}
-
-template <int D, int AX, typename T>
-__device__ __forceinline__ void rp_sampling(const Gas<T>& G, Side<D, T>& L, Side<D, T>& R, const T* l,
-                                            const T* r, Star<T>& s, T dxdt, T* u) {
-  if (dxdt > s.u) {
-    side_transverse<D, AX>(R, r);
-    rp_star_right<D, AX>(G, R, s);
-    if (s.r_shock) {
-      if (dxdt < s.r_speed) w_star<D, AX>(G, R, s, s.r_rho, u);
-      else prim_vars_to_cons<D>(G, R.rho, R.v, R.p, u);
-    } else {
-      if (dxdt < s.r_speedT) w_star<D, AX>(G, R, s, s.r_rho, u);
-      else if (dxdt < s.r_speedH) w_kfan<D, AX>(G, R, dxdt, true, u);
-      else prim_vars_to_cons<D>(G, R.rho, R.v, R.p, u);
-    }
+// rhyme_riemann_problem_star.f90:40-65 and rhyme_riemann_problem_sampling.f90:
+// 13-47 at x/t = dxdt, for the side S of the contact that holds it (u, p: the
+// star region's). The right side is the left one with the signs of its
+// sound speed turned and its comparisons swapped: negation is exact, so the
+// sums round alike. (The reference forms both sides' star states first; only
+// the one read here is formed, with the reference's operations.)
+template <int D, int AX>
+__device__ __forceinline__ void rp_sample_side(const Gas<double>& G, const Side<D>& S, bool right, double us,
+                                               double ps, double dxdt, double* u) {
+  const double cs = right ? -S.cs : S.cs;
+  const double ps_pk = m_div(ps, S.ip);
+  double rho_star, inner;  // the star density and the speed that bounds the star region
+  const bool shock = m_gt(ps, S.p);
+  if (shock) {
+    rho_star = m_div(S.rho * (G.gm1_gp1 + ps_pk), G.gm1_gp1 * ps_pk + 1.0);
+    inner = S.v[AX] - cs * m_sqrt(G.gp1_2g * ps_pk + G.gm1_2g);
   } else {
-    side_transverse<D, AX>(L, l);
-    rp_star_left<D, AX>(G, L, s);
-    if (s.l_shock) {
-      if (dxdt > s.l_speed) w_star<D, AX>(G, L, s, s.l_rho, u);
-      else prim_vars_to_cons<D>(G, L.rho, L.v, L.p, u);
-    } else {
-      if (dxdt > s.l_speedT) w_star<D, AX>(G, L, s, s.l_rho, u);
-      else if (dxdt > s.l_speedH) w_kfan<D, AX>(G, L, dxdt, false, u);
-      else prim_vars_to_cons<D>(G, L.rho, L.v, L.p, u);
-    }
+    double pg, pa;
+    m_pow2(ps_pk, G.g_inv, G.gm1_2g, pg, pa);
+    rho_star = S.rho * pg;
+    inner = us - cs * pa;
+  }
+  const bool star = right ? dxdt < inner : dxdt > inner;
+  bool outside = shock;
+  if (!star && !shock) {
+    const double head = S.v[AX] - cs;
+    outside = !(right ? dxdt < head : dxdt > head);
+  }
+  if (star || outside) {
+    // rhyme_riemann_problem_w_star{L,R}_{sho,fan}.f90:12-15, or the side itself
+    double v[D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) v[a] = S.v[a];
+    v[AX] = star ? us : S.v[AX];
+    prim_vars_to_cons<D>(G, star ? rho_star : S.rho, v, star ? ps : S.p, u);
+  } else {
+    w_kfan<D, AX>(G, S, dxdt, right, u);
   }
 }
 
-// Vacuum state W_0: prim_to_cons of w_vacuum (rho, 0.., p).
-template <int D, typename T>
-__device__ __forceinline__ void vacuum_state(const Gas<T>& G, const Rp<T>& rp, T* u) {
-  T v[D];
+// The velocities across AX of the side that is sampled, from its conserved
+// state q.
+template <int D, int AX>
+__device__ __forceinline__ void side_transverse(Side<D>& S, const double* q, const Inv<double>& i0) {
 #pragma unroll
-  for (int a = 0; a < D; ++a) v[a] = T(0);
+  for (int a = 0; a < D; ++a)
+    if (a != AX) S.v[a] = m_div(q[1 + a], i0);
+}
+
+// Vacuum state W_0: prim_to_cons of w_vacuum (rho, 0.., p).
+template <int D>
+__device__ __forceinline__ void vacuum_state(const Gas<double>& G, const Rp<double>& rp, double* u) {
+  double v[D];
+#pragma unroll
+  for (int a = 0; a < D; ++a) v[a] = 0.0;
   prim_vars_to_cons<D>(G, rp.vac_rho, v, rp.vac_p, u);
 }
 
 // rhyme_riemann_problem_solve.f90:17-103 sampled at x/t = dxdt. (The mixed
 // sweeps' FP32 interfaces go through rp_flux_f32 instead, which sends the
-// interfaces this solver handles in its vacuum branches to the FP64 one.)
-template <int D, int AX, typename T, bool LAZY = false>
-__device__ __forceinline__ void rp_solve(const Gas<T>& G, const Rp<T>& rp, const T* l, const T* r,
-                                         T dxdt, T* u) {
-  Side<D, T> L, R;
+// interfaces this solver handles in its vacuum branches to this one.)
+template <int D, int AX>
+__device__ __forceinline__ void rp_solve(const Gas<double>& G, const Rp<double>& rp, const double* l,
+                                         const double* r, double dxdt, double* u) {
+  Side<D> L, R;
   L.rho = fmax_ref(l[0], rp.vac_rho);
   R.rho = fmax_ref(r[0], rp.vac_rho);
-  const T e_rho = rp.vac_rho_next;
-  const bool vacuum_right = R.rho < e_rho && L.rho > e_rho;
-  const bool vacuum_left = L.rho < e_rho && R.rho > e_rho;
-  const bool vacuum_both = L.rho < e_rho && R.rho < e_rho;
-  const T tiny = Limits<T>::tiny();
+  const double e_rho = rp.vac_rho_next;
+  const bool l_below = m_gt(e_rho, L.rho), r_below = m_gt(e_rho, R.rho);
+  const bool vacuum_right = r_below && L.rho > e_rho;
+  const bool vacuum_left = l_below && R.rho > e_rho;
+  const bool vacuum_both = l_below && r_below;
+  const double tiny = Limits<double>::tiny();
 
   if (vacuum_right) {
 #pragma unroll
     for (int a = 0; a < D; ++a) L.v[a] = l[1 + a] / l[0];
     L.p = fmax_ref(pressure<D>(G, l), rp.vac_p);
     L.cs = fmax_ref(sound_speed<D>(G, l), tiny);
-#pragma unroll
-    for (int a = 0; a < D; ++a) R.v[a] = T(0);
-    R.p = rp.vac_p;
-    R.cs = T(0);
-    T s_starl = L.v[AX] - T(2) * L.cs / G.gm1;
+    double s_starl = L.v[AX] - 2.0 * L.cs / G.gm1;
     if (dxdt > s_starl) vacuum_state<D>(G, rp, u);
     else if (dxdt > L.v[AX] - L.cs) w_kfan<D, AX>(G, L, dxdt, false, u);
     else prim_vars_to_cons<D>(G, L.rho, L.v, L.p, u);
   } else if (vacuum_left) {
 #pragma unroll
-    for (int a = 0; a < D; ++a) L.v[a] = T(0);
-    L.p = rp.vac_p;
-    L.cs = T(0);
-#pragma unroll
     for (int a = 0; a < D; ++a) R.v[a] = r[1 + a] / r[0];
     R.p = fmax_ref(pressure<D>(G, r), rp.vac_p);
     R.cs = fmax_ref(sound_speed<D>(G, r), tiny);
-    T s_starr = R.v[AX] + T(2) * R.cs / G.gm1;
+    double s_starr = R.v[AX] + 2.0 * R.cs / G.gm1;
     if (dxdt > R.v[AX] + R.cs) prim_vars_to_cons<D>(G, R.rho, R.v, R.p, u);
     else if (dxdt > s_starr) w_kfan<D, AX>(G, R, dxdt, true, u);
     else vacuum_state<D>(G, rp, u);
@@ -594,32 +588,49 @@ __device__ __forceinline__ void rp_solve(const Gas<T>& G, const Rp<T>& rp, const
     vacuum_state<D>(G, rp, u);
   } else {
     // velocities across AX: only for the side sampled (side_transverse)
-    L.v[AX] = l[1 + AX] / l[0];
-    L.p = fmax_ref(pressure<D>(G, l), rp.vac_p);
-    L.cs = fmax_ref(sound_speed<D>(G, l), tiny);
-    R.v[AX] = r[1 + AX] / r[0];
-    R.p = fmax_ref(pressure<D>(G, r), rp.vac_p);
-    R.cs = fmax_ref(sound_speed<D>(G, r), tiny);
-    T du = R.v[AX] - L.v[AX];
-    T du_crit = T(2) * (L.cs + R.cs) / G.gm1;
+    const Inv<double> il = m_inv(l[0]), ir = m_inv(r[0]);
+    L.v[AX] = m_div(l[1 + AX], il);
+    L.p = fmax_ref(pressure<D>(G, l, il), rp.vac_p);
+    L.cs = fmax_ref(sound_speed<D>(G, l, il), tiny);
+    R.v[AX] = m_div(r[1 + AX], ir);
+    R.p = fmax_ref(pressure<D>(G, r, ir), rp.vac_p);
+    R.cs = fmax_ref(sound_speed<D>(G, r, ir), tiny);
+    const double du = R.v[AX] - L.v[AX];
+    const double du_crit = m_div(m_twice(L.cs + R.cs), G.by_gm1);
     if (du_crit < du) {  // vacuum generation
-      const T s_starl = L.v[AX] - T(2) * L.cs / G.gm1;
-      const T s_starr = R.v[AX] + T(2) * R.cs / G.gm1;
+      const double s_starl = L.v[AX] - 2.0 * L.cs / G.gm1;
+      const double s_starr = R.v[AX] + 2.0 * R.cs / G.gm1;
       if (dxdt > s_starr) {
-        side_transverse<D, AX>(R, r);
+        side_transverse<D, AX>(R, r, ir);
         if (dxdt > R.v[AX] + R.cs) prim_vars_to_cons<D>(G, R.rho, R.v, R.p, u);
         else w_kfan<D, AX>(G, R, dxdt, true, u);
       } else if (dxdt > s_starl) {
         vacuum_state<D>(G, rp, u);
       } else {
-        side_transverse<D, AX>(L, l);
+        side_transverse<D, AX>(L, l, il);
         if (dxdt > L.v[AX] - L.cs) w_kfan<D, AX>(G, L, dxdt, false, u);
         else prim_vars_to_cons<D>(G, L.rho, L.v, L.p, u);
       }
     } else {
-      Star<T> s;
-      rp_star_pu<D, AX, T, LAZY>(G, rp, L, R, s);
-      rp_sampling<D, AX>(G, L, R, l, r, s, dxdt, u);
+      // rhyme_riemann_problem_star.f90:12-38
+      double l_f = 0.0, r_f = 0.0;
+      const WaveSide WL = wave_side(G, L.rho, L.p, L.cs), WR = wave_side(G, R.rho, R.p, R.cs);
+      double ps = irs_exec(G, rp.tol, rp.n_iter, WL, WR, L.rho, L.v[AX], L.cs, l_f, R.rho, R.v[AX], R.cs, r_f);
+      if (m_gt(rp.vac_p, ps)) ps = rp.vac_p;
+      const double us = 0.5 * ((R.v[AX] + L.v[AX]) + (r_f - l_f));
+      // the side of the contact that x/t = dxdt lies on
+      const bool right = dxdt > us;
+      Side<D> S;
+      S.rho = right ? R.rho : L.rho;
+      S.v[AX] = right ? R.v[AX] : L.v[AX];
+      S.p = right ? R.p : L.p;
+      S.cs = right ? R.cs : L.cs;
+      S.ip = right ? WR.ip : WL.ip;
+      double q[D + 2];
+#pragma unroll
+      for (int c = 0; c < D + 2; ++c) q[c] = right ? r[c] : l[c];
+      side_transverse<D, AX>(S, q, right ? ir : il);
+      rp_sample_side<D, AX>(G, S, right, us, ps, dxdt, u);
     }
   }
 }
@@ -792,12 +803,11 @@ __device__ __forceinline__ void rp_flux_f32(const Gas<float>& G, const Rp<float>
 
 // Interface flux: Riemann state at x/t = 0 (dx = 0 in
 // rhyme_muscl_hancock_solve_memory_intensive.f90:110-116), then calc_flux.
-// LAZY: see WaveSide.
-template <int D, int AX, typename T, bool LAZY = false>
-__device__ __forceinline__ void interface_flux(const Gas<T>& G, const Rp<T>& rp, const T* l, const T* r,
-                                               T* f) {
-  T u[D + 2];
-  rp_solve<D, AX, T, LAZY>(G, rp, l, r, T(0), u);
+template <int D, int AX>
+__device__ __forceinline__ void interface_flux(const Gas<double>& G, const Rp<double>& rp, const double* l,
+                                               const double* r, double* f) {
+  double u[D + 2];
+  rp_solve<D, AX>(G, rp, l, r, 0.0, u);
   flux<D, AX>(G, u, f);
 }
 

@@ -125,6 +125,19 @@ __global__ void conversion_check_kernel(long long n, unsigned long long seed, un
       }
       default: bits = 0; break;
     }
+    // fp64_int.h: division, root and comparison of x and a second operand
+    // (of the same magnitude for half the values) against the hardware's
+    {
+      const double x = __longlong_as_double((long long)((t & 3) != 3 ? bits : r));
+      unsigned long long yb = splitmix(s);
+      if (t & 4) yb = (yb & 0x800fffffffffffffull) | ((1023ull - 8 + (yb >> 52 & 15)) << 52);
+      const double y = __longlong_as_double((long long)yb);
+      const double q[3] = {rgpu::div_rn(x, y), rgpu::sqrt_rn(x), rgpu::sqrt_rn(fabs(y))};
+      const double h[3] = {x / y, sqrt(x), sqrt(fabs(y))};
+      for (int k = 0; k < 3; ++k)
+        if (__double_as_longlong(q[k]) != __double_as_longlong(h[k]) && !(isnan(q[k]) && isnan(h[k]))) ++local;
+      if (rgpu::f64_gt(x, y) != (x > y) || rgpu::f64_above(x, 1.0) != (x > 1.0) || rgpu::f64_negative(x) != (x < 0.0)) ++local;
+    }
     if ((t & 3) != 3) {
       const double x = __longlong_as_double((long long)bits);
       const float a = rgpu::narrow_mirror(x), b = rgpu::mirror_of(x);

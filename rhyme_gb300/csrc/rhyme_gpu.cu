@@ -211,6 +211,9 @@ void rgpu::make_dev_params(const rhyme_gpu_params* p, DevParams* d) {
   G.gm1_half = 0.5 * G.gm1;
   G.half_gm1 = G.gm1 / 2.0;
   G.g_kb_amu = g * p->kb_amu;
+  G.by_gm1 = m_inv(G.gm1);
+  G.by_gp1 = m_inv(G.gp1);
+  G.by_kb_amu = m_inv(G.kb_amu);
   d->rp.vac_rho = p->vacuum_density;
   d->rp.vac_p = p->vacuum_pressure;
   d->rp.vac_rho_next = std::nextafter(p->vacuum_density, 1.0);
@@ -247,6 +250,9 @@ void make_mixed_params(const DevParams& d, MixedParams* m) {
   F.gm1_half = (float)G.gm1_half;
   F.half_gm1 = (float)G.half_gm1;
   F.g_kb_amu = (float)G.g_kb_amu;
+  F.by_gm1 = m_inv(F.gm1);
+  F.by_gp1 = m_inv(F.gp1);
+  F.by_kb_amu = m_inv(F.kb_amu);
   m->rp.vac_rho = (float)d.rp.vac_rho;
   m->rp.vac_p = (float)d.rp.vac_p;
   m->rp.vac_rho_next = std::nextafter((float)d.rp.vac_rho, 1.0f);
