@@ -33,95 +33,67 @@ __host__ __device__ inline BoxRules rules_of(const DevParams& P) {
   return r;
 }
 
-// Ghost lines of a box: axis a contributes (D+2) * prod_{b != a} n_b lines.
-template <int D>
-__host__ __device__ inline void ghost_offsets(const Geom& g, long long& off1, long long& off2,
-                                              long long& total) {
-  long long per_axis[3] = {0, 0, 0};
-  for (int a = 0; a < D; ++a) {
-    long long t = D + 2;
-    for (int b = 0; b < D; ++b)
-      if (b != a) t *= g.n[b];
-    per_axis[a] = t;
-  }
-  off1 = per_axis[0];
-  off2 = off1 + per_axis[1];
-  total = off2 + per_axis[2];
+// Ghost lines of a box: line q of (axis, component), q = 0 .. ghost_lines - 1,
+// the transverse positions in array order.
+__host__ __device__ inline long long ghost_lines(int D, const Geom& g, int axis) {
+  long long t = 1;
+  for (int b = 0; b < D; ++b)
+    if (b != axis) t *= g.n[b];
+  return t;
 }
 
 // K1 element: fills the left then the right 2-cell ghost layer of one line
-// (axis, component, transverse position) in the order of
-// rhyme_samr_bc_set_boundaries.f90:9-20; writes U and (if given) M.
-// M (optional) receives the same ghost values (the other state buffer); Mf
-// (optional) their FP32 images (the mirror of the mixed form), equal to what
-// a fill of the mirror from its own interior would write.
+// in the order of rhyme_samr_bc_set_boundaries.f90:9-20; writes U and (if
+// given) M. M (optional) receives the same ghost values (the other state
+// buffer); Mf (optional) their FP32 images (the mirror of the mixed form),
+// equal to what a fill of the mirror from its own interior would write.
+// A plane holds fewer than 2^32 lines (the array would not fit otherwise),
+// so the position is split in 32 bits.
 template <int D, typename T>
-__device__ __forceinline__ void ghost_elem(const BoxRules& R, T* __restrict__ U, T* __restrict__ M,
-                                           const Geom& g, long long off1, long long off2, long long t,
-                                           float* __restrict__ Mf = nullptr) {
-  int axis;
-  long long r;
-  if (t < off1) {
-    axis = 0;
-    r = t;
-  } else if (t < off2) {
-    axis = 1;
-    r = t - off1;
-  } else {
-    axis = 2;
-    r = t - off2;
+__device__ __forceinline__ void ghost_line(const BoxRules& R, T* __restrict__ U, T* __restrict__ M, const Geom& g,
+                                           int axis, int c, unsigned q, float* __restrict__ Mf) {
+  const unsigned n1 = (D == 1) ? 1u : (unsigned)g.n[axis == 0 ? 1 : 0];
+  unsigned i2 = 0, i1 = q;
+  if constexpr (D == 3) {
+    i2 = q / n1;
+    i1 = q - i2 * n1;
   }
+  // cell 0 of the line
+  long long base = g.s[0] + (D > 1 ? g.s[1] : 0) + (D > 2 ? g.s[2] : 0);
   const int t1 = (axis == 0) ? 1 : 0, t2 = (axis == 2) ? 1 : 2;
-  const int n1 = (t1 < D) ? g.n[t1] : 1, n2 = (t2 < D) ? g.n[t2] : 1;
-  const long long per_c = (long long)n1 * n2;
-  const int c = (int)(r / per_c);
-  const long long q = r - (long long)c * per_c;
-  int i1 = (int)(q % n1) + 1, i2 = (int)(q / n1) + 1;
-  int idx0 = 1, idx1 = 1, idx2 = 1;
-  if (t1 == 0) idx0 = i1; else idx1 = i1;
-  if (t2 == 1) idx1 = i2; else idx2 = i2;
-  if (axis == 0) idx0 = 0; else if (axis == 1) idx1 = 0; else idx2 = 0;
-  const long long base = g.at(D, idx0, idx1, idx2);  // cell 0 of the line
-  const long long sa = g.s[axis];
-  const long long N = g.n[axis];
+  if constexpr (D > 1) base += (long long)(i1 + 1) * g.s[t1];
+  if constexpr (D > 2) base += (long long)(i2 + 1) * g.s[t2];
+  const long long sa = g.s[axis], N = g.n[axis];
   T* f = U + (long long)c * g.field;
+  T* m = M ? M + (long long)c * g.field : nullptr;
+  float* mf = Mf ? Mf + (long long)c * g.field : nullptr;
+#pragma unroll
   for (int side = 0; side < 2; ++side) {
     const int type = R.bc[2 * axis + side];
-    long long g0, g1, s0, s1;
-    if (side == 0) {
-      g0 = base;
-      g1 = base - sa;
-      s0 = (type == 3) ? base + N * sa : base + sa;
-      s1 = (type == 3) ? base + (N - 1) * sa : base + 2 * sa;
-    } else {
-      g0 = base + (N + 1) * sa;
-      g1 = base + (N + 2) * sa;
-      s0 = (type == 3) ? base + sa : base + N * sa;
-      s1 = (type == 3) ? base + 2 * sa : base + (N - 1) * sa;
-    }
+    if (type < 1 || type > 4) continue;  // the caller fills this face
+    const bool far = (type == 3) != (side == 1);  // the sources lie at the line's other end
+    const long long g0 = side ? base + (N + 1) * sa : base, g1 = side ? g0 + sa : g0 - sa;
+    const long long s0 = far ? base + N * sa : base + sa, s1 = far ? s0 - sa : s0 + sa;
+    T v0, v1;
     if (type == 4) {  // inflow
-      const T v = (T)R.inflow[2 * axis + side][c];
-      f[g0] = v;
-      f[g1] = v;
-    } else if (type >= 1 && type <= 3) {
-      f[g0] = f[s0];
-      f[g1] = f[s1];
-      if (type == 1 && c == 1 + axis) {  // reflective: negate normal momentum
-        f[g0] = -f[s0];
-        f[g1] = -f[s1];
-      }
+      v0 = v1 = (T)R.inflow[2 * axis + side][c];
     } else {
-      continue;
+      v0 = f[s0];
+      v1 = (s1 == g0) ? v0 : f[s1];  // a periodic line of one cell: the first ghost is the second's source
+      if (type == 1 && c == 1 + axis) {  // reflective: negate normal momentum
+        v0 = -v0;
+        v1 = -v1;
+      }
     }
-    if (M) {
-      T* m = M + (long long)c * g.field;
-      m[g0] = f[g0];
-      m[g1] = f[g1];
+    f[g0] = v0;
+    f[g1] = v1;
+    if (m) {
+      m[g0] = v0;
+      m[g1] = v1;
     }
-    if (Mf) {
-      float* m = Mf + (long long)c * g.field;
-      m[g0] = mirror_of(f[g0]);
-      m[g1] = mirror_of(f[g1]);
+    if (mf) {
+      mf[g0] = mirror_of(v0);
+      mf[g1] = mirror_of(v1);
     }
   }
 }

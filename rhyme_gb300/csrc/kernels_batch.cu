@@ -1,45 +1,39 @@
 // kernels_batch.cu -- one step of a batch of independent boxes of uneven
 // sizes, each with its own dt, boundary types, limiter and cell size.
 //
-// Every pass is one persistent kernel (a few CTAs per SM) fed by a work
-// queue: the host lists, per box, the chunks of that pass's index space
-// (largest boxes first), and each CTA repeatedly takes the next chunk with an
-// atomic increment of the pass's queue head. The per-element arithmetic is
-// the single-box code (box_elems.cuh, the mixed sweep body), so a box gives
-// the same result alone and inside a batch. A step is captured once per
-// buffer parity in a CUDA graph by the host.
+// Every pass is one persistent kernel (a few CTAs per SM) over a list of work
+// items: the host lists, per box, the chunks of that pass's index space
+// (largest boxes first). Passes whose items differ in cost (the FP64 fluxes,
+// the mixed sweeps) take the next item from a queue head, an atomic whose
+// round trip the item before it hides; the others deal their items out in
+// turn. The per-element arithmetic is the single-box code (box_elems.cuh,
+// the mixed sweep body), so a box gives the same result alone and inside a
+// batch. A step is captured once per buffer parity in a CUDA graph by the
+// host.
 //
 // Compiled with --fmad=false (the FP64 passes must match the oracle).
+#include <algorithm>
+
 #include "box_elems.cuh"
 
 namespace rgpu {
 
 namespace {
 
-// Next work item of a pass for this CTA (-1 when the queue is empty).
-__device__ __forceinline__ int next_item(int* head, int n) {
-  __shared__ int s_item;
-  __syncthreads();
-  if (threadIdx.x == 0) s_item = atomicAdd(head, 1);
-  __syncthreads();
-  const int it = s_item;
-  return it < n ? it : -1;
-}
-
 template <int D>
 __global__ void __launch_bounds__(256)
     batch_cfl_kernel(Gas<double> G, double courant, const BoxDesc* __restrict__ T,
-                     const WorkItem* __restrict__ items, int n, int* head) {
+                     const WorkItem* __restrict__ items, int n) {
   __shared__ double sm[8];
   __shared__ int sb[8];
-  for (int it = next_item(head, n); it >= 0; it = next_item(head, n)) {
+  for (int it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
     const BoxDesc& b = T[w.box];
     const long long total = (long long)b.g.n[0] * b.g.n[1] * b.g.n[2];
-    const long long t = w.chunk * kBatchChunk + threadIdx.x;
+    const long long t1 = min(total, (w.chunk + 1) * kBatchCflChunk);
     double m = 0.0;
     int bad = 0;
-    if (t < total) {
+    for (long long t = w.chunk * kBatchCflChunk + threadIdx.x; t < t1; t += 256) {
       const double v = signal_speed_elem<D>(G, b.U, b.g, t, bad);
       if (v > m) m = v;
     }
@@ -74,29 +68,28 @@ __global__ void __launch_bounds__(256)
         atomicExch(counter, 0u);
       }
     }
+    __syncthreads();
   }
 }
 
-template <int D, typename T>
+// Ghost fill of every box: an item is a chunk of the lines of one axis and
+// component (item.axis = axis (D + 2) + component). In mixed precision it
+// writes the FP32 mirror's ghosts too, as the single-box fill.
+template <int D>
 __global__ void __launch_bounds__(256)
-    batch_ghost_kernel(const BoxDesc* __restrict__ TB, const WorkItem* __restrict__ items, int n,
-                       int* head, bool f32) {
-  for (int it = next_item(head, n); it >= 0; it = next_item(head, n)) {
+    batch_ghost_kernel(const BoxDesc* __restrict__ TB, const WorkItem* __restrict__ items, int n) {
+  for (int it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
     const BoxDesc& b = TB[w.box];
-    long long off1, off2, total;
-    ghost_offsets<D>(b.g, off1, off2, total);
-    const long long t = w.chunk * kBatchChunk + threadIdx.x;
-    if (t >= total) continue;
+    const int axis = w.axis / (D + 2), c = w.axis % (D + 2);
+    const long long q = w.chunk * kBatchChunk + threadIdx.x;
+    if (q >= ghost_lines(D, b.g, axis)) continue;
     BoxRules R;
     for (int i = 0; i < 6; ++i) {
       R.bc[i] = b.bc[i];
-      for (int c = 0; c < 5; ++c) R.inflow[i][c] = b.inflow[i][c];
+      for (int k = 0; k < 5; ++k) R.inflow[i][k] = b.inflow[i][k];
     }
-    if (f32)
-      ghost_elem<D, T>(R, (T*)b.Uf, (T*)nullptr, b.g, off1, off2, t);
-    else
-      ghost_elem<D, T>(R, (T*)b.U, (T*)b.V, b.g, off1, off2, t);
+    ghost_line<D, double>(R, b.U, b.V, b.g, axis, c, (unsigned)q, b.Uf);
   }
 }
 
@@ -113,8 +106,8 @@ __device__ __forceinline__ BoxRules rules_of_box(const BoxDesc& b) {
 template <int D>
 __global__ void __launch_bounds__(128)
     batch_faces_kernel(Gas<double> G, const BoxDesc* __restrict__ TB, const WorkItem* __restrict__ items,
-                       int n, int* head) {
-  for (int it = next_item(head, n); it >= 0; it = next_item(head, n)) {
+                       int n) {
+  for (int it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
     const BoxDesc& b = TB[w.box];
     const BoxRules R = rules_of_box<D>(b);
@@ -138,7 +131,10 @@ template <int D>
 __global__ void __launch_bounds__(128, 3)
     batch_flux_kernel(Gas<double> G, Rp<double> rp, const BoxDesc* __restrict__ TB,
                       const WorkItem* __restrict__ items, int n, int* head) {
-  for (int it = next_item(head, n); it >= 0; it = next_item(head, n)) {
+  __shared__ int s_next;
+  for (int it = blockIdx.x; it < n;) {
+    int next = 0;
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(head, 1);
     const WorkItem w = items[it];
     const BoxDesc& b = TB[w.box];
     const long long t = w.chunk * kBatchFluxChunk + threadIdx.x;
@@ -151,14 +147,17 @@ __global__ void __launch_bounds__(128, 3)
     if constexpr (D > 2) {
       if (w.axis == 2 && t < iface_count<2>(b.g)) flux_elem<D, 2>(G, rp, b.faces, b.g, b.fluxes, t);
     }
+    if (threadIdx.x == 0) s_next = next;
+    __syncthreads();
+    it = s_next;
+    __syncthreads();
   }
 }
 
 template <int D>
 __global__ void __launch_bounds__(256)
-    batch_update_kernel(const BoxDesc* __restrict__ TB, const WorkItem* __restrict__ items, int n,
-                        int* head) {
-  for (int it = next_item(head, n); it >= 0; it = next_item(head, n)) {
+    batch_update_kernel(const BoxDesc* __restrict__ TB, const WorkItem* __restrict__ items, int n) {
+  for (int it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
     const BoxDesc& b = TB[w.box];
     const long long total = (long long)b.g.n[0] * b.g.n[1] * b.g.n[2];
@@ -181,18 +180,16 @@ cudaError_t batch_step_d(const DevParams& P, const MixedParams& M, bool mixed, c
     e = launch_batch_cfl_mixed(M, P.courant, TB, L, st);
     if (e != cudaSuccess) return e;
   } else if (L.n_cfl) {
-    batch_cfl_kernel<D><<<152 * 4, 256, 0, st>>>(P.G, P.courant, TB, L.cfl, L.n_cfl, L.heads + 0);
+    batch_cfl_kernel<D><<<std::min(L.n_cfl, 152 * 4), 256, 0, st>>>(P.G, P.courant, TB, L.cfl, L.n_cfl);
   }
-  if (L.n_ghost) {
-    batch_ghost_kernel<D, double><<<152 * 4, 256, 0, st>>>(TB, L.ghost, L.n_ghost, L.heads + 1, false);
-    if (mixed) batch_ghost_kernel<D, float><<<152 * 4, 256, 0, st>>>(TB, L.ghost, L.n_ghost, L.heads + kHeadGhostF32, true);
-  }
+  if (L.n_ghost) batch_ghost_kernel<D><<<std::min(L.n_ghost, 152 * 8), 256, 0, st>>>(TB, L.ghost, L.n_ghost);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (mixed) return launch_batch_sweeps(M, TB, L, q, st);
-  if (L.n_faces) batch_faces_kernel<D><<<152 * 4, 128, 0, st>>>(P.G, TB, L.faces, L.n_faces, L.heads + 2);
-  if (L.n_flux) batch_flux_kernel<D><<<152 * 3, 128, 0, st>>>(P.G, P.rp, TB, L.flux, L.n_flux, L.heads + 3);
-  if (L.n_update) batch_update_kernel<D><<<152 * 4, 256, 0, st>>>(TB, L.update, L.n_update, L.heads + 4);
+  if (L.n_faces) batch_faces_kernel<D><<<std::min(L.n_faces, 152 * 8), 128, 0, st>>>(P.G, TB, L.faces, L.n_faces);
+  if (L.n_flux)
+    batch_flux_kernel<D><<<std::min(L.n_flux, 152 * 3), 128, 0, st>>>(P.G, P.rp, TB, L.flux, L.n_flux, L.heads + kHeadFlux);
+  if (L.n_update) batch_update_kernel<D><<<std::min(L.n_update, 152 * 8), 256, 0, st>>>(TB, L.update, L.n_update);
   return cudaGetLastError();
 }
 

@@ -20,7 +20,7 @@
 //
 // This file is compiled with --fmad=false so the double arithmetic performs
 // the same IEEE operations, in the same order, as the reference.
-#include <cstdio>
+#include <algorithm>
 
 #include "box_elems.cuh"
 
@@ -43,18 +43,18 @@ inline int grid_for(long long total, int block) {
 }
 
 // ------------------------------------------------------------------ K1 ---
-// One thread per (axis, component, transverse position): fills the left then
-// the right 2-cell ghost layer of its line in the order of
-// rhyme_samr_bc_set_boundaries.f90:9-20, writing U and (if given) the mirror
-// buffer, so both state buffers carry the ghost values the reference array
-// holds after the fill.
+// One thread per (axis, component, transverse position), the axis and the
+// component from blockIdx.y: fills the left then the right 2-cell ghost
+// layer of its line, writing U, the other state buffer M and the FP32 mirror
+// Mf (if given), so both state buffers carry the ghost values the reference
+// array holds after the fill. Bound by the scattered sectors of the x faces.
 template <int D, typename T>
 __global__ void __launch_bounds__(kFillBlock)
-    ghost_fill_kernel(BoxRules R, T* __restrict__ U, T* __restrict__ M, Geom g, long long off1,
-                      long long off2, long long total, float* __restrict__ Mf) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x)
-    ghost_elem<D, T>(R, U, M, g, off1, off2, t, Mf);
+    ghost_fill_kernel(BoxRules R, T* __restrict__ U, T* __restrict__ M, Geom g, float* __restrict__ Mf) {
+  const int axis = blockIdx.y / (D + 2), c = blockIdx.y % (D + 2);
+  const long long n = ghost_lines(D, g, axis);
+  for (long long q = (long long)blockIdx.x * kFillBlock + threadIdx.x; q < n; q += (long long)gridDim.x * kFillBlock)
+    ghost_line<D, T>(R, U, M, g, axis, c, (unsigned)q, Mf);
 }
 
 // ------------------------------------------------------------------ K2 ---
@@ -233,10 +233,10 @@ int max_cfl_blocks() { return kMaxBlocks; }
 
 template <int D, typename T>
 cudaError_t ghost_fill_d(const BoxRules& R, T* U, T* U_mirror, const Geom& g, cudaStream_t st, float* Uf) {
-  long long off1, off2, total;
-  ghost_offsets<D>(g, off1, off2, total);
-  ghost_fill_kernel<D, T><<<grid_for(total, kFillBlock), kFillBlock, 0, st>>>(R, U, U_mirror, g, off1, off2,
-                                                                              total, Uf);
+  long long lines = 0;
+  for (int a = 0; a < D; ++a) lines = std::max(lines, ghost_lines(D, g, a));
+  const dim3 grid(grid_for(lines, kFillBlock), D * (D + 2));
+  ghost_fill_kernel<D, T><<<grid, kFillBlock, 0, st>>>(R, U, U_mirror, g, Uf);
   return cudaGetLastError();
 }
 

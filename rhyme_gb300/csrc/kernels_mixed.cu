@@ -392,28 +392,38 @@ cudaError_t launch_fallback(const MixedParams& M, const FallbackQueue& q, const 
   return cudaGetLastError();
 }
 
-// Batched FP32 CFL over work items (chunks of 256 cells of a box): per-box
-// maximum through atomics, the last item of a box forms its dt in FP64.
+// Batched FP32 CFL over work items (chunks of a box's cells), per box as
+// cfl_carry_kernel: dt from the maximum that the box's last sweep folded,
+// unless *whole is set (some box was not stepped by a batch last) or the FP64
+// fix-up changed the box after that sweep (carry_ok cleared): then the pass
+// over its cells, per-box maximum through atomics, the last item of a box
+// forming its dt in FP64.
 template <int D>
 __global__ void __launch_bounds__(256)
     batch_cfl_f32_kernel(MixedParams M, double courant, const BoxDesc* __restrict__ TB,
-                         const WorkItem* __restrict__ items, int n, int* head) {
+                         const WorkItem* __restrict__ items, int n, const int* __restrict__ whole) {
   __shared__ float sm[8];
   __shared__ int sb[8];
-  __shared__ int s_item;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_item = atomicAdd(head, 1);
-    __syncthreads();
-    const int it = s_item;
-    if (it >= n) break;
+  const bool all = *whole != 0;
+  for (int it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
     const BoxDesc& b = TB[w.box];
+    // every thread sees the flag that the box's last item sets at its end as
+    // it was before the pass (that item ends after this one's own count)
+    const bool carried = !all && *(volatile int*)carry_ok_of(b) != 0;
+    if (carried) {
+      if (w.chunk == 0 && threadIdx.x == 0) {
+        const float mu = __uint_as_float((unsigned int)*carry_bits_of(b));
+        b.ctl[0] = courant * b.dx.min / (double)mu;
+        *carry_bits_of(b) = 0ull;
+      }
+      continue;
+    }
     const long long total = (long long)b.g.n[0] * b.g.n[1] * b.g.n[2];
-    const long long t = w.chunk * kBatchChunk + threadIdx.x;
+    const long long t1 = min(total, (w.chunk + 1) * kBatchCflChunk);
     float m = 0.f;
     int bad = 0;
-    if (t < total) {
+    for (long long t = w.chunk * kBatchCflChunk + threadIdx.x; t < t1; t += 256) {
       const float v = signal_speed_f32<D>(M, b.U, b.Uf, b.g, t, bad);
       if (v > m) m = v;
     }
@@ -446,8 +456,11 @@ __global__ void __launch_bounds__(256)
         b.ctl[0] = courant * b.dx.min / (double)mu;
         atomicExch(max_bits, 0ull);
         atomicExch(counter, 0u);
+        *carry_bits_of(b) = 0ull;
+        *(volatile int*)carry_ok_of(b) = 1;
       }
     }
+    __syncthreads();
   }
 }
 
@@ -460,6 +473,7 @@ __global__ void __launch_bounds__(128)
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const FallbackEntry e = q.e[i];
     const BoxDesc& b = TB[e.box];
+    *carry_ok_of(b) = 0;  // the box's cells change after its last sweep: its next CFL pass is whole
     double f[D + 2];
     redo_any_axis<D>(M, b.limiter, b.omega, b.U, b.g, e.axis, e.o, 0.5 * b.ctl[0] / b.dx.v[e.axis], f);
     const double dtdx = b.ctl[0] / b.dx.v[e.axis];
@@ -625,10 +639,11 @@ long long sweep_tile_count(int ndim, int axis, int shape, const int* n) {
 cudaError_t launch_batch_cfl_mixed(const MixedParams& M, double courant, const BoxDesc* TB,
                                    const BatchLists& L, cudaStream_t st) {
   if (!L.n_cfl) return cudaSuccess;
+  const int grid = L.n_cfl < 152 * 8 ? L.n_cfl : 152 * 8;
   switch (M.ndim) {
-    case 1: batch_cfl_f32_kernel<1><<<152 * 4, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.heads + 0); break;
-    case 2: batch_cfl_f32_kernel<2><<<152 * 4, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.heads + 0); break;
-    case 3: batch_cfl_f32_kernel<3><<<152 * 4, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.heads + 0); break;
+    case 1: batch_cfl_f32_kernel<1><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole); break;
+    case 2: batch_cfl_f32_kernel<2><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole); break;
+    case 3: batch_cfl_f32_kernel<3><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -644,9 +659,12 @@ cudaError_t launch_batch_sweeps(const MixedParams& M, const BoxDesc* TB, const B
   cudaError_t e = cudaMemsetAsync(q.n, 0, sizeof(int), st);
   for (int a = 0; a < D; ++a)
     for (int k = 0; k < kSweepShapes; ++k)
-      if (e == cudaSuccess && L.n_sweep[a][k])
-        e = launch_batch_sweep_axis(D, a, k, M, TB, L.sweep[a][k], L.n_sweep[a][k],
-                                    L.heads + kHeadSweep0 + kSweepShapes * a + k, q, st);
+      if (e == cudaSuccess && L.n_sweep[a][k]) {
+        int* head = L.heads + kHeadSweep0 + kSweepShapes * a + k;
+        e = (L.fuse_xy && a == 0)
+                ? launch_batch_sweep_xy_3(k, M, TB, L.sweep[a][k], L.n_sweep[a][k], head, q, st)
+                : launch_batch_sweep_axis(D, a, k, M, TB, L.sweep[a][k], L.n_sweep[a][k], head, q, st);
+      }
   if (e == cudaSuccess) {
     switch (D) {
       case 1: e = launch_batch_fallback<1>(M, TB, q, st); break;

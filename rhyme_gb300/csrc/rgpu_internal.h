@@ -309,6 +309,7 @@ struct BoxDesc {
   double* U;
   double* V;
   float* Uf;
+  float* Uf_next;  // the mirror of V
   float* acc;
   double* faces;
   double* fluxes;
@@ -331,6 +332,11 @@ struct WorkItem {
   long long chunk;
 };
 
+// The carried CFL of a box in its control block: the maximum the last sweep
+// folds for the next step, and whether it is the state's.
+__device__ __forceinline__ unsigned long long* carry_bits_of(const BoxDesc& b) { return (unsigned long long*)(b.ctl + 6); }
+__device__ __forceinline__ int* carry_ok_of(const BoxDesc& b) { return (int*)(b.ctl + 7); }
+
 // Device views of a batch's per-pass item lists and queue heads.
 struct BatchLists {
   const WorkItem* cfl;
@@ -340,8 +346,35 @@ struct BatchLists {
   const WorkItem* update;
   const WorkItem* sweep[3][kSweepShapes];  // tiles of each axis, grouped by shape
   int n_cfl, n_ghost, n_faces, n_flux, n_update, n_sweep[3][kSweepShapes];
+  bool fuse_xy;  // 3-D mixed: sweep[0] holds the tiles of the fused x and y sweep, by tile shape
   int* heads;  // one queue head per pass (kBatchHeads, reset before each step)
+  const int* whole;  // nonzero: the step's CFL pass is whole for every box (mixed)
 };
+
+// Tiles of the fused x and y sweep of a batch: 8 x 32, 16 x 16 or 32 x 8
+// cells of a z plane, whichever covers the box's plane with the fewest (a
+// tile costs the same within 2 % whatever its shape; edges of 8, 24, 40 or
+// 56 cells leave half of a 16-cell tile idle), 16 x 16 on a tie.
+constexpr int kXYShapes = 3;
+__host__ __device__ inline void xy_shape(int k, int* tx, int* ty) {
+  *tx = 8 << k;
+  *ty = 256 / *tx;
+}
+inline int batch_xy_shape(int nx, int ny) {
+  int best = 1;
+  long long least = 0;
+  for (int i = 0; i < kXYShapes; ++i) {
+    const int k = (i == 0) ? 1 : (i == 1 ? 0 : 2);
+    int tx, ty;
+    xy_shape(k, &tx, &ty);
+    const long long t = (long long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
+    if (i == 0 || t < least) {
+      best = k;
+      least = t;
+    }
+  }
+  return best;
+}
 
 // Tile count of a sweep of a box of dims n along `axis` with tile shape
 // `shape` (the work items of a batch enumerate these).
@@ -395,6 +428,9 @@ inline cudaError_t launch_batch_sweep_axis(int ndim, int axis, int shape, const 
   }
 }
 
+cudaError_t launch_batch_sweep_xy_3(int shape, const MixedParams& M, const BoxDesc* TB, const WorkItem* items, int n,
+                                    int* head, const FallbackQueue& q, cudaStream_t st);
+
 cudaError_t launch_batch_cfl_mixed(const MixedParams& M, double courant, const BoxDesc* TB,
                                    const BatchLists& L, cudaStream_t st);
 cudaError_t launch_batch_sweeps(const MixedParams& M, const BoxDesc* TB, const BatchLists& L,
@@ -403,14 +439,18 @@ cudaError_t launch_batch_step(const DevParams& P, const MixedParams& M, bool mix
                               const BoxDesc* table, const BatchLists& L, FallbackQueue q,
                               cudaStream_t st);
 
-// Queue heads of a batch step: 0 cfl, 1 ghost, 2 faces, 3 flux, 4 update,
-// 5 ghost (FP32 mirror), 6 + kSweepShapes * axis + shape the sweeps.
-constexpr int kBatchHeads = 32;
-constexpr int kHeadGhostF32 = 5;
-constexpr int kHeadSweep0 = 6;
+// Queue heads of a batch step: 0 the FP64 fluxes, 1 + kSweepShapes * axis +
+// shape the sweeps. The passes whose items all cost the same (CFL, ghosts,
+// faces, update) deal them out in turn instead.
+constexpr int kBatchHeads = 16;
+constexpr int kHeadFlux = 0;
+constexpr int kHeadSweep0 = 1;
 
-// Chunk sizes of the batched passes (elements per work item).
+// Chunk sizes of the batched passes (elements per work item). A CFL item
+// ends in a reduction over its CTA: at 256 cells (one a thread) the pass
+// spent its time in barriers and took 0.20 ms for 5.4 M cells.
 constexpr int kBatchChunk = 256;
+constexpr int kBatchCflChunk = 2048;
 constexpr int kBatchFluxChunk = 128;
 
 // One box of a level output (kernels_output.cu): its current state, its

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/rhyme_gpu.h"
+#include "box_elems.cuh"
 #include "rgpu_internal.h"
 
 using namespace rgpu;
@@ -79,6 +80,7 @@ struct Box {
   unsigned long long* carry_bits = nullptr;
   int* carry_ok = nullptr;
   bool carry_valid = false;
+  bool batch_carry = false;  // likewise since the last batch run
   bool wb = false;
   bool wb_pending = false;
 };
@@ -403,6 +405,7 @@ void state_changed(Box* b) {
   b->mirror_valid = false;
   b->maxu_valid = false;
   b->carry_valid = false;
+  b->batch_carry = false;
   b->wb_pending = false;
 }
 
@@ -1491,7 +1494,7 @@ struct rhyme_gpu_batch {
   int* heads = nullptr;
   BatchLists L{};
   FallbackQueue q{};
-  int* qblock = nullptr;  // n, status, total
+  int* qblock = nullptr;  // n, status, total, whole (BatchLists)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   int runs = 0;  // batch_run calls since the tables were built
 };
@@ -1539,6 +1542,7 @@ int batch_build(rhyme_gpu_batch* B) {
   tab[0].resize(n);
   tab[1].resize(n);
   std::vector<WorkItem> cfl, ghost, faces, flux, update, sweep[3][kSweepShapes];
+  const bool fuse = ctx->mixed && D == 3 && ctx->fuse_xy;
   long long qcap = 0;
   for (int i = 0; i < n; ++i) {
     Box* b = ctx->boxes[B->handles[i]];
@@ -1554,6 +1558,7 @@ int batch_build(rhyme_gpu_batch* B) {
       d.U = b->state[c];
       d.V = b->state[1 - c];
       d.Uf = b->Uf[c];
+      d.Uf_next = b->Uf[1 - c];
       d.acc = b->acc;
       d.faces = b->s.faces;
       d.fluxes = b->s.fluxes;
@@ -1568,7 +1573,7 @@ int batch_build(rhyme_gpu_batch* B) {
         d.bc[f] = b->dp.bc[f];
         for (int cc = 0; cc < 5; ++cc) d.inflow[f][cc] = b->dp.inflow[f][cc];
       }
-      d.cfl_items = (int)((cells + kBatchChunk - 1) / kBatchChunk);
+      d.cfl_items = (int)((cells + kBatchCflChunk - 1) / kBatchCflChunk);
     }
   }
   for (int oi = 0; oi < n; ++oi) {
@@ -1576,17 +1581,19 @@ int batch_build(rhyme_gpu_batch* B) {
     const Box* b = ctx->boxes[B->handles[i]];
     const Geom& g = b->g;
     const long long cells = (long long)g.n[0] * g.n[1] * g.n[2];
-    for (long long c = 0; c * kBatchChunk < cells; ++c) cfl.push_back({i, 0, c});
-    long long lines = 0;
-    for (int a = 0; a < D; ++a) {
-      long long t = D + 2;
-      for (int o = 0; o < D; ++o)
-        if (o != a) t *= g.n[o];
-      lines += t;
-    }
-    for (long long c = 0; c * kBatchChunk < lines; ++c) ghost.push_back({i, 0, c});
+    for (long long c = 0; c * kBatchCflChunk < cells; ++c) cfl.push_back({i, 0, c});
+    for (int a = 0; a < D; ++a)
+      for (int c = 0; c < D + 2; ++c)
+        for (long long k = 0; k * kBatchChunk < ghost_lines(D, g, a); ++k) ghost.push_back({i, a * (D + 2) + c, k});
     if (ctx->mixed) {
-      for (int a = 0; a < D; ++a) {
+      if (fuse) {
+        int tx, ty;
+        const int k = batch_xy_shape(g.n[0], g.n[1]);
+        xy_shape(k, &tx, &ty);
+        const long long nt = (long long)((g.n[0] + tx - 1) / tx) * ((g.n[1] + ty - 1) / ty) * g.n[2];
+        for (long long t = 0; t < nt; ++t) sweep[0][k].push_back({i, 0, t});
+      }
+      for (int a = fuse ? 2 : 0; a < D; ++a) {
         const int k = b->plan.shape[a];
         const long long nt = sweep_tile_count(D, a, k, g.n);
         for (long long t = 0; t < nt; ++t) sweep[a][k].push_back({i, a, t});
@@ -1647,7 +1654,9 @@ int batch_build(rhyme_gpu_batch* B) {
   L.n_faces = (int)faces.size();
   L.n_flux = (int)flux.size();
   L.n_update = (int)update.size();
+  L.fuse_xy = fuse;
   L.heads = B->heads;
+  L.whole = B->qblock + 3;
   return RHYME_GPU_OK;
 }
 
@@ -1723,7 +1732,13 @@ extern "C" int rhyme_gpu_batch_run(rhyme_gpu_batch* B, int nsteps) {
     if (rc != RHYME_GPU_OK) return rc;
   }
   B->runs++;
+  // the first CFL pass is whole if a box's state was last changed by
+  // something other than a batch run
+  bool whole = false;
+  for (int h : B->handles) whole = whole || !ctx->boxes[h]->batch_carry;
+  if (ctx->mixed && whole && nsteps > 0) CK(cudaMemsetAsync(B->qblock + 3, 1, sizeof(int), ctx->stream));
   for (int s = 0; s < nsteps; ++s) {
+    if (s == 1 && ctx->mixed && whole) CK(cudaMemsetAsync(B->qblock + 3, 0, sizeof(int), ctx->stream));
     if (B->graph[0])
       CK(cudaGraphLaunch(B->graph[B->k], ctx->stream));
     else
@@ -1735,7 +1750,9 @@ extern "C" int rhyme_gpu_batch_run(rhyme_gpu_batch* B, int nsteps) {
     Box* b = ctx->boxes[B->handles[i]];
     b->cur = B->base_cur[i] ^ B->k;
     if (nsteps > 0) state_changed(b);
+    if (nsteps > 0) b->batch_carry = true;
   }
+  if (ctx->mixed && whole && nsteps == 1) CK(cudaMemsetAsync(B->qblock + 3, 0, sizeof(int), ctx->stream));
   return RHYME_GPU_OK;
 }
 

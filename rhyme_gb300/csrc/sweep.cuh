@@ -439,7 +439,10 @@ __global__ void __launch_bounds__(TileCfg<S, P>::threads, TileCfg<S, P>::templat
 }
 
 // The same sweep over the tiles of a batch of boxes, taken from a work queue
-// (item.chunk = the tile's linear index tA + nA * (tB + nB * (cC - 1))).
+// (item.chunk = the tile's linear index tA + nA * (tB + nB * (cC - 1))): a
+// CTA's first item is its index, the head deals out the rest, and the atomic
+// for the next item is in flight while the current tile is swept. The last
+// sweep carries the boxes' CFL pass as the single box's does.
 template <int D, int A, int S, int P, int MODE>
 __global__ void __launch_bounds__(TileCfg<S, P>::threads, TileCfg<S, P>::template ctas<MODE>())
     batch_sweep_kernel(MixedParams M, const BoxDesc* __restrict__ TB, const WorkItem* __restrict__ items,
@@ -449,22 +452,29 @@ __global__ void __launch_bounds__(TileCfg<S, P>::threads, TileCfg<S, P>::templat
   __shared__ int s_item;
   unsigned parity = 0;
   const TmaStage tma{nullptr, 0, 0};
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_item = atomicAdd(head, 1);
-    __syncthreads();
-    const int it = s_item;
-    if (it >= n) break;
+  for (int it = blockIdx.x; it < n;) {
+    int next = 0;
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(head, 1);
     const WorkItem w = items[it];
     const BoxDesc& b = TB[w.box];
     const int nA = (b.g.n[A] + S - 1) / S;
     const int nB = ((B < D ? b.g.n[B] : 1) + P - 1) / P;
-    const int tA = (int)(w.chunk % nA);
-    const long long r = w.chunk / nA;
+    const unsigned chunk = (unsigned)w.chunk;
+    const int tA = (int)(chunk % nA);
+    const unsigned r = chunk / nA;
     const int tB = (int)(r % nB);
     const int cC = (int)(r / nB) + 1;
+    SweepCarry carry;
+    if (MODE == LAST || MODE == ONLY) {
+      carry.Uf_next = b.Uf_next;
+      carry.bits = carry_bits_of(b);
+      carry.status = (int*)(b.ctl + 2) + 1;
+    }
     sweep_tile<D, A, S, P, MODE>(M, b.limiter, b.omega_f, b.Uf, b.U, b.g, b.dx, b.ctl, b.acc, b.V,
-                                 q, w.box, tA, tB, cC, sh, tma, nullptr, parity);
+                                 q, w.box, tA, tB, cC, sh, tma, nullptr, parity, carry);
+    if (threadIdx.x == 0) s_item = next;
+    __syncthreads();
+    it = s_item;
   }
 }
 
@@ -500,27 +510,26 @@ struct XYSmem {
   float f[2][5][NI];                              // interface fluxes per axis (normal-first)
 };
 
+// One tile. map: the tensor map of the mirror's planes, or null: the plane is
+// staged with loads (batches, whose boxes may be smaller than the copy's
+// box). bar: the copy's barrier, in phase 0. `box` tags queued interfaces.
 template <int TX, int TY>
-__global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
-    sweep_xy_kernel(MixedParams M, Geom g, Dx dx, const double* __restrict__ dtp, float* __restrict__ acc,
-                    FallbackQueue q, const __grid_constant__ CUtensorMap map, int o_off) {
+__device__ __forceinline__ void sweep_xy_tile(const MixedParams& M, int limiter, float omega,
+                                              const float* __restrict__ Uf, const Geom& g, const Dx& dx,
+                                              const double* __restrict__ dtp, float* __restrict__ acc,
+                                              const FallbackQueue& q, int box, int x0, int y0, int cz,
+                                              XYSmem<TX, TY>& sh, const CUtensorMap* map, unsigned long long* bar) {
   using Cfg = XYCfg<TX, TY>;
   constexpr int NT = Cfg::threads;
   constexpr int PW = TX + 4;               // plane row
   constexpr int PL = (TX + 4) * (TY + 4);  // plane of one component
-  __shared__ XYSmem<TX, TY> sh;
-  __shared__ __align__(8) unsigned long long bar;
   __shared__ float s_dt[4];  // dt/dx, (0.5 dt)/dx, dt/dy, (0.5 dt)/dy
   const int NX = g.n[0], NY = g.n[1];
-  const int x0 = blockIdx.x * TX + 1, y0 = blockIdx.y * TY + 1;
-  const int cz = (int)blockIdx.z + 1;
   const long long F = g.field;
   float* su = sh.u;
-  if (threadIdx.x == 0) mbar_init(&bar);
-  __syncthreads();
   // 1. stage the plane: cells x0-2 .. x0+TX+1, y0-2 .. y0+TY+1 of plane cz
-  if (threadIdx.x == 0)
-    tma_load_4d(su, &map, x0 - 1, y0 - 1, cz + 1 + o_off, 0, &bar, (unsigned)(5 * PL * sizeof(float)));
+  if (map && threadIdx.x == 0)
+    tma_load_4d(su, map, x0 - 1, y0 - 1, cz + 1, 0, bar, (unsigned)(5 * PL * sizeof(float)));
   if (threadIdx.x == 32) {
     const float dt = __double2float_rn(*dtp);
     s_dt[0] = dt * dx.inv_f[0];
@@ -528,9 +537,23 @@ __global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
     s_dt[2] = dt * dx.inv_f[1];
     s_dt[3] = (0.5f * dt) * dx.inv_f[1];
   }
-  if (threadIdx.x < 32 && !mbar_wait(&bar, 0)) {
-    if (threadIdx.x == 0) atomicOr(q.status, kStatusTmaTimeout);
-    mbar_wait(&bar, 0);
+  if (map) {
+    if (threadIdx.x < 32 && !mbar_wait(bar, 0)) {
+      if (threadIdx.x == 0) atomicOr(q.status, kStatusTmaTimeout);
+      mbar_wait(bar, 0);
+    }
+  } else {
+    for (int it = threadIdx.x; it < PL; it += NT) {
+      const int px = it % PW, py = it / PW;
+      const int gx = x0 - 2 + px, gy = y0 - 2 + py;
+      const bool ok = gx <= NX + 2 && gy <= NY + 2;
+      const long long o = ok ? g.at(3, gx, gy, cz) : 0;
+      float v[5];
+#pragma unroll
+      for (int c = 0; c < 5; ++c) v[c] = ok ? Uf[(long long)c * F + o] : 0.f;
+#pragma unroll
+      for (int c = 0; c < 5; ++c) su[c * PL + it] = v[c];
+    }
   }
   __syncthreads();
 
@@ -563,7 +586,7 @@ __global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
       u0[k] = su[b + stride];
       up[k] = su[b + 2 * stride];
     }
-    face_states<3, 0>(M.G, M.limiter, M.omega, um, u0, up, s_dt[ax ? 3 : 1], l, r);
+    face_states<3, 0>(M.G, limiter, omega, um, u0, up, s_dt[ax ? 3 : 1], l, r);
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       sh.fl[ax][k][slot] = l[k];
@@ -618,7 +641,7 @@ __global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
           FallbackEntry& e = q.e[slot];
           e.axis = ax;
           e.ga = ga;
-          e.box = 0;
+          e.box = box;
           e.o = (ax ? g.at(3, x0 + lb, ga, cz) : g.at(3, ga, y0 + lb, cz)) + q.o_base;
         } else {
           atomicOr(q.status, 2);
@@ -644,6 +667,42 @@ __global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
       acc[(long long)c * F + o] =
           __fmaf_rn(s_dt[2], __fsub_rn(sh.f[1][ky][lv * TX + lu], sh.f[1][ky][(lv + 1) * TX + lu]), ax_);
     }
+  }
+}
+
+template <int TX, int TY>
+__global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
+    sweep_xy_kernel(MixedParams M, Geom g, Dx dx, const double* __restrict__ dtp, float* __restrict__ acc,
+                    FallbackQueue q, const __grid_constant__ CUtensorMap map) {
+  __shared__ XYSmem<TX, TY> sh;
+  __shared__ __align__(8) unsigned long long bar;
+  if (threadIdx.x == 0) mbar_init(&bar);
+  __syncthreads();
+  sweep_xy_tile<TX, TY>(M, M.limiter, M.omega, nullptr, g, dx, dtp, acc, q, 0, blockIdx.x * TX + 1,
+                        blockIdx.y * TY + 1, (int)blockIdx.z + 1, sh, &map, &bar);
+}
+
+// The tiles of a batch of boxes from a work queue, as batch_sweep_kernel
+// (item.chunk = tx + nx * (ty + ny * (z - 1))).
+template <int TX, int TY>
+__global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
+    batch_sweep_xy_kernel(MixedParams M, const BoxDesc* __restrict__ TB, const WorkItem* __restrict__ items, int n,
+                          int* head, FallbackQueue q) {
+  __shared__ XYSmem<TX, TY> sh;
+  __shared__ int s_item;
+  for (int it = blockIdx.x; it < n;) {
+    int next = 0;
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(head, 1);
+    const WorkItem w = items[it];
+    const BoxDesc& b = TB[w.box];
+    const unsigned nx = (unsigned)(b.g.n[0] + TX - 1) / TX, ny = (unsigned)(b.g.n[1] + TY - 1) / TY;
+    const unsigned chunk = (unsigned)w.chunk, r = chunk / nx;
+    sweep_xy_tile<TX, TY>(M, b.limiter, b.omega_f, b.Uf, b.g, b.dx, b.ctl, b.acc, q, w.box,
+                          (int)(chunk - r * nx) * TX + 1, (int)(r % ny) * TY + 1, (int)(r / ny) + 1, sh, nullptr,
+                          nullptr);
+    if (threadIdx.x == 0) s_item = next;
+    __syncthreads();
+    it = s_item;
   }
 }
 

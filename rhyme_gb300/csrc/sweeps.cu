@@ -2,6 +2,7 @@
 // one dimensionality. Compiled three times (-DSWEEP_D=1, 2, 3) so the
 // instantiations (axes x candidate shapes, single box and batched) build in
 // parallel.
+#include <algorithm>
 #include <cstring>
 
 #include "sweep.cuh"
@@ -70,8 +71,8 @@ cudaError_t launch_batch_one(const MixedParams& M, const BoxDesc* TB, const Work
                              const FallbackQueue& q, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   constexpr int MODE = mode_of<D, A>();
-  batch_sweep_kernel<D, A, S, P, MODE><<<152 * TileCfg<S, P>::template ctas<MODE>(), TileCfg<S, P>::threads, 0, st>>>(
-      M, TB, items, n, head, q);
+  const int grid = std::min(n, 152 * TileCfg<S, P>::template ctas<MODE>());
+  batch_sweep_kernel<D, A, S, P, MODE><<<grid, TileCfg<S, P>::threads, 0, st>>>(M, TB, items, n, head, q);
   return cudaGetLastError();
 }
 
@@ -168,8 +169,28 @@ cudaError_t launch_sweep_xy_3(const MixedParams& M, const float* Uf, const Geom&
   memset(&map, 0, sizeof map);
   if (!encode_xy_map(&map, Uf, g, TX, TY)) return cudaErrorNotSupported;
   sweep_xy_kernel<TX, TY><<<dim3(gx, gy, (unsigned)g.n[2]), XYCfg<TX, TY>::threads, 0, st>>>(M, g, dx, dtp, acc, q,
-                                                                                             map, 0);
+                                                                                             map);
   return cudaGetLastError();
+}
+
+namespace {
+template <int TX, int TY>
+cudaError_t launch_batch_xy(const MixedParams& M, const BoxDesc* TB, const WorkItem* items, int n, int* head,
+                            const FallbackQueue& q, cudaStream_t st) {
+  using Cfg = XYCfg<TX, TY>;
+  batch_sweep_xy_kernel<TX, TY><<<std::min(n, 152 * Cfg::ctas), Cfg::threads, 0, st>>>(M, TB, items, n, head, q);
+  return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_batch_sweep_xy_3(int shape, const MixedParams& M, const BoxDesc* TB, const WorkItem* items, int n,
+                                    int* head, const FallbackQueue& q, cudaStream_t st) {
+  switch (shape) {
+    case 0: return launch_batch_xy<8, 32>(M, TB, items, n, head, q, st);
+    case 1: return launch_batch_xy<16, 16>(M, TB, items, n, head, q, st);
+    case 2: return launch_batch_xy<32, 8>(M, TB, items, n, head, q, st);
+  }
+  return cudaErrorInvalidValue;
 }
 #endif
 

@@ -110,3 +110,41 @@ def test_batch_survives_single_steps_in_between():
     for i, (cells, dx, p) in enumerate(items):
         ref, _ = _alone(p, cells, dx, 5 if i == 1 else 4)
         assert np.array_equal(states[i], ref), i
+
+
+@pytest.mark.parametrize("dims", [(1, 9, 4), (33, 7, 3), (16, 16, 2), (17, 15, 1), (40, 24, 5), (8, 33, 6), (3, 2, 2)])
+def test_mixed_batch_of_odd_boxes_equals_alone(dims):
+    """Tiles of every shape of the fused x and y sweep with remainders, the
+    carried CFL over runs of uneven length, a box stepped alone in between
+    (the next batch step's CFL is then whole): states and dts bit for bit."""
+    rng = np.random.default_rng(sum(dims))
+    items = []
+    for d in (dims, dims[::-1], (12, 20, 9)):
+        cells = ic.empty_box(3, list(d))
+        shp = tuple(d[::-1])
+        vel = [0.2 * rng.uniform(-1, 1, shp) for _ in range(3)]
+        cells[ic.interior(3, list(d))] = ic.prim_to_cons(1.0 + 0.3 * rng.uniform(size=shp), vel,
+                                                         1.0 + 0.3 * rng.uniform(size=shp), 5.0 / 3.0)
+        bc = [int(rng.choice([REFLECTIVE, OUTFLOW])) for _ in range(6)]
+        items.append((cells, [1.0 / 20] * 3, hydro_params(3, limiter=int(rng.integers(1, 5)), bc=bc, courant=0.2,
+                                                          precision=MIXED)))
+    states = [c.copy() for c, _, _ in items]
+    with gpu.Context(items[0][2]) as ctx:
+        boxes = []
+        for st, (_, _, p) in zip(states, items):
+            boxes.append(ctx.register_box(st))
+            ctx.set_box_params(boxes[-1], bc=p["bc"], limiter=p["limiter"])
+        with ctx.batch(boxes, [dx for _, dx, _ in items]) as bt:
+            bt.run(1)
+            bt.run(3)
+            ctx.run(boxes[1], items[1][1], 2)
+            bt.run(2)
+            dts = bt.dts()
+        redone = [ctx.fallback_count(b) for b in boxes]
+        for b in boxes:
+            ctx.sync_to_host(b)
+    assert redone == [0, 0, 0]
+    for i, (cells, dx, p) in enumerate(items):
+        ref, dt = _alone(p, cells, dx, 8 if i == 1 else 6)
+        assert np.array_equal(states[i], ref), i
+        assert dts[i] == dt
