@@ -50,7 +50,7 @@ __host__ __device__ inline long long ghost_lines(int D, const Geom& g, int axis)
 // A plane holds fewer than 2^32 lines (the array would not fit otherwise),
 // so the position is split in 32 bits.
 template <int D, typename T>
-__device__ __forceinline__ void ghost_line(const BoxRules& R, T* __restrict__ U, T* __restrict__ M, const Geom& g,
+__device__ __forceinline__ void ghost_line(const int* bc, const double (*inflow)[5], T* __restrict__ U, T* __restrict__ M, const Geom& g,
                                            int axis, int c, unsigned q, float* __restrict__ Mf) {
   const unsigned n1 = (D == 1) ? 1u : (unsigned)g.n[axis == 0 ? 1 : 0];
   unsigned i2 = 0, i1 = q;
@@ -69,14 +69,14 @@ __device__ __forceinline__ void ghost_line(const BoxRules& R, T* __restrict__ U,
   float* mf = Mf ? Mf + (long long)c * g.field : nullptr;
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
-    const int type = R.bc[2 * axis + side];
+    const int type = bc[2 * axis + side];
     if (type < 1 || type > 4) continue;  // the caller fills this face
     const bool far = (type == 3) != (side == 1);  // the sources lie at the line's other end
     const long long g0 = side ? base + (N + 1) * sa : base, g1 = side ? g0 + sa : g0 - sa;
     const long long s0 = far ? base + N * sa : base + sa, s1 = far ? s0 - sa : s0 + sa;
     T v0, v1;
     if (type == 4) {  // inflow
-      v0 = v1 = (T)R.inflow[2 * axis + side][c];
+      v0 = v1 = (T)inflow[2 * axis + side][c];
     } else {
       v0 = f[s0];
       v1 = (s1 == g0) ? v0 : f[s1];  // a periodic line of one cell: the first ghost is the second's source

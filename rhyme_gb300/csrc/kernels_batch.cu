@@ -84,12 +84,7 @@ __global__ void __launch_bounds__(256)
     const int axis = w.axis / (D + 2), c = w.axis % (D + 2);
     const long long q = w.chunk * kBatchChunk + threadIdx.x;
     if (q >= ghost_lines(D, b.g, axis)) continue;
-    BoxRules R;
-    for (int i = 0; i < 6; ++i) {
-      R.bc[i] = b.bc[i];
-      for (int k = 0; k < 5; ++k) R.inflow[i][k] = b.inflow[i][k];
-    }
-    ghost_line<D, double>(R, b.U, b.V, b.g, axis, c, (unsigned)q, b.Uf);
+    ghost_line<D, double>(b.bc, b.inflow, b.U, b.V, b.g, axis, c, (unsigned)q, b.Uf);
   }
 }
 
@@ -172,6 +167,12 @@ __global__ void __launch_bounds__(256)
 }
 
 template <int D>
+cudaError_t batch_ghosts_d(const BoxDesc* TB, const BatchLists& L, cudaStream_t st) {
+  if (L.n_ghost) batch_ghost_kernel<D><<<std::min(L.n_ghost, 152 * 8), 256, 0, st>>>(TB, L.ghost, L.n_ghost);
+  return cudaGetLastError();
+}
+
+template <int D>
 cudaError_t batch_step_d(const DevParams& P, const MixedParams& M, bool mixed, const BoxDesc* TB,
                          const BatchLists& L, FallbackQueue q, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(L.heads, 0, kBatchHeads * sizeof(int), st);
@@ -182,8 +183,7 @@ cudaError_t batch_step_d(const DevParams& P, const MixedParams& M, bool mixed, c
   } else if (L.n_cfl) {
     batch_cfl_kernel<D><<<std::min(L.n_cfl, 152 * 4), 256, 0, st>>>(P.G, P.courant, TB, L.cfl, L.n_cfl);
   }
-  if (L.n_ghost) batch_ghost_kernel<D><<<std::min(L.n_ghost, 152 * 8), 256, 0, st>>>(TB, L.ghost, L.n_ghost);
-  e = cudaGetLastError();
+  if (L.fill_each) e = batch_ghosts_d<D>(TB, L, st);
   if (e != cudaSuccess) return e;
   if (mixed) return launch_batch_sweeps(M, TB, L, q, st);
   if (L.n_faces) batch_faces_kernel<D><<<std::min(L.n_faces, 152 * 8), 128, 0, st>>>(P.G, TB, L.faces, L.n_faces);
@@ -194,6 +194,15 @@ cudaError_t batch_step_d(const DevParams& P, const MixedParams& M, bool mixed, c
 }
 
 }  // namespace
+
+cudaError_t launch_batch_ghosts(int ndim, const BoxDesc* table, const BatchLists& L, cudaStream_t st) {
+  switch (ndim) {
+    case 1: return batch_ghosts_d<1>(table, L, st);
+    case 2: return batch_ghosts_d<2>(table, L, st);
+    case 3: return batch_ghosts_d<3>(table, L, st);
+  }
+  return cudaErrorInvalidValue;
+}
 
 cudaError_t launch_batch_step(const DevParams& P, const MixedParams& M, bool mixed, int ndim,
                               const BoxDesc* table, const BatchLists& L, FallbackQueue q,

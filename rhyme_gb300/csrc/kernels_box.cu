@@ -50,11 +50,11 @@ inline int grid_for(long long total, int block) {
 // array holds after the fill. Bound by the scattered sectors of the x faces.
 template <int D, typename T>
 __global__ void __launch_bounds__(kFillBlock)
-    ghost_fill_kernel(BoxRules R, T* __restrict__ U, T* __restrict__ M, Geom g, float* __restrict__ Mf) {
+    ghost_fill_kernel(const __grid_constant__ BoxRules R, T* __restrict__ U, T* __restrict__ M, Geom g, float* __restrict__ Mf) {
   const int axis = blockIdx.y / (D + 2), c = blockIdx.y % (D + 2);
   const long long n = ghost_lines(D, g, axis);
   for (long long q = (long long)blockIdx.x * kFillBlock + threadIdx.x; q < n; q += (long long)gridDim.x * kFillBlock)
-    ghost_line<D, T>(R, U, M, g, axis, c, (unsigned)q, Mf);
+    ghost_line<D, T>(R.bc, R.inflow, U, M, g, axis, c, (unsigned)q, Mf);
 }
 
 // ------------------------------------------------------------------ K2 ---

@@ -309,22 +309,33 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // FP64 flux of the interface between cell o (index ga along AX) and cell
-// o + s_AX, from U^n: face states of both cells (cells ga-1 .. ga+2, the
-// ghost layer included) and the exact Riemann problem at x/t = 0.
+// o + s_AX, from U^n: face states of both cells (cells ga-1 .. ga+2, those
+// beyond a face of bc type 1..4 from the interior, as the sweeps take them)
+// and the exact Riemann problem at x/t = 0. bc: null where every ghost cell
+// is in memory.
 template <int D, int AX>
 __device__ __noinline__ void redo_interface(const MixedParams& M, int limiter, double omega,
-                                            const double* __restrict__ U, const Geom& g, long long o,
-                                            double hdtdx, double* f) {
+                                            const double* __restrict__ U, const Geom& g, int ga, long long o,
+                                            const int* bc, const double (*inflow)[5], double hdtdx, double* f) {
   const long long F = g.field, sa = g.s[AX];
+  const int N = g.n[AX];
   double w0[D + 2], w1[D + 2], w2[D + 2], w3[D + 2];
+  auto cell = [&](int k, double* w) {  // cell ga + k
+    const int i = ga + k;
+    const int side = 2 * AX + (i < 1 ? 0 : 1);
+    const int type = (bc && (i < 1 || i > N)) ? bc[side] : 0;
+    const bool from = type >= 1 && type <= 4;
+    const long long at = o + (long long)((from && type != 4 ? ghost_source(i, N, type) : i) - ga) * sa;
 #pragma unroll
-  for (int c = 0; c < D + 2; ++c) {
-    const double* p = U + (long long)c * F + o;
-    w0[c] = p[-sa];
-    w1[c] = p[0];
-    w2[c] = p[sa];
-    w3[c] = p[2 * sa];
-  }
+    for (int c = 0; c < D + 2; ++c) {
+      w[c] = (type == 4) ? inflow[side][c] : U[(long long)c * F + at];
+      if (type == 1 && c == 1 + AX) w[c] = -w[c];
+    }
+  };
+  cell(-1, w0);
+  cell(0, w1);
+  cell(1, w2);
+  cell(2, w3);
   // a non-finite U^n (a box the scheme has already lost) makes the FP64
   // solve iterate to its cap for a NaN result: give the NaN directly
   bool finite = true;
@@ -343,16 +354,24 @@ __device__ __noinline__ void redo_interface(const MixedParams& M, int limiter, d
 
 template <int D>
 __device__ __forceinline__ void redo_any_axis(const MixedParams& M, int limiter, double omega,
-                                              const double* __restrict__ U, const Geom& g, int axis,
-                                              long long o, double hdtdx, double* f) {
-  if (axis == 0) redo_interface<D, 0>(M, limiter, omega, U, g, o, hdtdx, f);
+                                              const double* __restrict__ U, const Geom& g,
+                                              const FallbackEntry& e, const int* bc, const double (*inflow)[5],
+                                              double hdtdx, double* f) {
+  const int axis = e.axis;
+  if (axis == 0) redo_interface<D, 0>(M, limiter, omega, U, g, e.ga, e.o, bc, inflow, hdtdx, f);
   if constexpr (D > 1) {
-    if (axis == 1) redo_interface<D, 1>(M, limiter, omega, U, g, o, hdtdx, f);
+    if (axis == 1) redo_interface<D, 1>(M, limiter, omega, U, g, e.ga, e.o, bc, inflow, hdtdx, f);
   }
   if constexpr (D > 2) {
-    if (axis == 2) redo_interface<D, 2>(M, limiter, omega, U, g, o, hdtdx, f);
+    if (axis == 2) redo_interface<D, 2>(M, limiter, omega, U, g, e.ga, e.o, bc, inflow, hdtdx, f);
   }
 }
+
+// Boundary types and inflow values for the fix-up (types 0: from memory).
+struct FixBC {
+  int bc[6];
+  double inflow[6][5];
+};
 
 // FP64 redo of the queued interfaces; -+ dt/dx * F applied to the adjacent
 // interior cells of U^{n+1} (atomically: a cell can border two queued
@@ -362,7 +381,8 @@ __device__ __forceinline__ void redo_any_axis(const MixedParams& M, int limiter,
 template <int D>
 __global__ void __launch_bounds__(128)
     fallback_fix_kernel(MixedParams M, FallbackQueue q, Geom g, Dx dx, const double* __restrict__ dtp,
-                        const double* __restrict__ U, double* __restrict__ Unew, const int* __restrict__ from) {
+                        const double* __restrict__ U, double* __restrict__ Unew, const int* __restrict__ from,
+                        const __grid_constant__ FixBC fbc) {
   const int n = min(*q.n, q.cap);
   const int lo = from ? min(*from, n) : 0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && n > lo) atomicAdd(q.total, n - lo);
@@ -371,7 +391,7 @@ __global__ void __launch_bounds__(128)
   for (int i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const FallbackEntry e = q.e[i];
     double f[D + 2];
-    redo_any_axis<D>(M, M.limiter, M.omega64, U, g, e.axis, e.o, 0.5 * dt / dx.v[e.axis], f);
+    redo_any_axis<D>(M, M.limiter, M.omega64, U, g, e, fbc.bc, fbc.inflow, 0.5 * dt / dx.v[e.axis], f);
     const double dtdx = dt / dx.v[e.axis];
     const long long sa = g.s[e.axis];
     const int NA = g.n[e.axis];
@@ -387,8 +407,13 @@ __global__ void __launch_bounds__(128)
 template <int D>
 cudaError_t launch_fallback(const MixedParams& M, const FallbackQueue& q, const Geom& g, const Dx& dx,
                             const double* dtp, const double* U, double* Unew, cudaStream_t st,
-                            const int* from = nullptr) {
-  fallback_fix_kernel<D><<<152, 128, 0, st>>>(M, q, g, dx, dtp, U, Unew, from);
+                            const HaloBC& halo, const int* from = nullptr) {
+  FixBC fbc;
+  for (int i = 0; i < 6; ++i) {
+    fbc.bc[i] = halo.type[i];
+    for (int c = 0; c < 5; ++c) fbc.inflow[i][c] = halo.inflow64[i][c];
+  }
+  fallback_fix_kernel<D><<<152, 128, 0, st>>>(M, q, g, dx, dtp, U, Unew, from, fbc);
   return cudaGetLastError();
 }
 
@@ -475,7 +500,7 @@ __global__ void __launch_bounds__(128)
     const BoxDesc& b = TB[e.box];
     *carry_ok_of(b) = 0;  // the box's cells change after its last sweep: its next CFL pass is whole
     double f[D + 2];
-    redo_any_axis<D>(M, b.limiter, b.omega, b.U, b.g, e.axis, e.o, 0.5 * b.ctl[0] / b.dx.v[e.axis], f);
+    redo_any_axis<D>(M, b.limiter, b.omega, b.U, b.g, e, b.halo.type, b.inflow, 0.5 * b.ctl[0] / b.dx.v[e.axis], f);
     const double dtdx = b.ctl[0] / b.dx.v[e.axis];
     const long long sa = b.g.s[e.axis];
     const int NA = b.g.n[e.axis];
@@ -541,7 +566,7 @@ cudaError_t launch_cfl_carry(const MixedParams& M, const double* U, float* Uf, c
 cudaError_t launch_mh_solve_mixed(const MixedParams& M, const double* U, const float* Uf,
                                   double* Unew, float* acc, const Geom& g,
                                   const Dx& dx, const StepScratch& s, const FallbackQueue& q,
-                                  const SweepPlan& plan, cudaStream_t st, cudaEvent_t* ev,
+                                  const SweepPlan& plan, cudaStream_t st, const HaloBC& halo, cudaEvent_t* ev,
                                   const SweepCarry& carry, int* fused) {
   // ev (optional, 3 events): recorded after the x sweep, after the y sweep
   // and at the end (the z sweep and the FP64 fix-up); absent axes record
@@ -555,7 +580,7 @@ cudaError_t launch_mh_solve_mixed(const MixedParams& M, const double* U, const f
   if (e == cudaSuccess && D == 3 && plan.fuse_xy) {
     // the x and y sweeps in one kernel where the mirror's rows allow the
     // plane's tensor copy (bit-identical to the two sweeps)
-    e = launch_sweep_xy_3(M, Uf, g, dx, s.dt, acc, q, st);
+    e = launch_sweep_xy_3(M, Uf, g, dx, s.dt, acc, q, halo, st);
     if (e == cudaSuccess) {
       first = 2;
       if (fused) *fused = 1;
@@ -568,16 +593,16 @@ cudaError_t launch_mh_solve_mixed(const MixedParams& M, const double* U, const f
   for (int a = first; a < D; ++a) {
     if (e == cudaSuccess)
       e = launch_sweep_axis(D, a, plan.shape[a], M, Uf, U, g, dx, s.dt, acc, Unew, q, st,
-                            a == D - 1 ? carry : SweepCarry());
+                            a == D - 1 ? carry : SweepCarry(), halo);
     if (e == cudaSuccess && ev && a < 2) e = cudaEventRecord(ev[a], st);
   }
   for (int a = D; a < 2; ++a)
     if (e == cudaSuccess && ev) e = cudaEventRecord(ev[a], st);
   if (e == cudaSuccess) {
     switch (D) {
-      case 1: e = launch_fallback<1>(M, q, g, dx, s.dt, U, Unew, st); break;
-      case 2: e = launch_fallback<2>(M, q, g, dx, s.dt, U, Unew, st); break;
-      case 3: e = launch_fallback<3>(M, q, g, dx, s.dt, U, Unew, st); break;
+      case 1: e = launch_fallback<1>(M, q, g, dx, s.dt, U, Unew, st, halo); break;
+      case 2: e = launch_fallback<2>(M, q, g, dx, s.dt, U, Unew, st, halo); break;
+      case 3: e = launch_fallback<3>(M, q, g, dx, s.dt, U, Unew, st, halo); break;
     }
   }
   if (e == cudaSuccess && ev) e = cudaEventRecord(ev[2], st);
@@ -595,9 +620,9 @@ cudaError_t launch_mh_solve_mixed_slab(const MixedParams& M, const double* U, co
     e = launch_sweep_slab(D, a, plan.shape[a], M, Uf, U, g, dx, s.dt, acc, Unew, q, lo, hi, st);
   if (e == cudaSuccess) {
     switch (D) {
-      case 1: e = launch_fallback<1>(M, q, g, dx, s.dt, U, Unew, st, done); break;
-      case 2: e = launch_fallback<2>(M, q, g, dx, s.dt, U, Unew, st, done); break;
-      case 3: e = launch_fallback<3>(M, q, g, dx, s.dt, U, Unew, st, done); break;
+      case 1: e = launch_fallback<1>(M, q, g, dx, s.dt, U, Unew, st, no_halo(), done); break;
+      case 2: e = launch_fallback<2>(M, q, g, dx, s.dt, U, Unew, st, no_halo(), done); break;
+      case 3: e = launch_fallback<3>(M, q, g, dx, s.dt, U, Unew, st, no_halo(), done); break;
     }
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(done, q.n, sizeof(int), cudaMemcpyDeviceToDevice, st);

@@ -4,6 +4,10 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <cfloat>
+#include <cmath>
+#include <cstring>
+
 #include "hydro.cuh"
 
 namespace rgpu {
@@ -252,6 +256,50 @@ struct SweepCarry {
   int* status = nullptr;
 };
 
+// The boundary rules as the mixed sweeps apply them: a face of type 1..4
+// (reflective, outflow, periodic, inflow) gives its two ghost layers from
+// the interior while a tile is staged, so a resident run does not fill the
+// ghost cells of its intermediate states in memory (the scattered sectors of
+// the x faces made that fill 5 % of a 256^3 step, 12 % of a 64^3 one and 22 %
+// of a batch of small boxes); it fills them once after its last step. Type
+// 0: the array's own ghost cells are read. Boxes with an extent of one cell
+// keep filling every step (their ghosts depend on earlier ghosts).
+struct HaloBC {
+  int type[6];
+  float inflow[6][5];     // the mirror's values
+  double inflow64[6][5];  // the FP64 fix-up's
+};
+
+inline HaloBC no_halo() {
+  HaloBC h;
+  memset(&h, 0, sizeof h);
+  return h;
+}
+inline bool halo_from_interior(int D, const Geom& g) {
+  for (int a = 0; a < D; ++a)
+    if (g.n[a] < 2) return false;
+  return true;
+}
+inline HaloBC make_halo(int D, const Geom& g, const int* bc, const double (*inflow)[5]) {
+  HaloBC h = no_halo();
+  if (!halo_from_interior(D, g)) return h;
+  for (int f = 0; f < 2 * D; ++f) {
+    h.type[f] = (bc[f] >= 1 && bc[f] <= 4) ? bc[f] : 0;
+    for (int c = 0; c < 5; ++c) {
+      const float v = (float)inflow[f][c];  // mirror_of
+      h.inflow[f][c] = (std::fabs(v) < FLT_MIN) ? std::copysign(0.f, v) : v;
+      h.inflow64[f][c] = inflow[f][c];
+    }
+  }
+  return h;
+}
+// The interior cell that ghost cell i (-1, 0, N+1 or N+2) of a face of type
+// 1..3 copies (rhyme_samr_bc_set_*_boundary.f90).
+__host__ __device__ inline int ghost_source(int i, int N, int type) {
+  if (i < 1) return type == 3 ? i + N : 1 - i;
+  return type == 3 ? i - N : 2 * N + 1 - i;
+}
+
 // Mixed-precision launchers (kernels_mixed.cu).
 cudaError_t launch_to_f32(const double* U, float* Uf, long long n, cudaStream_t st);
 // The CFL of a step whose previous step carried the pass: when *carry_ok and
@@ -269,14 +317,16 @@ cudaError_t launch_cfl_mixed(const MixedParams& M, const double* U, float* Uf, c
 cudaError_t launch_mh_solve_mixed(const MixedParams& M, const double* U, const float* Uf,
                                   double* Unew, float* acc, const Geom& g,
                                   const Dx& dx, const StepScratch& s, const FallbackQueue& q,
-                                  const SweepPlan& plan, cudaStream_t st, cudaEvent_t* ev = nullptr,
-                                  const SweepCarry& carry = SweepCarry(), int* fused = nullptr);
+                                  const SweepPlan& plan, cudaStream_t st, const HaloBC& halo,
+                                  cudaEvent_t* ev = nullptr, const SweepCarry& carry = SweepCarry(),
+                                  int* fused = nullptr);
 // The x and y sweeps of a 3-D box as one kernel (sweeps.cu, sweep_xy_kernel):
 // cudaErrorNotSupported where its tensor copy cannot be used (rows of the
 // mirror not a multiple of 16 bytes, the encoder unavailable, too many tiles);
 // the caller then runs the two sweeps.
 cudaError_t launch_sweep_xy_3(const MixedParams& M, const float* Uf, const Geom& g, const Dx& dx,
-                              const double* dtp, float* acc, const FallbackQueue& q, cudaStream_t st);
+                              const double* dtp, float* acc, const FallbackQueue& q, const HaloBC& halo,
+                              cudaStream_t st);
 // The tensor map of sweep_xy_kernel's plane copies (kernels_mixed.cu).
 bool encode_xy_map(CUtensorMap* out, const float* Uf, const Geom& g, int TX, int TY);
 cudaError_t launch_ghost_fill_f32(const DevParams& P, float* Uf, const Geom& g, cudaStream_t st);
@@ -323,6 +373,7 @@ struct BoxDesc {
   int bc[6];
   double inflow[6][5];
   int cfl_items;  // CFL work items of this box (last one finishes dt)
+  HaloBC halo;    // mixed: as the sweeps apply them (types 0: ghosts read from memory)
 };
 
 // A work item: `chunk` of pass `axis` of box `box` (or a sweep tile).
@@ -349,6 +400,7 @@ struct BatchLists {
   bool fuse_xy;  // 3-D mixed: sweep[0] holds the tiles of the fused x and y sweep, by tile shape
   int* heads;  // one queue head per pass (kBatchHeads, reset before each step)
   const int* whole;  // nonzero: the step's CFL pass is whole for every box (mixed)
+  bool fill_each;    // ghosts filled in memory every step (FP64, or a box of one cell's extent)
 };
 
 // Tiles of the fused x and y sweep of a batch: 8 x 32, 16 x 16 or 32 x 8
@@ -387,7 +439,7 @@ long long sweep_tile_count(int ndim, int axis, int shape, const int* n);
   cudaError_t launch_sweep_axis_##D(int axis, int shape, const MixedParams& M, const float* Uf,         \
                                     const double* U, const Geom& g, const Dx& dx, const double* dtp,    \
                                     float* acc, double* Unew, const FallbackQueue& q, int lo, int hi,   \
-                                    cudaStream_t st, const SweepCarry& carry);                          \
+                                    cudaStream_t st, const SweepCarry& carry, const HaloBC& halo);      \
   cudaError_t launch_batch_sweep_axis_##D(int axis, int shape, const MixedParams& M, const BoxDesc* TB, \
                                           const WorkItem* items, int n, int* head, const FallbackQueue& q, \
                                           cudaStream_t st);
@@ -399,11 +451,12 @@ RGPU_SWEEP_DECL(3)
 inline cudaError_t launch_sweep_slab(int ndim, int axis, int shape, const MixedParams& M, const float* Uf,
                                      const double* U, const Geom& g, const Dx& dx, const double* dtp,
                                      float* acc, double* Unew, const FallbackQueue& q, int lo, int hi,
-                                     cudaStream_t st, const SweepCarry& carry = SweepCarry()) {
+                                     cudaStream_t st, const SweepCarry& carry = SweepCarry(),
+                                     const HaloBC& halo = no_halo()) {
   switch (ndim) {
-    case 1: return launch_sweep_axis_1(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
-    case 2: return launch_sweep_axis_2(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
-    case 3: return launch_sweep_axis_3(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
+    case 1: return launch_sweep_axis_1(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+    case 2: return launch_sweep_axis_2(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+    case 3: return launch_sweep_axis_3(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -412,9 +465,10 @@ inline cudaError_t launch_sweep_slab(int ndim, int axis, int shape, const MixedP
 inline cudaError_t launch_sweep_axis(int ndim, int axis, int shape, const MixedParams& M, const float* Uf,
                                      const double* U, const Geom& g, const Dx& dx, const double* dtp,
                                      float* acc, double* Unew, const FallbackQueue& q, cudaStream_t st,
-                                     const SweepCarry& carry = SweepCarry()) {
+                                     const SweepCarry& carry = SweepCarry(), const HaloBC& halo = no_halo()) {
   if (ndim < 1 || ndim > 3) return cudaErrorInvalidValue;
-  return launch_sweep_slab(ndim, axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, 1, g.n[ndim - 1], st, carry);
+  return launch_sweep_slab(ndim, axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, 1, g.n[ndim - 1], st, carry,
+                           halo);
 }
 
 inline cudaError_t launch_batch_sweep_axis(int ndim, int axis, int shape, const MixedParams& M,
@@ -435,6 +489,8 @@ cudaError_t launch_batch_cfl_mixed(const MixedParams& M, double courant, const B
                                    const BatchLists& L, cudaStream_t st);
 cudaError_t launch_batch_sweeps(const MixedParams& M, const BoxDesc* TB, const BatchLists& L,
                                 const FallbackQueue& q, cudaStream_t st);
+// The ghost fill of a batch's boxes (kernels_batch.cu), from table.U.
+cudaError_t launch_batch_ghosts(int ndim, const BoxDesc* table, const BatchLists& L, cudaStream_t st);
 cudaError_t launch_batch_step(const DevParams& P, const MixedParams& M, bool mixed, int ndim,
                               const BoxDesc* table, const BatchLists& L, FallbackQueue q,
                               cudaStream_t st);

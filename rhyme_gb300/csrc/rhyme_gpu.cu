@@ -800,6 +800,20 @@ SweepCarry carry_of(Box* b, int cur) {
   return c;
 }
 
+// A resident mixed run's steps take their ghost cells from the interior
+// (HaloBC) and its end fills them in memory, in both state buffers, from the
+// last step's U^n: what the fill before every solve leaves behind.
+bool fills_last(const rhyme_gpu_ctx* ctx, const Box* b) {
+  return ctx->mixed && halo_from_interior(ctx->params.ndim, b->g);
+}
+HaloBC box_halo(const rhyme_gpu_ctx* ctx, const Box* b) {
+  return make_halo(ctx->params.ndim, b->g, b->dp.bc, b->dp.inflow);
+}
+cudaError_t fill_after_run(rhyme_gpu_ctx* ctx, Box* b) {
+  if (!fills_last(ctx, b)) return cudaSuccess;
+  return launch_ghost_fill(b->dp, b->state[1 - b->cur], b->state[b->cur], b->g, ctx->stream);
+}
+
 // In mixed precision the step carries its CFL pass into the next one: the
 // next step's CFL pass only forms dt from the carried maximum (unless the
 // FP64 fix-up changed cells after the sweep; launch_cfl_carry).
@@ -810,11 +824,12 @@ cudaError_t enqueue_step(rhyme_gpu_ctx* ctx, Box* b, int cur, const Dx& dx, bool
   cudaError_t e = ctx->mixed ? launch_cfl_carry(b->mp, U, b->Uf[cur], b->g, b->dp.courant, dx, s, b->carry_bits,
                                                 b->carry_ok, b->fbq.n, ctx->stream)
                              : launch_cfl(b->dp, U, b->g, dx, s, ctx->stream);
-  if (e == cudaSuccess) e = launch_ghost_fill(b->dp, U, V, b->g, ctx->stream, ctx->mixed ? b->Uf[cur] : nullptr);
+  if (e == cudaSuccess && !fills_last(ctx, b))
+    e = launch_ghost_fill(b->dp, U, V, b->g, ctx->stream, ctx->mixed ? b->Uf[cur] : nullptr);
   if (e != cudaSuccess) return e;
   if (ctx->mixed)
     return launch_mh_solve_mixed(b->mp, U, b->Uf[cur], V, b->acc, b->g, dx, s, b->fbq, b->plan, ctx->stream,
-                                 nullptr, carry_of(b, cur));
+                                 box_halo(ctx, b), nullptr, carry_of(b, cur));
   return launch_mh_solve(b->dp, U, V, b->g, dx, s, ctx->stream);
 }
 
@@ -959,7 +974,7 @@ int rhyme_gpu_mh_solve(rhyme_gpu_ctx* ctx, int handle, const double dx[3], doubl
       written_back = true;
     } else {
       CK(launch_mh_solve_mixed(b->mp, b->state[b->cur], b->Uf[b->cur], b->state[1 - b->cur], b->acc, b->g, d,
-                               scratch_of(b, false), b->fbq, b->plan, ctx->stream));
+                               scratch_of(b, false), b->fbq, b->plan, ctx->stream, no_halo()));
     }
   }
   else
@@ -996,6 +1011,7 @@ int rhyme_gpu_run(rhyme_gpu_ctx* ctx, int handle, const double dx[3], int nsteps
       CK(cudaGraphLaunch(b->graph[b->cur], ctx->stream));
       b->cur = 1 - b->cur;
     }
+    if (done + chunk == nsteps) CK(fill_after_run(ctx, b));
     if (dt_trace) {
       CK(cudaMemcpyAsync(dt_trace + done, b->trace_buf, sizeof(double) * chunk, cudaMemcpyDeviceToHost,
                          ctx->stream));
@@ -1148,11 +1164,12 @@ extern "C" int rhyme_gpu_profile_steps(rhyme_gpu_ctx* ctx, int handle, const dou
         e = launch_cfl_carry(b->mp, U, b->Uf[b->cur], b->g, b->dp.courant, d, sc, b->carry_bits, b->carry_ok,
                              b->fbq.n, ctx->stream);
       if (e == cudaSuccess) e = cudaEventRecord(ev[1], ctx->stream);
-      if (e == cudaSuccess) e = launch_ghost_fill(b->dp, U, V, b->g, ctx->stream, b->Uf[b->cur]);
+      if (e == cudaSuccess && !fills_last(ctx, b))
+        e = launch_ghost_fill(b->dp, U, V, b->g, ctx->stream, b->Uf[b->cur]);
       if (e == cudaSuccess) e = cudaEventRecord(ev[2], ctx->stream);
       if (e == cudaSuccess)
         e = launch_mh_solve_mixed(b->mp, U, b->Uf[b->cur], V, b->acc, b->g, d, sc,
-                                  b->fbq, b->plan, ctx->stream, ev + 3, carry_of(b, b->cur), &fused);
+                                  b->fbq, b->plan, ctx->stream, box_halo(ctx, b), ev + 3, carry_of(b, b->cur), &fused);
     } else {
       if (e == cudaSuccess) e = launch_cfl(b->dp, U, b->g, d, sc, ctx->stream);
       if (e == cudaSuccess) e = cudaEventRecord(ev[1], ctx->stream);
@@ -1173,6 +1190,7 @@ extern "C" int rhyme_gpu_profile_steps(rhyme_gpu_ctx* ctx, int handle, const dou
     }
   }
   for (int i = 0; i < 6; ++i) cudaEventDestroy(ev[i]);
+  if (rc == RHYME_GPU_OK) CK(fill_after_run(ctx, b));
   for (int k = 0; k < 5; ++k) ms[k] = acc[k] / nsteps;
   if (fused) ms[3] = -1.0;  // ms[2]: the x and y sweeps as one kernel
   b->carry_valid = ctx->mixed && rc == RHYME_GPU_OK;
@@ -1543,6 +1561,8 @@ int batch_build(rhyme_gpu_batch* B) {
   tab[1].resize(n);
   std::vector<WorkItem> cfl, ghost, faces, flux, update, sweep[3][kSweepShapes];
   const bool fuse = ctx->mixed && D == 3 && ctx->fuse_xy;
+  bool fill_each = !ctx->mixed;
+  for (int h : B->handles) fill_each = fill_each || !halo_from_interior(D, ctx->boxes[h]->g);
   long long qcap = 0;
   for (int i = 0; i < n; ++i) {
     Box* b = ctx->boxes[B->handles[i]];
@@ -1573,6 +1593,7 @@ int batch_build(rhyme_gpu_batch* B) {
         d.bc[f] = b->dp.bc[f];
         for (int cc = 0; cc < 5; ++cc) d.inflow[f][cc] = b->dp.inflow[f][cc];
       }
+      if (!fill_each) d.halo = make_halo(D, b->g, d.bc, d.inflow);
       d.cfl_items = (int)((cells + kBatchCflChunk - 1) / kBatchCflChunk);
     }
   }
@@ -1655,6 +1676,7 @@ int batch_build(rhyme_gpu_batch* B) {
   L.n_flux = (int)flux.size();
   L.n_update = (int)update.size();
   L.fuse_xy = fuse;
+  L.fill_each = fill_each;
   L.heads = B->heads;
   L.whole = B->qblock + 3;
   return RHYME_GPU_OK;
@@ -1746,6 +1768,8 @@ extern "C" int rhyme_gpu_batch_run(rhyme_gpu_batch* B, int nsteps) {
                            ctx->stream));
     B->k ^= 1;
   }
+  // as after a box's resident run, from the last step's U^n
+  if (nsteps > 0 && !B->L.fill_each) CK(launch_batch_ghosts(ctx->params.ndim, B->table[B->k ^ 1], B->L, ctx->stream));
   for (size_t i = 0; i < B->handles.size(); ++i) {
     Box* b = ctx->boxes[B->handles[i]];
     b->cur = B->base_cur[i] ^ B->k;

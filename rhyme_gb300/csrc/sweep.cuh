@@ -195,6 +195,21 @@ struct SweepSmem {
   float f[D + 2][(S + 1) * P];   // interface fluxes (normal-first)
 };
 
+// Ghost cell i (outside 1..N) along axis A of a line whose cells lie at
+// line + i stride, from the interior: component c in v[c] (every component
+// of the mirror; F the component stride). type: 1..4.
+template <int D>
+__device__ __forceinline__ void ghost_value(const float* __restrict__ Uf, long long line, long long stride,
+                                            long long F, int A, int i, int N, int type,
+                                            const float* __restrict__ inflow, float* v) {
+  const long long o = line + ghost_source(i, N, type) * stride;
+#pragma unroll
+  for (int c = 0; c < D + 2; ++c) {
+    v[c] = (type == 4) ? inflow[c] : Uf[(long long)c * F + o];
+    if (type == 1 && c == 1 + A) v[c] = -v[c];  // reflective: the normal momentum negated
+  }
+}
+
 // One slab (tile tA along the sweep axis, tB across the pencils, plane cC)
 // of a sweep. `box` tags queued FP64 interfaces (0 for a single box).
 template <int D, int A, int S, int P, int MODE>
@@ -205,7 +220,7 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
                                            const FallbackQueue& q, int box,
                                            int tA, int tB, int cC, SweepSmem<D, S, P>& sh,
                                            const TmaStage& tma, unsigned long long* bar, unsigned& parity,
-                                           const SweepCarry& carry = SweepCarry()) {
+                                           const SweepCarry& carry, const HaloBC& halo) {
   constexpr int B = Axes<D, A>::B, C = Axes<D, A>::C;
   // component plane of the staged slab, and the index of (la, lb) in it
   constexpr int PLANE = (A == 0) ? (S + 4) * P : (S + 4) * (P + 4);
@@ -265,6 +280,23 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
     cp_async_commit();
   }
 
+  // the ghost cells of a face that gives them from the interior: fetched now,
+  // put in place over what the staging brought
+  const bool lo_halo = a0 == 1 && halo.type[2 * A] != 0;
+  const bool hi_halo = a0 + S + 1 > NA && halo.type[2 * A + 1] != 0;
+  float hv[D + 2];
+  int hx = -1;
+  if ((lo_halo || hi_halo) && threadIdx.x < 4 * P) {
+    const int layer = threadIdx.x / P, lb = threadIdx.x % P;
+    const int ga = layer < 2 ? layer - 1 : NA - 1 + layer;
+    const int la = ga - (a0 - 2);
+    if ((layer < 2 ? lo_halo : hi_halo) && la >= 0 && la < S + 4 && b0 + lb <= NB) {
+      hx = ixu(la, lb);
+      ghost_value<D>(Uf, offset(0, b0 + lb), g.s[A], F, A, ga, NA, halo.type[2 * A + (layer >> 1)],
+                     halo.inflow[2 * A + (layer >> 1)], hv);
+    }
+  }
+
   // 1. stage the FP32 slab: cells a0-2 .. a0+S+1 along A
   if (tma.on) {
     // one tensor copy of the whole slab (every component), zero-filled
@@ -306,6 +338,13 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
     }
   }
   __syncthreads();
+  if (lo_halo || hi_halo) {
+    if (hx >= 0) {
+#pragma unroll
+      for (int c = 0; c < D + 2; ++c) su[c * PLANE + hx] = hv[c];
+    }
+    __syncthreads();
+  }
   const float dtdx = s_dtdx[0];
   const float hdtdx = s_dtdx[1];
 
@@ -423,7 +462,7 @@ __global__ void __launch_bounds__(TileCfg<S, P>::threads, TileCfg<S, P>::templat
     sweep_kernel(MixedParams M, const float* __restrict__ Uf, const double* __restrict__ U, Geom g,
                  Dx dx, const double* __restrict__ dtp, float* __restrict__ acc,
                  double* __restrict__ Unew, FallbackQueue q, const __grid_constant__ CUtensorMap map,
-                 int tma_on, int o_off, SweepCarry carry) {
+                 int tma_on, int o_off, SweepCarry carry, const __grid_constant__ HaloBC halo) {
   constexpr int C = Axes<D, A>::C;
   __shared__ SweepSmem<D, S, P> sh;
   __shared__ __align__(8) unsigned long long bar;
@@ -435,7 +474,7 @@ __global__ void __launch_bounds__(TileCfg<S, P>::threads, TileCfg<S, P>::templat
   const int tB = (A == 0) ? blockIdx.y : blockIdx.x;
   const int cC = (C < D) ? (int)blockIdx.z + 1 : 1;
   sweep_tile<D, A, S, P, MODE>(M, M.limiter, M.omega, Uf, U, g, dx, dtp, acc, Unew, q, 0, tA, tB, cC,
-                               sh, tma, &bar, parity, carry);
+                               sh, tma, &bar, parity, carry, halo);
 }
 
 // The same sweep over the tiles of a batch of boxes, taken from a work queue
@@ -471,7 +510,7 @@ __global__ void __launch_bounds__(TileCfg<S, P>::threads, TileCfg<S, P>::templat
       carry.status = (int*)(b.ctl + 2) + 1;
     }
     sweep_tile<D, A, S, P, MODE>(M, b.limiter, b.omega_f, b.Uf, b.U, b.g, b.dx, b.ctl, b.acc, b.V,
-                                 q, w.box, tA, tB, cC, sh, tma, nullptr, parity, carry);
+                                 q, w.box, tA, tB, cC, sh, tma, nullptr, parity, carry, b.halo);
     if (threadIdx.x == 0) s_item = next;
     __syncthreads();
     it = s_item;
@@ -518,7 +557,8 @@ __device__ __forceinline__ void sweep_xy_tile(const MixedParams& M, int limiter,
                                               const float* __restrict__ Uf, const Geom& g, const Dx& dx,
                                               const double* __restrict__ dtp, float* __restrict__ acc,
                                               const FallbackQueue& q, int box, int x0, int y0, int cz,
-                                              XYSmem<TX, TY>& sh, const CUtensorMap* map, unsigned long long* bar) {
+                                              XYSmem<TX, TY>& sh, const CUtensorMap* map, unsigned long long* bar,
+                                              const HaloBC& halo) {
   using Cfg = XYCfg<TX, TY>;
   constexpr int NT = Cfg::threads;
   constexpr int PW = TX + 4;               // plane row
@@ -527,6 +567,31 @@ __device__ __forceinline__ void sweep_xy_tile(const MixedParams& M, int limiter,
   const int NX = g.n[0], NY = g.n[1];
   const long long F = g.field;
   float* su = sh.u;
+  // the ghost cells of faces that give them from the interior (as in
+  // sweep_tile): 4 layers of TY rows along x, then 4 of TX columns along y
+  const bool xlo = x0 == 1 && halo.type[0] != 0, xhi = x0 + TX + 1 > NX && halo.type[1] != 0;
+  const bool ylo = y0 == 1 && halo.type[2] != 0, yhi = y0 + TY + 1 > NY && halo.type[3] != 0;
+  const bool patch = xlo || xhi || ylo || yhi;
+  float hv[5];
+  int hx = -1;
+  if (patch && threadIdx.x < 4 * (TX + TY)) {
+    const int ax = threadIdx.x >= 4 * TY;
+    const int t = ax ? threadIdx.x - 4 * TY : threadIdx.x;
+    const int T = ax ? TX : TY;  // positions across the axis
+    const int layer = t / T, lb = t % T;
+    const int N = ax ? NY : NX;
+    const int gi = layer < 2 ? layer - 1 : N - 1 + layer;     // along the axis
+    const int gb = (ax ? x0 : y0) + lb;                       // across it
+    const int la = gi - ((ax ? y0 : x0) - 2);
+    const bool on = layer < 2 ? (ax ? ylo : xlo) : (ax ? yhi : xhi);
+    if (on && la >= 0 && la < (ax ? TY : TX) + 4 && gb <= (ax ? NX : NY)) {
+      hx = ax ? la * PW + lb + 2 : (lb + 2) * PW + la;
+      const int f = 2 * ax + (layer >> 1);
+      const int type = layer < 2 ? (ax ? halo.type[2] : halo.type[0]) : (ax ? halo.type[3] : halo.type[1]);
+      ghost_value<3>(Uf, ax ? g.at(3, gb, 0, cz) : g.at(3, 0, gb, cz), ax ? g.s[1] : 1, F, ax, gi, N, type,
+                     halo.inflow[f], hv);
+    }
+  }
   // 1. stage the plane: cells x0-2 .. x0+TX+1, y0-2 .. y0+TY+1 of plane cz
   if (map && threadIdx.x == 0)
     tma_load_4d(su, map, x0 - 1, y0 - 1, cz + 1, 0, bar, (unsigned)(5 * PL * sizeof(float)));
@@ -556,6 +621,13 @@ __device__ __forceinline__ void sweep_xy_tile(const MixedParams& M, int limiter,
     }
   }
   __syncthreads();
+  if (patch) {
+    if (hx >= 0) {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) su[c * PL + hx] = hv[c];
+    }
+    __syncthreads();
+  }
 
   // 2. face states: x of cells x0-1 .. x0+TX (rows y0 ..), then y of cells
   // y0-1 .. y0+TY (columns x0 ..); one loop, the axis only in the indices
@@ -672,14 +744,15 @@ __device__ __forceinline__ void sweep_xy_tile(const MixedParams& M, int limiter,
 
 template <int TX, int TY>
 __global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
-    sweep_xy_kernel(MixedParams M, Geom g, Dx dx, const double* __restrict__ dtp, float* __restrict__ acc,
-                    FallbackQueue q, const __grid_constant__ CUtensorMap map) {
+    sweep_xy_kernel(MixedParams M, const float* __restrict__ Uf, Geom g, Dx dx, const double* __restrict__ dtp,
+                    float* __restrict__ acc, FallbackQueue q, const __grid_constant__ CUtensorMap map,
+                    const __grid_constant__ HaloBC halo) {
   __shared__ XYSmem<TX, TY> sh;
   __shared__ __align__(8) unsigned long long bar;
   if (threadIdx.x == 0) mbar_init(&bar);
   __syncthreads();
-  sweep_xy_tile<TX, TY>(M, M.limiter, M.omega, nullptr, g, dx, dtp, acc, q, 0, blockIdx.x * TX + 1,
-                        blockIdx.y * TY + 1, (int)blockIdx.z + 1, sh, &map, &bar);
+  sweep_xy_tile<TX, TY>(M, M.limiter, M.omega, Uf, g, dx, dtp, acc, q, 0, blockIdx.x * TX + 1,
+                        blockIdx.y * TY + 1, (int)blockIdx.z + 1, sh, &map, &bar, halo);
 }
 
 // The tiles of a batch of boxes from a work queue, as batch_sweep_kernel
@@ -699,7 +772,7 @@ __global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
     const unsigned chunk = (unsigned)w.chunk, r = chunk / nx;
     sweep_xy_tile<TX, TY>(M, b.limiter, b.omega_f, b.Uf, b.g, b.dx, b.ctl, b.acc, q, w.box,
                           (int)(chunk - r * nx) * TX + 1, (int)(r % ny) * TY + 1, (int)(r / ny) + 1, sh, nullptr,
-                          nullptr);
+                          nullptr, b.halo);
     if (threadIdx.x == 0) s_item = next;
     __syncthreads();
     it = s_item;

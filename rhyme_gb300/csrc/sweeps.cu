@@ -32,7 +32,7 @@ constexpr int mode_of() {
 template <int D, int A, int S, int P>
 cudaError_t launch_one(const MixedParams& M, const float* Uf, const double* U, const Geom& g, const Dx& dx,
                        const double* dtp, float* acc, double* Unew, const FallbackQueue& q, int lo, int hi,
-                       cudaStream_t st, const SweepCarry& carry) {
+                       cudaStream_t st, const SweepCarry& carry, const HaloBC& halo) {
   constexpr int B = Axes<D, A>::B, C = Axes<D, A>::C;
   constexpr int O = D - 1;
   const int NO = g.n[O];
@@ -62,7 +62,7 @@ cudaError_t launch_one(const MixedParams& M, const float* Uf, const double* U, c
   SweepCarry cs = carry;
   if (cs.Uf_next) cs.Uf_next += shift;
   sweep_kernel<D, A, S, P, mode_of<D, A>()><<<grid, TileCfg<S, P>::threads, 0, st>>>(
-      M, Uf + shift, U + shift, gs, dx, dtp, acc + shift, Unew + shift, qs, map, tma_on, lo - 1, cs);
+      M, Uf + shift, U + shift, gs, dx, dtp, acc + shift, Unew + shift, qs, map, tma_on, lo - 1, cs, halo);
   return cudaGetLastError();
 }
 
@@ -80,20 +80,21 @@ cudaError_t launch_batch_one(const MixedParams& M, const BoxDesc* TB, const Work
 template <int D, int A>
 cudaError_t by_shape(int shape, const MixedParams& M, const float* Uf, const double* U, const Geom& g,
                      const Dx& dx, const double* dtp, float* acc, double* Unew,
-                     const FallbackQueue& q, int lo, int hi, cudaStream_t st, const SweepCarry& carry) {
+                     const FallbackQueue& q, int lo, int hi, cudaStream_t st, const SweepCarry& carry,
+                     const HaloBC& halo) {
   if constexpr (D == 1) {
     switch (shape) {
-      case 0: return launch_one<D, A, 64, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
-      case 1: return launch_one<D, A, 128, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
-      case 2: return launch_one<D, A, 256, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
-      case 3: return launch_one<D, A, 512, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
+      case 0: return launch_one<D, A, 64, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      case 1: return launch_one<D, A, 128, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      case 2: return launch_one<D, A, 256, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      case 3: return launch_one<D, A, 512, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
     }
   } else {
     switch (shape) {
-      case 0: return launch_one<D, A, 8, 32>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
-      case 1: return launch_one<D, A, 16, 16>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
-      case 2: return launch_one<D, A, 32, 8>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
-      case 3: return launch_one<D, A, 64, 4>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
+      case 0: return launch_one<D, A, 8, 32>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      case 1: return launch_one<D, A, 16, 16>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      case 2: return launch_one<D, A, 32, 8>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      case 3: return launch_one<D, A, 64, 4>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
     }
   }
   return cudaErrorInvalidValue;
@@ -129,15 +130,15 @@ cudaError_t RGPU_CAT(launch_sweep_axis_, SWEEP_D)(int axis, int shape, const Mix
                                                  const double* U, const Geom& g, const Dx& dx,
                                                  const double* dtp, float* acc, double* Unew,
                                                  const FallbackQueue& q, int lo, int hi, cudaStream_t st,
-                                                 const SweepCarry& carry) {
+                                                 const SweepCarry& carry, const HaloBC& halo) {
   constexpr int D = SWEEP_D;
   switch (axis) {
-    case 0: return by_shape<D, 0>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
+    case 0: return by_shape<D, 0>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
     case 1:
-      if constexpr (D > 1) return by_shape<D, 1>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
+      if constexpr (D > 1) return by_shape<D, 1>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
       break;
     case 2:
-      if constexpr (D > 2) return by_shape<D, 2>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry);
+      if constexpr (D > 2) return by_shape<D, 2>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
       break;
   }
   return cudaErrorInvalidValue;
@@ -161,15 +162,16 @@ cudaError_t RGPU_CAT(launch_batch_sweep_axis_, SWEEP_D)(int axis, int shape, con
 
 #if SWEEP_D == 3
 cudaError_t launch_sweep_xy_3(const MixedParams& M, const float* Uf, const Geom& g, const Dx& dx,
-                              const double* dtp, float* acc, const FallbackQueue& q, cudaStream_t st) {
+                              const double* dtp, float* acc, const FallbackQueue& q, const HaloBC& halo,
+                              cudaStream_t st) {
   constexpr int TX = 16, TY = 16;
   const unsigned gx = (unsigned)((g.n[0] + TX - 1) / TX), gy = (unsigned)((g.n[1] + TY - 1) / TY);
   if (gy > 65535 || g.n[2] > 65535) return cudaErrorNotSupported;
   CUtensorMap map;
   memset(&map, 0, sizeof map);
   if (!encode_xy_map(&map, Uf, g, TX, TY)) return cudaErrorNotSupported;
-  sweep_xy_kernel<TX, TY><<<dim3(gx, gy, (unsigned)g.n[2]), XYCfg<TX, TY>::threads, 0, st>>>(M, g, dx, dtp, acc, q,
-                                                                                             map);
+  sweep_xy_kernel<TX, TY><<<dim3(gx, gy, (unsigned)g.n[2]), XYCfg<TX, TY>::threads, 0, st>>>(M, Uf, g, dx, dtp, acc,
+                                                                                             q, map, halo);
   return cudaGetLastError();
 }
 
