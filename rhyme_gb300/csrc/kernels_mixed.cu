@@ -13,7 +13,7 @@
 // FP64 adds are scarce (the next step's CFL makes the new mirror, where the
 // conversions cost nothing but bandwidth).
 //
-// Interfaces that near vacuum, or whose FP32 Newton iteration misses the
+// Interfaces that near vacuum, or whose FP32 iteration does not reach the
 // tolerance on its first guess, or whose FP32 face states or flux are not
 // finite, get a zero flux in the sweep and are appended (once, by the tile
 // that owns them) to a device queue. After the last sweep one kernel redoes

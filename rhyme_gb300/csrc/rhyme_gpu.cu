@@ -255,11 +255,17 @@ void make_mixed_params(const DevParams& d, MixedParams* m) {
   F.by_gm1 = m_inv(F.gm1);
   F.by_gp1 = m_inv(F.gp1);
   F.by_kb_amu = m_inv(F.kb_amu);
+  F.gm1_lo = (float)(G.gm1 - (double)F.gm1);
+  F.g_gm1 = (float)(G.g / G.gm1);
   m->rp.vac_rho = (float)d.rp.vac_rho;
   m->rp.vac_p = (float)d.rp.vac_p;
   m->rp.vac_rho_next = std::nextafter((float)d.rp.vac_rho, 1.0f);
   m->rp.tol = (float)d.rp.tol;
   m->rp.n_iter = d.rp.n_iter;
+  // third order: a last step of cbrt(tol) leaves less than tol, one of 5e-3
+  // less than 1.3e-8; with few iterations allowed the FP64 form may stop
+  // short of the root, and only steps below tol agree with it
+  m->rp.last = d.rp.n_iter < 8 ? (float)d.rp.tol : (float)std::min(5e-3, std::cbrt(d.rp.tol));
   m->G64 = d.G;
   m->rp64 = d.rp;
   m->ndim = d.ndim;
