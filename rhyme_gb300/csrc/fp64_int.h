@@ -180,12 +180,41 @@ RGPU_HD double sqrt_rn(double a) {
 #endif
 }
 
-// a > b. Two non-negative numbers order like their bits; a negative one or a
-// NaN takes the hardware comparison.
+// The hardware's operations where an operand is out of the integer forms'
+// range: behind an opaque asm on the device, because the compiler would
+// otherwise run such a cheap instruction for every lane and select.
+RGPU_HD double hw_mul(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  double r;
+  asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+#else
+  return a * b;
+#endif
+}
+RGPU_HD bool hw_gt(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n setp.gt.f64 p, %1, %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r) : "d"(a), "d"(b));
+  return r != 0;
+#else
+  return a > b;
+#endif
+}
+
+// a > b. Two non-negative finite numbers order like their bits, others like
+// their signed magnitudes; infinities and NaNs take the hardware comparison.
 RGPU_HD bool f64_gt(double a, double b) {
   const uint32_t ha = f64_hi(a), hb = f64_hi(b);
   if ((ha > hb ? ha : hb) < 0x7ff00000u) return f64_bits(a) > f64_bits(b);
-  return a > b;
+  const uint32_t ma = ha & 0x7fffffffu, mb = hb & 0x7fffffffu;
+  if ((ma > mb ? ma : mb) < 0x7ff00000u) {
+    const int64_t ia = (int64_t)f64_bits(a), ib = (int64_t)f64_bits(b);
+    const int64_t ka = ia < 0 ? (int64_t)(fp64_int::kSign - (uint64_t)ia) : ia;
+    const int64_t kb = ib < 0 ? (int64_t)(fp64_int::kSign - (uint64_t)ib) : ib;
+    return ka > kb;
+  }
+  return hw_gt(a, b);
 }
 // x > c for a positive constant c or zero: x in (c, infinity].
 RGPU_HD bool f64_above(double x, double c) {
@@ -196,6 +225,8 @@ RGPU_HD bool f64_above(double x, double c) {
 RGPU_HD bool f64_negative(double x) {
   return f64_bits(x) - (fp64_int::kSign + 1u) < fp64_int::kInf;
 }
+// x == 0.
+RGPU_HD bool f64_zero(double x) { return (f64_bits(x) << 1) == 0; }
 // |x| below the smallest normal number.
 RGPU_HD bool f64_tiny(double x) { return (f64_hi(x) & 0x7ff00000u) == 0; }
 
@@ -207,7 +238,7 @@ RGPU_HD double f64_scale(double x) {
   constexpr uint32_t lo = (uint32_t)(1 + (K < 0 ? -K : 0)) << 20, hi = (uint32_t)(2047 - (K > 0 ? K : 0)) << 20;
   if (h - lo < hi - lo) return f64_from(f64_bits(x) + ((uint64_t)(int64_t)K << 52));
   if ((f64_bits(x) << 1) == 0) return x;
-  return x * (K < 0 ? 1.0 / (double)(1 << (K < 0 ? -K : 0)) : (double)(1 << (K > 0 ? K : 0)));
+  return hw_mul(x, K < 0 ? 1.0 / (double)(1 << (K < 0 ? -K : 0)) : (double)(1 << (K > 0 ? K : 0)));
 }
 
 }  // namespace rgpu

@@ -212,10 +212,10 @@ __device__ __forceinline__ double limited_slope_f64(int type, double w, double u
   const double r = f64_tiny(d_R) ? 0.0 : div_rn(d_L, d_R);
   if (!f64_above(r, 0.0)) return 0.0;
   double d;
-  if (w == 0.0) {
+  if (f64_zero(w)) {
     d = d_L + d_R;
     // half the sum, exactly, well above the subnormal range
-    d = ((f64_hi(d) & 0x7fffffffu) - 0x08000000u < 0x7fe00000u - 0x08000000u) ? f64_scale<-1>(d) : 0.5 * d_L + 0.5 * d_R;
+    d = ((f64_hi(d) & 0x7fffffffu) - 0x08000000u < 0x7fe00000u - 0x08000000u) ? f64_scale<-1>(d) : hw_mul(0.5, d_L) + hw_mul(0.5, d_R);
     const bool big = f64_above(r, 1.0);
     if (f64_hi(r) < 0x7ff00000u) {
       if (type == 1) return div_rn(big ? 2.0 : f64_scale<1>(r), 1.0 + r) * d;
@@ -431,8 +431,8 @@ __device__ __forceinline__ void nonlinear_waves(const Gas<double>& G, const Wave
 __device__ __forceinline__ double guess_p_star_adaptive(const Gas<double>& G, double l_rho, double vl, double l_p,
                                                         double l_cs, double r_rho, double vr, double r_p,
                                                         double r_cs) {
-  const double cup = 0.25 * (l_rho + r_rho) * (l_cs + r_cs);
-  const double ppv = fmax_ref(0.5 * (l_p + r_p) + 0.5 * (vl - vr) * cup, 0.0);
+  const double cup = f64_scale<-2>(l_rho + r_rho) * (l_cs + r_cs);
+  const double ppv = fmax_ref(m_half(l_p + r_p) + m_half(vl - vr) * cup, 0.0);
   const double p_min = fmin_ref(l_p, r_p);
   const double p_max = fmax_ref(l_p, r_p);
   // q_max = p_max/p_min <= q_user = 2: for normal numbers the quotient
@@ -448,7 +448,7 @@ __device__ __forceinline__ double guess_p_star_adaptive(const Gas<double>& G, do
                             m_div(pq, icl) + m_div(1.0, icr));
     const double ptl = 1.0 + m_div(G.half_gm1 * (vl - um), icl);
     const double ptr = 1.0 + m_div(G.half_gm1 * (um - vr), icr);
-    return 0.5 * (l_p * m_pow(ptl, G.inv_gm1_2g) + r_p * m_pow(ptr, G.inv_gm1_2g));
+    return m_half(l_p * m_pow(ptl, G.inv_gm1_2g) + r_p * m_pow(ptr, G.inv_gm1_2g));
   }
   // two-shock
   const double gel = m_sqrt(m_div(m_div(G.two_gp1, l_rho), G.gm1_gp1 * l_p + ppv));
@@ -549,11 +549,11 @@ __device__ __forceinline__ void rp_sample_side(const Gas<double>& G, const Side<
     rho_star = S.rho * pg;
     inner = us - cs * pa;
   }
-  const bool star = right ? dxdt < inner : dxdt > inner;
+  const bool star = m_gt(right ? inner : dxdt, right ? dxdt : inner);
   bool outside = shock;
   if (!star && !shock) {
     const double head = S.v[AX] - cs;
-    outside = !(right ? dxdt < head : dxdt > head);
+    outside = !m_gt(right ? head : dxdt, right ? dxdt : head);
   }
   if (star || outside) {
     // rhyme_riemann_problem_w_star{L,R}_{sho,fan}.f90:12-15, or the side itself
@@ -632,7 +632,7 @@ __device__ __forceinline__ void rp_solve(const Gas<double>& G, const Rp<double>&
     R.cs = fmax_ref(sound_speed<D>(G, r, ir), tiny);
     const double du = R.v[AX] - L.v[AX];
     const double du_crit = m_div(m_twice(L.cs + R.cs), G.by_gm1);
-    if (du_crit < du) {  // vacuum generation
+    if (m_gt(du, du_crit)) {  // vacuum generation
       const double s_starl = L.v[AX] - 2.0 * L.cs / G.gm1;
       const double s_starr = R.v[AX] + 2.0 * R.cs / G.gm1;
       if (dxdt > s_starr) {
@@ -652,9 +652,9 @@ __device__ __forceinline__ void rp_solve(const Gas<double>& G, const Rp<double>&
       const WaveSide WL = wave_side(G, L.rho, L.p, L.cs), WR = wave_side(G, R.rho, R.p, R.cs);
       double ps = irs_exec(G, rp.tol, rp.n_iter, WL, WR, L.rho, L.v[AX], L.cs, l_f, R.rho, R.v[AX], R.cs, r_f);
       if (m_gt(rp.vac_p, ps)) ps = rp.vac_p;
-      const double us = 0.5 * ((R.v[AX] + L.v[AX]) + (r_f - l_f));
+      const double us = m_half((R.v[AX] + L.v[AX]) + (r_f - l_f));
       // the side of the contact that x/t = dxdt lies on
-      const bool right = dxdt > us;
+      const bool right = m_gt(dxdt, us);
       Side<D> S;
       S.rho = right ? R.rho : L.rho;
       S.v[AX] = right ? R.v[AX] : L.v[AX];

@@ -48,9 +48,9 @@ int main(int argc, char** argv) {
     const double near = (double)((long double)d * ((long double)m + 0x1p-53L));
     const double sq = (double)(((long double)m + 0x1p-53L) * ((long double)m + 0x1p-53L));
     bad[2] += !same(div_rn(near, d), near / d) + !same(sqrt_rn(sq), std::sqrt(sq)) + !same(sqrt_rn(m * m), std::sqrt(m * m));
-    bad[3] += f64_gt(a, b) != (a > b) || f64_gt(a, a) != (a > a);
+    bad[3] += f64_gt(a, b) != (a > b) || f64_gt(b, a) != (b > a) || f64_gt(a, a) != (a > a) || f64_gt(a, -a) != (a > -a);
     bad[4] += f64_above(a, 0.0) != (a > 0.0) || f64_above(a, 1.0) != (a > 1.0) || f64_negative(a) != (a < 0.0);
-    bad[5] += f64_tiny(a) != (std::fabs(a) < std::numeric_limits<double>::min());
+    bad[5] += f64_tiny(a) != (std::fabs(a) < std::numeric_limits<double>::min()) || f64_zero(a) != (a == 0.0);
     bad[6] += !same(f64_scale<1>(a), 2.0 * a) || !same(f64_scale<-1>(a), 0.5 * a) || !same(f64_scale<-3>(a), 0.125 * a);
   }
   long all = 0;
