@@ -46,7 +46,8 @@ UNITS = [
     ("kernels_paint", "kernels_paint.cu", ["--fmad=false"]),
     ("kernels_probe", "kernels_probe.cu", FP32_SWEEP_FLAGS),
 ]
-HEADERS = ["hydro.cuh", "fp64_int.h", "rgpu_internal.h", "detmath.h", "libm_pow.h", "libm_pow_tables.h", "box_elems.cuh", "sweep.cuh"]
+HEADERS = ["hydro.cuh", "fp64_int.h", "rgpu_internal.h", "detmath.h", "libm_pow.h", "libm_pow_tables.h", "libm_pow_int.h", "libm_pow_int_tables.h",
+           "box_elems.cuh", "sweep.cuh"]
 
 
 def nvcc():

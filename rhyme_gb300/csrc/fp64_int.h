@@ -29,9 +29,11 @@
 
 #if defined(__CUDACC__)
 #define RGPU_HD __host__ __device__ __forceinline__
+#define RGPU_CALL static __host__ __device__ __noinline__
 #else
 #include <cmath>
 #define RGPU_HD inline
+#define RGPU_CALL inline
 #endif
 
 #ifndef RGPU_SEED_ERROR
@@ -123,10 +125,10 @@ RGPU_HD Divisor divisor(double b) {
   return {b, 2u * R0 + (uint32_t)(int32_t)(c >> 43)};
 }
 
-// a / d.b, rounded to nearest even.
-RGPU_HD double div_by(double a, const Divisor& d) {
+// a / b, R from divisor(b), rounded to nearest even.
+RGPU_HD double div_core(double a, double b, uint32_t R) {
   using namespace fp64_int;
-  const uint64_t ua = f64_bits(a), ub = f64_bits(d.b);
+  const uint64_t ua = f64_bits(a), ub = f64_bits(b);
   const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu, eb = (uint32_t)(ub >> 52) & 0x7ffu;
   if (ea - 1u < 2046u && eb - 1u < 2046u && ea - eb + 1021u < 2044u) {
     uint64_t A = (ua & kFrac) | kUnit;
@@ -136,21 +138,25 @@ RGPU_HD double div_by(double a, const Divisor& d) {
       A <<= 1;
       e -= 1u;
     }
-    const uint32_t q1 = mul_hi((uint32_t)(A >> 22), d.R) >> 2;  // 2^27 A/B, short by less than 1.75
+    const uint32_t q1 = mul_hi((uint32_t)(A >> 22), R) >> 2;  // 2^27 A/B, short by less than 1.75
     const uint64_t r1 = (A << 27) - (uint64_t)q1 * B;
-    const uint32_t q2 = mul_hi((uint32_t)(r1 >> 23), d.R);  // 2^28 r1/B, short by less than 2.4
+    const uint32_t q2 = mul_hi((uint32_t)(r1 >> 23), R);  // 2^28 r1/B, short by less than 2.4
     const uint64_t r2 = (r1 << 28) - (uint64_t)q2 * B;
     const uint64_t Q = ((uint64_t)q1 << 28) + (q2 + 4u) + (r2 >= B ? 1u : 0u) + (r2 >= 2 * B ? 1u : 0u);
     return f64_from(((ua ^ ub) & kSign) | (((uint64_t)e << 52) + (Q >> 3)));
   }
   if ((ua << 1) == 0 && eb - 1u < 2046u) return f64_from((ua ^ ub) & kSign);
-  return a / d.b;
+  return a / b;
 }
 
-RGPU_HD double div_rn(double a, double b) { return div_by(a, divisor(b)); }
+// Calls, not inlined: the interface solve divides at some fifty places, and
+// with a copy at each its warps waited for instructions half of the time.
+RGPU_CALL double div_with(double a, double b, uint32_t R) { return div_core(a, b, R); }
+RGPU_CALL double div_rn(double a, double b) { return div_core(a, b, divisor(b).R); }
+RGPU_HD double div_by(double a, const Divisor& d) { return div_with(a, d.b, d.R); }
 
 // sqrt(a), rounded to nearest even.
-RGPU_HD double sqrt_rn(double a) {
+RGPU_CALL double sqrt_rn(double a) {
   using namespace fp64_int;
   const uint64_t ua = f64_bits(a);
   const uint32_t ea = (uint32_t)(ua >> 52);

@@ -19,18 +19,18 @@
 #include <cstdint>
 
 #include "fp64_int.h"
-#include "libm_pow.h"
+#include "libm_pow_int.h"
 
 namespace rgpu {
 
 // ---- math by type --------------------------------------------------------
-// Double powers go through libm_pow::pow, a restatement of the C library's
-// pow that the compiled reference calls for every real `**`, so the FP64 path
-// returns the reference's bits even in flows that amplify a one-ulp
-// difference.
+// Double powers return the bits of libm_pow::pow, a restatement of the C
+// library's pow that the compiled reference calls for every real `**`, so the
+// FP64 path returns the reference's bits even in flows that amplify a one-ulp
+// difference; libm_pow_int.h forms them mostly in integers.
 __device__ __forceinline__ double m_sqrt(double x) { return sqrt_rn(x); }
 __device__ __forceinline__ float m_sqrt(float x) { return sqrtf(x); }
-__device__ __forceinline__ double m_pow(double x, double y) { return libm_pow::pow(x, y); }
+__device__ __forceinline__ double m_pow(double x, double y) { return libm_pow_int::pow(x, y); }
 // Float powers as 2^(y log2 x) with CUDA's log2f and exp2f: the rounding of
 // the product adds a relative error of about 2^-24 |y log2 x| to the result
 // (for the positive bases of this path), against powf's ~1 ulp, for a
@@ -38,7 +38,9 @@ __device__ __forceinline__ double m_pow(double x, double y) { return libm_pow::p
 __device__ __forceinline__ float m_pow(float x, float y) { return exp2f(y * log2f(x)); }
 // x**y1 and x**y2 of one base (one logarithm).
 __device__ __forceinline__ void m_pow2(double x, double y1, double y2, double& r1, double& r2) {
-  libm_pow::pow2(x, y1, y2, &r1, &r2);
+  const double2 r = libm_pow_int::pow2(x, y1, y2);
+  r1 = r.x;
+  r2 = r.y;
 }
 __device__ __forceinline__ void m_pow2(float x, float y1, float y2, float& r1, float& r2) {
   const float l = log2f(x);
@@ -61,7 +63,8 @@ __host__ __device__ __forceinline__ Inv<double> m_inv(double b) { return {diviso
 // without the scaling that the division operator adds for larger divisors.
 __device__ __forceinline__ float m_div(float a, const Inv<float>& i) { return __fdividef(a, i.b); }
 __device__ __forceinline__ double m_div(double a, const Inv<double>& i) { return div_by(a, i.d); }
-template <typename T> __device__ __forceinline__ T m_div(T a, T b) { return m_div(a, m_inv(b)); }
+__device__ __forceinline__ float m_div(float a, float b) { return __fdividef(a, b); }
+__device__ __forceinline__ double m_div(double a, double b) { return div_rn(a, b); }
 // a / (2 b): the significand of 2 b is that of b
 __device__ __forceinline__ double div_half(double a, const Inv<double>& i) {
   Divisor d = i.d;
@@ -207,36 +210,41 @@ __device__ __forceinline__ void prim_vars_to_cons(const Gas<T>& G, T rho, const 
 // 2/(1+r), and of two quotients with the same divisor the smaller one is
 // known from the numerators (rounding is monotonic), so van Leer, minmod
 // and superbee need one division after r.
+__device__ __forceinline__ double limiter_phi(int type, double w, double r) {  // r > 0
+  const double xi = div_rn(2.0, 1.0 - w + (1.0 + w) * r);
+  if (type == 1) return fmin_ref(div_rn(f64_scale<1>(r), 1.0 + r), xi);
+  if (type == 2) return f64_above(r, 1.0) ? fmin_ref(1.0, xi) : r;
+  if (type == 3) return fmin_ref(div_rn(r * (1.0 + r), 1.0 + r * r), xi);
+  if (f64_above(r, 1.0)) return fmin_ref(fmin_ref(r, xi), 2.0);
+  return f64_above(r, 0.5) ? 1.0 : f64_scale<1>(r);
+}
+
 __device__ __forceinline__ double limited_slope_f64(int type, double w, double ul, double u, double ur) {
   const double d_L = u - ul, d_R = ur - u;
   const double r = f64_tiny(d_R) ? 0.0 : div_rn(d_L, d_R);
   if (!f64_above(r, 0.0)) return 0.0;
-  double d;
+  // phi first, by integer selections and divisions, then one product with d
+  // for every lane
+  double d, phi;
   if (f64_zero(w)) {
     d = d_L + d_R;
     // half the sum, exactly, well above the subnormal range
     d = ((f64_hi(d) & 0x7fffffffu) - 0x08000000u < 0x7fe00000u - 0x08000000u) ? f64_scale<-1>(d) : hw_mul(0.5, d_L) + hw_mul(0.5, d_R);
     const bool big = f64_above(r, 1.0);
-    if (f64_hi(r) < 0x7ff00000u) {
-      if (type == 1) return div_rn(big ? 2.0 : f64_scale<1>(r), 1.0 + r) * d;
-      if (type == 2) return (big ? div_rn(2.0, 1.0 + r) : r) * d;
-      if (type == 4) {
-        if (big) return div_rn(2.0, 1.0 + r) * d;
-        return f64_above(r, 0.5) ? d : f64_scale<1>(r) * d;
-      }
-      const double xi = div_rn(2.0, 1.0 + r);
-      return fmin_ref(div_rn(r * (1.0 + r), 1.0 + r * r), xi) * d;
+    if (type == 3 || f64_hi(r) >= 0x7ff00000u) {
+      phi = limiter_phi(type, 0.0, r);
+    } else if (type == 1) {
+      phi = div_rn(big ? 2.0 : f64_scale<1>(r), 1.0 + r);
+    } else {
+      phi = (type == 2) ? r : f64_above(r, 0.5) ? 1.0 : f64_scale<1>(r);
+      if (big) phi = div_rn(2.0, 1.0 + r);
     }
   } else {
     const double h = 0.5 * (1.0 + w);
     d = h * d_L + h * d_R;
+    phi = limiter_phi(type, w, r);
   }
-  const double xi = div_rn(2.0, 1.0 - w + (1.0 + w) * r);
-  if (type == 1) return fmin_ref(div_rn(f64_scale<1>(r), 1.0 + r), xi) * d;
-  if (type == 2) return (f64_above(r, 1.0) ? fmin_ref(1.0, xi) : r) * d;
-  if (type == 3) return fmin_ref(div_rn(r * (1.0 + r), 1.0 + r * r), xi) * d;
-  if (f64_above(r, 1.0)) return fmin_ref(fmin_ref(r, xi), 2.0) * d;
-  return f64_above(r, 0.5) ? d : f64_scale<1>(r) * d;
+  return phi * d;
 }
 
 // The FP32 limiter of the mixed sweeps. With w = 0 the products with

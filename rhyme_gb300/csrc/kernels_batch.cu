@@ -109,21 +109,20 @@ __global__ void __launch_bounds__(128)
     const long long t = w.chunk * kBatchFluxChunk + threadIdx.x;
     const double dt = b.ctl[0];
     if (w.axis == 0) {
-      if (t < face_count<0>(b.g)) faces_elem<D, 0>(G, R, b.U, b.g, 0.5 * dt / b.dx.v[0], b.faces, t);
+      if (t < face_count<0>(b.g)) faces_elem<D, 0>(G, R, b.U, b.g, m_div(m_half(dt), b.dx.v[0]), b.faces, t);
     }
     if constexpr (D > 1) {
-      if (w.axis == 1 && t < face_count<1>(b.g)) faces_elem<D, 1>(G, R, b.U, b.g, 0.5 * dt / b.dx.v[1], b.faces, t);
+      if (w.axis == 1 && t < face_count<1>(b.g)) faces_elem<D, 1>(G, R, b.U, b.g, m_div(m_half(dt), b.dx.v[1]), b.faces, t);
     }
     if constexpr (D > 2) {
-      if (w.axis == 2 && t < face_count<2>(b.g)) faces_elem<D, 2>(G, R, b.U, b.g, 0.5 * dt / b.dx.v[2], b.faces, t);
+      if (w.axis == 2 && t < face_count<2>(b.g)) faces_elem<D, 2>(G, R, b.U, b.g, m_div(m_half(dt), b.dx.v[2]), b.faces, t);
     }
   }
 }
 
-// At least 3 CTAs per SM: the persistent grid is 152 x 3 CTAs (and in 3-D
-// the FP64 solver would otherwise take 216 registers, 2 CTAs per SM).
+// 8 CTAs per SM, as flux_kernel.
 template <int D>
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, 8)
     batch_flux_kernel(Gas<double> G, Rp<double> rp, const BoxDesc* __restrict__ TB,
                       const WorkItem* __restrict__ items, int n, int* head) {
   __shared__ int s_next;
@@ -161,7 +160,7 @@ __global__ void __launch_bounds__(256)
     const double dt = b.ctl[0];
     double dtdx[3];
 #pragma unroll
-    for (int a = 0; a < D; ++a) dtdx[a] = dt / b.dx.v[a];
+    for (int a = 0; a < D; ++a) dtdx[a] = m_div(dt, b.dx.v[a]);
     update_elem<D>(b.solver_type, b.U, b.fluxes, b.g, dtdx, b.V, t);
   }
 }
@@ -188,7 +187,7 @@ cudaError_t batch_step_d(const DevParams& P, const MixedParams& M, bool mixed, c
   if (mixed) return launch_batch_sweeps(M, TB, L, q, st);
   if (L.n_faces) batch_faces_kernel<D><<<std::min(L.n_faces, 152 * 8), 128, 0, st>>>(P.G, TB, L.faces, L.n_faces);
   if (L.n_flux)
-    batch_flux_kernel<D><<<std::min(L.n_flux, 152 * 3), 128, 0, st>>>(P.G, P.rp, TB, L.flux, L.n_flux, L.heads + kHeadFlux);
+    batch_flux_kernel<D><<<std::min(L.n_flux, 152 * 8), 128, 0, st>>>(P.G, P.rp, TB, L.flux, L.n_flux, L.heads + kHeadFlux);
   if (L.n_update) batch_update_kernel<D><<<std::min(L.n_update, 152 * 8), 256, 0, st>>>(TB, L.update, L.n_update);
   return cudaGetLastError();
 }

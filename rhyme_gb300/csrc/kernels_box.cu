@@ -13,10 +13,13 @@
 // interface-axis) and keeps face states and fluxes in device scratch (that
 // traffic is well under 1% of HBM bandwidth at the FP64 rate), and whatever
 // integers compute exactly is kept off the pipe (fp64_int.h: divisions,
-// roots, comparisons, powers of two; with the limiters' spared divisions and
-// the two sides' waves run in common passes, a step of the 2-D 256^2 slab
-// 346 -> 198 us, of 3-D 128^3 17.5 -> 13.2 ms, of 16 boxes of 8..64^3 5.5 ->
-// 2.7 ms).
+// roots, comparisons, powers of two; libm_pow_int.h: most of a power), with
+// the limiters' spared divisions and the two sides' waves run in common
+// passes, and the solve calls those functions instead of inlining them (its
+// warps waited for instructions half of the time): a step of the 2-D 256^2
+// slab 348 -> 118 us, of 3-D 128^3 17.5 -> 6.0 ms, of 16 boxes of 8..64^3 5.5
+// -> 2.0 ms. A third of the FP64 warp instructions of the flux pass that are
+// left run with part of their lanes.
 //
 // This file is compiled with --fmad=false so the double arithmetic performs
 // the same IEEE operations, in the same order, as the reference.
@@ -130,18 +133,18 @@ __global__ void __launch_bounds__(kFaceBlock)
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (axis == 0) {
-    const double h = 0.5 * dt / dx.v[0];
+    const double h = m_div(m_half(dt), dx.v[0]);
     for (long long t = t0; t < face_count<0>(g); t += stride) faces_elem<D, 0>(P.G, R, U, g, h, FS, t);
   }
   if constexpr (D > 1) {
     if (axis == 1) {
-      const double h = 0.5 * dt / dx.v[1];
+      const double h = m_div(m_half(dt), dx.v[1]);
       for (long long t = t0; t < face_count<1>(g); t += stride) faces_elem<D, 1>(P.G, R, U, g, h, FS, t);
     }
   }
   if constexpr (D > 2) {
     if (axis == 2) {
-      const double h = 0.5 * dt / dx.v[2];
+      const double h = m_div(m_half(dt), dx.v[2]);
       for (long long t = t0; t < face_count<2>(g); t += stride) faces_elem<D, 2>(P.G, R, U, g, h, FS, t);
     }
   }
@@ -166,19 +169,15 @@ __device__ __forceinline__ void flux_pass(const DevParams& P, const double* __re
   }
 }
 
+// At least 8 CTAs per SM in 2-D and 3-D (64 registers, some spilled): the
+// solve's chains of dependent FP64 and integer instructions need the warps
+// more than the registers (128^3: 4.96 ms at 3 CTAs, 4.32 at 5, 3.97 at 8,
+// 3.86 at 12; 2-D 256^2: 97 us at 3, 75 at 8). A 1-D box rarely fills the SMs
+// once; there the unbounded kernel is the faster one (512 cells: 31 against
+// 33 us).
 template <int D>
-__global__ void __launch_bounds__(kFluxBlock)
+__global__ void __launch_bounds__(kFluxBlock, D == 1 ? 1 : 8)
     flux_kernel(DevParams P, const double* __restrict__ FS, Geom g, double* __restrict__ FR) {
-  flux_pass<D>(P, FS, g, FR);
-}
-
-// The 3-D pass with at least 3 CTAs per SM (<= 168 registers, some spilled):
-// the FP64 pipe needs the warps to hide its latency more than the solver
-// needs the registers (at 216 registers and 2 CTAs per SM the 256^3 step
-// was 5 % slower). In 1-D and 2-D the unbounded kernel is the faster one.
-template <int D>
-__global__ void __launch_bounds__(kFluxBlock, 3)
-    flux_kernel_3cta(DevParams P, const double* __restrict__ FS, Geom g, double* __restrict__ FR) {
   flux_pass<D>(P, FS, g, FR);
 }
 
@@ -190,7 +189,7 @@ __global__ void __launch_bounds__(kUpdBlock)
   const double dt = *dtp;
   double dtdx[3];
 #pragma unroll
-  for (int a = 0; a < D; ++a) dtdx[a] = dt / dx.v[a];
+  for (int a = 0; a < D; ++a) dtdx[a] = m_div(dt, dx.v[a]);
   const long long total = (long long)g.n[0] * g.n[1] * (long long)g.n[2];
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x)
@@ -215,10 +214,7 @@ cudaError_t mh_solve_d(const DevParams& P, const double* U, double* Unew, const 
   faces_kernel<D><<<gf, kFaceBlock, 0, st>>>(P, rules_of(P), U, g, dx, s.dt, s.faces);
   if (ev) cudaEventRecord(ev[1], st);
   dim3 gr(grid_for(tot_r, kFluxBlock), D);
-  if constexpr (D == 3)
-    flux_kernel_3cta<D><<<gr, kFluxBlock, 0, st>>>(P, s.faces, g, s.fluxes);
-  else
-    flux_kernel<D><<<gr, kFluxBlock, 0, st>>>(P, s.faces, g, s.fluxes);
+  flux_kernel<D><<<gr, kFluxBlock, 0, st>>>(P, s.faces, g, s.fluxes);
   if (ev) cudaEventRecord(ev[2], st);
   const long long tot_u = (long long)g.n[0] * g.n[1] * g.n[2];
   update_kernel<D><<<grid_for(tot_u, kUpdBlock), kUpdBlock, 0, st>>>(P, U, s.fluxes, g, dx, s.dt,
