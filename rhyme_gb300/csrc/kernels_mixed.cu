@@ -118,41 +118,48 @@ __device__ __forceinline__ void block_fold(float m, int bad, unsigned long long*
 // rows of the outermost axis, ghosts included) of a box just copied into U:
 // the FP32 mirror Uf of every cell is written, the ghost cells are copied
 // into the other state buffer V, whose interior the next solve writes, and
-// the FP32 signal speed of every interior cell (the arithmetic of
-// cfl_f32_kernel) is folded into *bits, so that the CFL maximum is ready
-// when the last row has arrived.
+// its mirror Vf, and (bits given) the FP32 signal speed of every interior
+// cell (the arithmetic of cfl_f32_kernel) is folded into *bits, so that the
+// CFL maximum is ready when the last row has arrived. Indexes are split in 32
+// bits (a component block of 2^32 elements does not fit the GPU).
 template <int D>
 __global__ void __launch_bounds__(kThreads)
     ingest_kernel(MixedParams M, const double* __restrict__ U, double* __restrict__ V, float* __restrict__ Uf,
-                  Geom g, long long e0, long long e1, unsigned long long* bits, int* status) {
+                  float* __restrict__ Vf, Geom g, unsigned e0, unsigned e1, unsigned long long* bits, int* status) {
   const long long F = g.field;
-  const long long E0 = g.s[1];                       // row length along x, ghosts included
-  const long long E1 = (D > 2) ? g.s[2] / g.s[1] : 1;  // rows per plane
+  const unsigned E0 = (unsigned)g.n[0] + 4;  // row length along x, ghosts included
+  const unsigned E1 = (unsigned)g.n[1] + 4;  // rows per plane
   float m = 0.f;
   int bad = 0;
-  for (long long t = e0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; t < e1;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % E0);
-    const long long r = t / E0;
-    const int j = (D > 2) ? (int)(r % E1) : (int)r;
-    const int k = (D > 2) ? (int)(r / E1) : 0;
+  for (unsigned long long tt = e0 + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; tt < e1;
+       tt += (unsigned long long)gridDim.x * blockDim.x) {
+    const unsigned t = (unsigned)tt;
+    const unsigned r = (D > 1) ? t / E0 : 0;
+    const int i = (int)(t - r * E0);
     bool in = i >= 2 && i <= g.n[0] + 1;
-    if (D > 1) in = in && j >= 2 && j <= g.n[1] + 1;
-    if (D > 2) in = in && k >= 2 && k <= g.n[2] + 1;
+    if constexpr (D == 2) in = in && (int)r >= 2 && (int)r <= g.n[1] + 1;
+    if constexpr (D > 2) {
+      const unsigned k = r / E1;
+      const int j = (int)(r - k * E1);
+      in = in && j >= 2 && j <= g.n[1] + 1 && (int)k >= 2 && (int)k <= g.n[2] + 1;
+    }
     float u[D + 2];
 #pragma unroll
     for (int c = 0; c < D + 2; ++c) {
       const double x = U[(long long)c * F + t];
       u[c] = mirror_of(x);
       Uf[(long long)c * F + t] = u[c];
-      if (!in) V[(long long)c * F + t] = x;
+      if (!in) {
+        V[(long long)c * F + t] = x;
+        Vf[(long long)c * F + t] = u[c];
+      }
     }
-    if (in) {
+    if (in && bits) {
       const float v = speed_f32<D>(M, u, bad);
       if (v > m) m = v;
     }
   }
-  block_fold(m, bad, bits, status);
+  if (bits) block_fold(m, bad, bits, status);
 }
 
 // dt from a maximum folded by ingest_kernel: the last step of cfl_f32_kernel.
@@ -629,16 +636,18 @@ cudaError_t launch_mh_solve_mixed_slab(const MixedParams& M, const double* U, co
   return e;
 }
 
-cudaError_t launch_ingest_mixed(const MixedParams& M, const double* U, double* V, float* Uf, const Geom& g,
-                                long long e0, long long e1, unsigned long long* bits, int* status,
+cudaError_t launch_ingest_mixed(const MixedParams& M, const double* U, double* V, float* Uf, float* Vf,
+                                const Geom& g, long long e0, long long e1, unsigned long long* bits, int* status,
                                 cudaStream_t st) {
   if (e1 <= e0) return cudaSuccess;
+  if (e1 > 0xffffffffLL) return cudaErrorInvalidValue;
   int grid = grid_for(e1 - e0, kThreads);
   if (grid > 152 * 8) grid = 152 * 8;
+  const unsigned a = (unsigned)e0, b = (unsigned)e1;
   switch (M.ndim) {
-    case 1: ingest_kernel<1><<<grid, kThreads, 0, st>>>(M, U, V, Uf, g, e0, e1, bits, status); break;
-    case 2: ingest_kernel<2><<<grid, kThreads, 0, st>>>(M, U, V, Uf, g, e0, e1, bits, status); break;
-    case 3: ingest_kernel<3><<<grid, kThreads, 0, st>>>(M, U, V, Uf, g, e0, e1, bits, status); break;
+    case 1: ingest_kernel<1><<<grid, kThreads, 0, st>>>(M, U, V, Uf, Vf, g, a, b, bits, status); break;
+    case 2: ingest_kernel<2><<<grid, kThreads, 0, st>>>(M, U, V, Uf, Vf, g, a, b, bits, status); break;
+    case 3: ingest_kernel<3><<<grid, kThreads, 0, st>>>(M, U, V, Uf, Vf, g, a, b, bits, status); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

@@ -13,39 +13,43 @@ namespace rgpu {
 
 namespace {
 
-// Element e of the flattened hydro data of all boxes: box by binary search
-// on the prefix offsets, then component and cell.
+// A CTA packs kPackChunk cells of one component of one box, found by binary
+// search on the boxes' first CTAs; a cell's indexes are split in 32 bits (a
+// box of 2^32 cells does not fit the GPU). Bound by HBM (12 B a value). With
+// a search and 64-bit divisions per value it ran at 1.4 TB/s (27 M values of
+// 96 boxes: 230 us).
 __global__ void __launch_bounds__(256)
-    pack_level_kernel(const PackDesc* __restrict__ D, int n, long long total, int ndim, float* __restrict__ out) {
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (D[mid].hydro_off <= e) lo = mid;
-      else hi = mid - 1;
-    }
-    const PackDesc& d = D[lo];
-    const long long r = e - d.hydro_off;
-    const int c = (int)(r / d.cells);
-    const long long cell = r - (long long)c * d.cells;
-    const long long n0 = d.g.n[0], n1 = d.g.n[1];
-    const int i = (int)(cell % n0) + 1;
-    const long long q = cell / n0;
-    const int j = (int)(q % n1) + 1;
-    const int k = (int)(q / n1) + 1;
-    out[d.out_off + r] = (float)d.U[(long long)c * d.g.field + d.g.at(ndim, i, j, k)];
+    pack_level_kernel(const PackDesc* __restrict__ D, int n, int ndim, float* __restrict__ out) {
+  int lo = 0, hi = n - 1;
+  const long long block = blockIdx.x;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (D[mid].first_block <= block) lo = mid;
+    else hi = mid - 1;
+  }
+  const PackDesc& d = D[lo];
+  const unsigned cells = (unsigned)d.cells, chunks = (cells + kPackChunk - 1) / kPackChunk;
+  const unsigned local = (unsigned)(block - d.first_block);
+  const unsigned c = local / chunks, c0 = (local - c * chunks) * kPackChunk;
+  const unsigned n0 = (unsigned)d.g.n[0], n1 = (unsigned)d.g.n[1];
+  const double* U = d.U + (long long)c * d.g.field;
+  float* o = out + d.out_off + (long long)c * d.cells;
+#pragma unroll
+  for (int i = 0; i < kPackChunk / 256; ++i) {
+    const unsigned cell = c0 + i * 256 + threadIdx.x;
+    if (cell >= cells) break;
+    const unsigned q = cell / n0, k = q / n1;
+    o[cell] = (float)U[d.g.at(ndim, (int)(cell - q * n0) + 1, (int)(q - k * n1) + 1, (int)k + 1)];
   }
 }
 
 }  // namespace
 
-cudaError_t launch_pack_level(const PackDesc* desc, int n, long long total, int ndim, float* out,
+cudaError_t launch_pack_level(const PackDesc* desc, int n, long long blocks, int ndim, float* out,
                               cudaStream_t st) {
-  if (n <= 0 || total <= 0) return cudaSuccess;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 152 * 16) blocks = 152 * 16;
-  pack_level_kernel<<<(int)blocks, 256, 0, st>>>(desc, n, total, ndim, out);
+  if (n <= 0 || blocks <= 0) return cudaSuccess;
+  if (blocks > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  pack_level_kernel<<<(unsigned)blocks, 256, 0, st>>>(desc, n, ndim, out);
   return cudaGetLastError();
 }
 

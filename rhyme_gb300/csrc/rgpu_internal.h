@@ -342,11 +342,11 @@ cudaError_t launch_mh_solve_mixed_slab(const MixedParams& M, const double* U, co
                                        const FallbackQueue& q, int* done, const SweepPlan& plan, int lo, int hi,
                                        cudaStream_t st);
 // Elements [e0, e1) of a box's component blocks just copied into U: their
-// FP32 mirror written to Uf, ghost cells copied into V, FP32 CFL maximum of
-// the interior folded into *bits (launch_cfl_finish turns it into dt as
-// launch_cfl_mixed would).
-cudaError_t launch_ingest_mixed(const MixedParams& M, const double* U, double* V, float* Uf, const Geom& g,
-                                long long e0, long long e1, unsigned long long* bits, int* status,
+// FP32 mirror written to Uf, ghost cells copied into V and its mirror Vf, the
+// FP32 CFL maximum of the interior folded into *bits if given
+// (launch_cfl_finish turns it into dt as launch_cfl_mixed would).
+cudaError_t launch_ingest_mixed(const MixedParams& M, const double* U, double* V, float* Uf, float* Vf,
+                                const Geom& g, long long e0, long long e1, unsigned long long* bits, int* status,
                                 cudaStream_t st);
 cudaError_t launch_cfl_finish(const unsigned long long* bits, double courant, const Dx& dx, const StepScratch& s,
                               cudaStream_t st);
@@ -510,18 +510,20 @@ constexpr int kBatchCflChunk = 2048;
 constexpr int kBatchFluxChunk = 128;
 
 // One box of a level output (kernels_output.cu): its current state, its
-// interior cell count, the start of its hydro elements in the flattened
-// list of all boxes' hydro elements, and its offset in the output dataset
-// (sum over the boxes before it of cells x NCMP).
+// interior cell count, its first CTA (the sum of pack_blocks over the boxes
+// before it) and its offset in the output dataset (sum over the boxes before
+// it of cells x NCMP).
 struct PackDesc {
   const double* U;
   Geom g;
   long long cells;
-  long long hydro_off;
+  long long first_block;
   long long out_off;
 };
+constexpr int kPackChunk = 1024;
+inline long long pack_blocks(int ndim, long long cells) { return (ndim + 2) * ((cells + kPackChunk - 1) / kPackChunk); }
 
-cudaError_t launch_pack_level(const PackDesc* desc, int n, long long total, int ndim, float* out,
+cudaError_t launch_pack_level(const PackDesc* desc, int n, long long blocks, int ndim, float* out,
                               cudaStream_t st);
 
 // Sanity checks (kernels_sanity.cu): the properties of

@@ -451,7 +451,7 @@ int upload_slabs(rhyme_gpu_ctx* ctx, Box* b) {
                          cudaMemcpyHostToDevice, ctx->copy));
     CK(cudaEventRecord(ctx->pipe_ev[j], ctx->copy));
     CK(cudaStreamWaitEvent(ctx->stream, ctx->pipe_ev[j], 0));
-    CK(launch_ingest_mixed(b->mp, U, V, b->Uf[b->cur], b->g, (long long)off, (long long)r1 * row, b->ingest_bits,
+    CK(launch_ingest_mixed(b->mp, U, V, b->Uf[b->cur], b->Uf[1 - b->cur], b->g, (long long)off, (long long)r1 * row, b->ingest_bits,
                            b->s.status, ctx->stream));
   }
   b->mirror_valid = true;
@@ -576,14 +576,17 @@ int rhyme_gpu_sync_to_device(rhyme_gpu_ctx* ctx, int handle) {
   if (!b) return fail(ctx, RHYME_GPU_ENOTFOUND, "unknown box handle %d", handle);
   if (pipelined(ctx, b)) return upload_slabs(ctx, b);
   state_changed(b);
-  // Both buffers receive the full hydro blocks (ghosts and corners included).
+  // The other buffer receives the ghost cells (corners included); in FP64 by
+  // a copy of everything, in mixed precision by the pass that writes the
+  // mirror.
   CK(cudaMemcpyAsync(b->state[b->cur], b->host, b->hydro_bytes, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(b->state[1 - b->cur], b->state[b->cur], b->hydro_bytes, cudaMemcpyDeviceToDevice,
-                     ctx->stream));
   if (ctx->mixed) {
-    const long long n = (long long)(ctx->params.ndim + 2) * b->g.field;
-    CK(launch_to_f32(b->state[b->cur], b->Uf[b->cur], n, ctx->stream));
-    CK(launch_to_f32(b->state[b->cur], b->Uf[1 - b->cur], n, ctx->stream));
+    CK(launch_ingest_mixed(b->mp, b->state[b->cur], b->state[1 - b->cur], b->Uf[b->cur], b->Uf[1 - b->cur], b->g, 0,
+                           b->g.field, nullptr, nullptr, ctx->stream));
+    b->mirror_valid = true;
+  } else {
+    CK(cudaMemcpyAsync(b->state[1 - b->cur], b->state[b->cur], b->hydro_bytes, cudaMemcpyDeviceToDevice,
+                       ctx->stream));
   }
   if (!b->registered_host && !b->host_pinned) return wait_stream(ctx);
   return RHYME_GPU_OK;
@@ -1229,7 +1232,7 @@ extern "C" int rhyme_gpu_output_level(rhyme_gpu_ctx* ctx, const int* handles, in
   const int D = ctx->params.ndim;
   if (ncmp < D + 2) return fail(ctx, RHYME_GPU_EINVAL, "ncmp %d < NDIM+2", ncmp);
   std::vector<PackDesc> desc(n);
-  long long out_len = 0, hydro = 0;
+  long long out_len = 0, blocks = 0;
   for (int i = 0; i < n; ++i) {
     Box* b = find_box(ctx, handles[i]);
     if (!b) return fail(ctx, RHYME_GPU_ENOTFOUND, "unknown box handle %d", handles[i]);
@@ -1237,9 +1240,9 @@ extern "C" int rhyme_gpu_output_level(rhyme_gpu_ctx* ctx, const int* handles, in
     d.U = b->state[b->cur];
     d.g = b->g;
     d.cells = (long long)b->g.n[0] * b->g.n[1] * b->g.n[2];
-    d.hydro_off = hydro;
+    d.first_block = blocks;
     d.out_off = out_len;
-    hydro += (D + 2) * d.cells;
+    blocks += pack_blocks(D, d.cells);
     out_len += (long long)ncmp * d.cells;
   }
   if (capacity < out_len)
@@ -1272,7 +1275,7 @@ extern "C" int rhyme_gpu_output_level(rhyme_gpu_ctx* ctx, const int* handles, in
   }
   // pageable source: the copy is staged before the call returns
   CK(cudaMemcpyAsync(ctx->out_desc, desc.data(), sizeof(PackDesc) * n, cudaMemcpyHostToDevice, ctx->stream));
-  CK(launch_pack_level(ctx->out_desc, n, hydro, D, ctx->out_dev, ctx->stream));
+  CK(launch_pack_level(ctx->out_desc, n, blocks, D, ctx->out_dev, ctx->stream));
   CK(cudaEventRecord(ctx->out_packed, ctx->stream));
   CK(cudaStreamWaitEvent(ctx->copy, ctx->out_packed, 0));
   if (ncmp == D + 2) {
@@ -2069,14 +2072,14 @@ int rhyme_gpu_server_tick(rhyme_gpu_server* S, int* n_active, int* n_pending, in
         pd.U = b->state[b->cur];
         pd.g = b->g;
         pd.cells = q.cells;
-        pd.hydro_off = 0;
+        pd.first_block = 0;
         pd.out_off = 0;
         PackDesc* d_pd = nullptr;
         float* d_out = nullptr;
         cudaError_t e = cudaMallocAsync((void**)&d_pd, sizeof(PackDesc), ctx->stream);
         if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_out, ob, ctx->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_pd, &pd, sizeof(PackDesc), cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess) e = launch_pack_level(d_pd, 1, (long long)(D + 2) * q.cells, D, d_out, ctx->stream);
+        if (e == cudaSuccess) e = launch_pack_level(d_pd, 1, pack_blocks(D, q.cells), D, d_out, ctx->stream);
         cudaEvent_t packed;
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&packed, cudaEventDisableTiming);
         if (e == cudaSuccess) {
