@@ -403,26 +403,45 @@ struct BatchLists {
   bool fill_each;    // ghosts filled in memory every step (FP64, or a box of one cell's extent)
 };
 
-// Tiles of the fused x and y sweep of a batch: 8 x 32, 16 x 16 or 32 x 8
-// cells of a z plane, whichever covers the box's plane with the fewest (a
-// tile costs the same within 2 % whatever its shape; edges of 8, 24, 40 or
-// 56 cells leave half of a 16-cell tile idle), 16 x 16 on a tie.
+// Tile shapes of a 3-D mixed batch, by the warps a box's tiles occupy. Lanes
+// run along x first, so columns beyond the box idle in every row of a tile,
+// while rows beyond it cost nothing; a tile adds two face rows and an
+// interface row of its own along each axis it sweeps (together about 1.05 of
+// a row's instructions). The autotuner's shapes (timed on a box alone, with
+// tensor copies) left the sweeps of 96 boxes of 8..64^3 10 % slower, and its
+// launches are spared.
+// Fused x and y sweep: 8 x 32, 16 x 16 or 32 x 8 cells of a z plane.
 constexpr int kXYShapes = 3;
 __host__ __device__ inline void xy_shape(int k, int* tx, int* ty) {
   *tx = 8 << k;
   *ty = 256 / *tx;
 }
 inline int batch_xy_shape(int nx, int ny) {
-  int best = 1;
-  long long least = 0;
-  for (int i = 0; i < kXYShapes; ++i) {
-    const int k = (i == 0) ? 1 : (i == 1 ? 0 : 2);
+  int best = 0;
+  double least = 0.0;
+  for (int k = 0; k < kXYShapes; ++k) {
     int tx, ty;
     xy_shape(k, &tx, &ty);
-    const long long t = (long long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
-    if (i == 0 || t < least) {
+    const double along_x = (tx + 1.05) * ny, along_y = tx * (ny + 1.05 * ((ny + ty - 1) / ty));
+    const double cost = ((nx + tx - 1) / tx) * (along_x + along_y);
+    if (k == 0 || cost < least) {
       best = k;
-      least = t;
+      least = cost;
+    }
+  }
+  return best;
+}
+// z sweep: S cells by 256/S pencils along x, of 8 at least (32-byte rows).
+inline int batch_z_shape(int nx, int nz) {
+  int best = 0;
+  double least = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    int S, P;
+    sweep_shape(3, k, &S, &P);
+    const double cost = (double)P * ((nx + P - 1) / P) * (nz + 1.05 * ((nz + S - 1) / S));
+    if (k == 0 || cost < least) {
+      best = k;
+      least = cost;
     }
   }
   return best;

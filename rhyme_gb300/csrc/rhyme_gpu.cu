@@ -1575,8 +1575,10 @@ int batch_build(rhyme_gpu_batch* B) {
   long long qcap = 0;
   for (int i = 0; i < n; ++i) {
     Box* b = ctx->boxes[B->handles[i]];
-    int rc = box_plan(ctx, b, b->dx);
-    if (rc != RHYME_GPU_OK) return rc;
+    if (!fuse) {  // (a fused batch's shapes follow from its boxes' sizes)
+      int rc = box_plan(ctx, b, b->dx);
+      if (rc != RHYME_GPU_OK) return rc;
+    }
     B->base_cur[i] = b->cur;
     const long long cells = (long long)b->g.n[0] * b->g.n[1] * b->g.n[2];
     qcap += D * cells / 16;
@@ -1624,7 +1626,7 @@ int batch_build(rhyme_gpu_batch* B) {
         for (long long t = 0; t < nt; ++t) sweep[0][k].push_back({i, 0, t});
       }
       for (int a = fuse ? 2 : 0; a < D; ++a) {
-        const int k = b->plan.shape[a];
+        const int k = fuse ? batch_z_shape(g.n[0], g.n[2]) : b->plan.shape[a];
         const long long nt = sweep_tile_count(D, a, k, g.n);
         for (long long t = 0; t < nt; ++t) sweep[a][k].push_back({i, a, t});
       }

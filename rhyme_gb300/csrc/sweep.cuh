@@ -82,6 +82,15 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_but() {  // all but the last N groups
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// 4 bytes, or 4 zero bytes where !ok (src is then not read).
+__device__ __forceinline__ void cp_async4_or_zero(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(ok ? 4 : 0)
+               : "memory");
+}
 
 // Sweep modes: the flux difference X of this axis becomes acc = X (FIRST),
 // acc += X (MID), U^{n+1} = U + (acc + X) (LAST) or U^{n+1} = U + X (ONLY).
@@ -263,22 +272,24 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
   };
   auto ix = [&](int la, int lb, int na) -> int { return (A == 0) ? lb * na + la : la * P + lb; };
 
-  // 0. start the copies of the accumulator and U^n of the tile's cells
-  if (PRE_ACC || PRE_U) {
-    for (int it = threadIdx.x; it < S * P; it += TileCfg<S, P>::threads) {
-      int lu, lb;
-      split(it, S, lu, lb);
-      const int ga = a0 + lu, gb = b0 + lb;
-      if (ga > NA || gb > NB) continue;
-      const long long o = offset(ga, gb);
+  // start the copies of the accumulator and U^n of the tile's cells
+  auto prefetch = [&]() {
+    if (PRE_ACC || PRE_U) {
+      for (int it = threadIdx.x; it < S * P; it += TileCfg<S, P>::threads) {
+        int lu, lb;
+        split(it, S, lu, lb);
+        const int ga = a0 + lu, gb = b0 + lb;
+        if (ga > NA || gb > NB) continue;
+        const long long o = offset(ga, gb);
 #pragma unroll
-      for (int c = 0; c < D + 2; ++c) {
-        if (PRE_ACC) cp_async4(&pre_acc[c * S * P + it], &acc[(long long)c * F + o]);
-        if (PRE_U) cp_async8(&pre_u[c * S * P + it], &U[(long long)c * F + o]);
+        for (int c = 0; c < D + 2; ++c) {
+          if (PRE_ACC) cp_async4(&pre_acc[c * S * P + it], &acc[(long long)c * F + o]);
+          if (PRE_U) cp_async8(&pre_u[c * S * P + it], &U[(long long)c * F + o]);
+        }
       }
+      cp_async_commit();
     }
-    cp_async_commit();
-  }
+  };
 
   // the ghost cells of a face that gives them from the interior: fetched now,
   // put in place over what the staging brought
@@ -299,6 +310,7 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
 
   // 1. stage the FP32 slab: cells a0-2 .. a0+S+1 along A
   if (tma.on) {
+    prefetch();
     // one tensor copy of the whole slab (every component), zero-filled
     // beyond the array; coordinates are array indices (Fortran index + 1)
     if (threadIdx.x == 0) {
@@ -327,6 +339,9 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
       s_dtdx[0] = dt * dx.inv_f[A];
       s_dtdx[1] = (0.5f * dt) * dx.inv_f[A];
     }
+    // asynchronous copies, all in flight at once (loads through registers
+    // left the z sweep of a batch waiting for them: 36-50 % of its issue
+    // slots used), the slab before what the tile's end adds to
     for (int it = threadIdx.x; it < (S + 4) * P; it += TileCfg<S, P>::threads) {
       int la, lb;
       split(it, S + 4, la, lb);
@@ -334,8 +349,12 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
       const bool ok = ga <= NA + 2 && gb <= NB;
       const long long o = ok ? offset(ga, gb) : 0;
 #pragma unroll
-      for (int c = 0; c < D + 2; ++c) su[c * PLANE + ixu(la, lb)] = ok ? Uf[(long long)c * F + o] : 0.f;
+      for (int c = 0; c < D + 2; ++c) cp_async4_or_zero(&su[c * PLANE + ixu(la, lb)], &Uf[(long long)c * F + o], ok);
     }
+    cp_async_commit();
+    prefetch();
+    if (PRE_ACC || PRE_U) cp_async_wait_but<1>();
+    else cp_async_wait_all();
   }
   __syncthreads();
   if (lo_halo || hi_halo) {
@@ -613,12 +632,11 @@ __device__ __forceinline__ void sweep_xy_tile(const MixedParams& M, int limiter,
       const int gx = x0 - 2 + px, gy = y0 - 2 + py;
       const bool ok = gx <= NX + 2 && gy <= NY + 2;
       const long long o = ok ? g.at(3, gx, gy, cz) : 0;
-      float v[5];
 #pragma unroll
-      for (int c = 0; c < 5; ++c) v[c] = ok ? Uf[(long long)c * F + o] : 0.f;
-#pragma unroll
-      for (int c = 0; c < 5; ++c) su[c * PL + it] = v[c];
+      for (int c = 0; c < 5; ++c) cp_async4_or_zero(&su[c * PL + it], &Uf[(long long)c * F + o], ok);
     }
+    cp_async_commit();
+    cp_async_wait_all();
   }
   __syncthreads();
   if (patch) {
