@@ -122,10 +122,14 @@ __device__ __forceinline__ void block_fold(float m, int bad, unsigned long long*
 // cell (the arithmetic of cfl_f32_kernel) is folded into *bits, so that the
 // CFL maximum is ready when the last row has arrived. Indexes are split in 32
 // bits (a component block of 2^32 elements does not fit the GPU).
+// With H the elements are read from there, page-locked host memory mapped
+// for the GPU, and written to U as well: one launch per upload of a box too
+// small to be sent in overlapped slabs (the host link carries SM loads as
+// fast as copies; 96 boxes of 3 MB took 2.97 ms as a copy and a pass each).
 template <int D>
 __global__ void __launch_bounds__(kThreads)
-    ingest_kernel(MixedParams M, const double* __restrict__ U, double* __restrict__ V, float* __restrict__ Uf,
-                  float* __restrict__ Vf, Geom g, unsigned e0, unsigned e1, unsigned long long* bits, int* status) {
+    ingest_kernel(MixedParams M, const double* __restrict__ H, double* __restrict__ U, double* __restrict__ V,
+                  float* __restrict__ Uf, float* __restrict__ Vf, Geom g, unsigned e0, unsigned e1, unsigned long long* bits, int* status) {
   const long long F = g.field;
   const unsigned E0 = (unsigned)g.n[0] + 4;  // row length along x, ghosts included
   const unsigned E1 = (unsigned)g.n[1] + 4;  // rows per plane
@@ -143,10 +147,15 @@ __global__ void __launch_bounds__(kThreads)
       const int j = (int)(r - k * E1);
       in = in && j >= 2 && j <= g.n[1] + 1 && (int)k >= 2 && (int)k <= g.n[2] + 1;
     }
+    const double* src = H ? H : U;
+    double x5[D + 2];
     float u[D + 2];
 #pragma unroll
+    for (int c = 0; c < D + 2; ++c) x5[c] = src[(long long)c * F + t];
+#pragma unroll
     for (int c = 0; c < D + 2; ++c) {
-      const double x = U[(long long)c * F + t];
+      const double x = x5[c];
+      if (H) U[(long long)c * F + t] = x;
       u[c] = mirror_of(x);
       Uf[(long long)c * F + t] = u[c];
       if (!in) {
@@ -636,7 +645,7 @@ cudaError_t launch_mh_solve_mixed_slab(const MixedParams& M, const double* U, co
   return e;
 }
 
-cudaError_t launch_ingest_mixed(const MixedParams& M, const double* U, double* V, float* Uf, float* Vf,
+cudaError_t launch_ingest_mixed(const MixedParams& M, const double* H, double* U, double* V, float* Uf, float* Vf,
                                 const Geom& g, long long e0, long long e1, unsigned long long* bits, int* status,
                                 cudaStream_t st) {
   if (e1 <= e0) return cudaSuccess;
@@ -645,9 +654,9 @@ cudaError_t launch_ingest_mixed(const MixedParams& M, const double* U, double* V
   if (grid > 152 * 8) grid = 152 * 8;
   const unsigned a = (unsigned)e0, b = (unsigned)e1;
   switch (M.ndim) {
-    case 1: ingest_kernel<1><<<grid, kThreads, 0, st>>>(M, U, V, Uf, Vf, g, a, b, bits, status); break;
-    case 2: ingest_kernel<2><<<grid, kThreads, 0, st>>>(M, U, V, Uf, Vf, g, a, b, bits, status); break;
-    case 3: ingest_kernel<3><<<grid, kThreads, 0, st>>>(M, U, V, Uf, Vf, g, a, b, bits, status); break;
+    case 1: ingest_kernel<1><<<grid, kThreads, 0, st>>>(M, H, U, V, Uf, Vf, g, a, b, bits, status); break;
+    case 2: ingest_kernel<2><<<grid, kThreads, 0, st>>>(M, H, U, V, Uf, Vf, g, a, b, bits, status); break;
+    case 3: ingest_kernel<3><<<grid, kThreads, 0, st>>>(M, H, U, V, Uf, Vf, g, a, b, bits, status); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

@@ -344,8 +344,9 @@ cudaError_t launch_mh_solve_mixed_slab(const MixedParams& M, const double* U, co
 // Elements [e0, e1) of a box's component blocks just copied into U: their
 // FP32 mirror written to Uf, ghost cells copied into V and its mirror Vf, the
 // FP32 CFL maximum of the interior folded into *bits if given
-// (launch_cfl_finish turns it into dt as launch_cfl_mixed would).
-cudaError_t launch_ingest_mixed(const MixedParams& M, const double* U, double* V, float* Uf, float* Vf,
+// (launch_cfl_finish turns it into dt as launch_cfl_mixed would). H given:
+// they come from there (mapped host memory) and are written to U too.
+cudaError_t launch_ingest_mixed(const MixedParams& M, const double* H, double* U, double* V, float* Uf, float* Vf,
                                 const Geom& g, long long e0, long long e1, unsigned long long* bits, int* status,
                                 cudaStream_t st);
 cudaError_t launch_cfl_finish(const unsigned long long* bits, double courant, const Dx& dx, const StepScratch& s,

@@ -451,12 +451,24 @@ int upload_slabs(rhyme_gpu_ctx* ctx, Box* b) {
                          cudaMemcpyHostToDevice, ctx->copy));
     CK(cudaEventRecord(ctx->pipe_ev[j], ctx->copy));
     CK(cudaStreamWaitEvent(ctx->stream, ctx->pipe_ev[j], 0));
-    CK(launch_ingest_mixed(b->mp, U, V, b->Uf[b->cur], b->Uf[1 - b->cur], b->g, (long long)off, (long long)r1 * row, b->ingest_bits,
+    CK(launch_ingest_mixed(b->mp, nullptr, U, V, b->Uf[b->cur], b->Uf[1 - b->cur], b->g, (long long)off, (long long)r1 * row, b->ingest_bits,
                            b->s.status, ctx->stream));
   }
   b->mirror_valid = true;
   b->maxu_valid = true;
   return RHYME_GPU_OK;
+}
+
+// The GPU's address of the box's page-locked host array, null where it has
+// none (the array is pageable, or the mapping is refused).
+const double* mapped_host(const Box* b) {
+  if (!b->registered_host && !b->host_pinned) return nullptr;
+  void* p = nullptr;
+  if (cudaHostGetDevicePointer(&p, b->host, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return (const double*)p;
 }
 
 int register_box_impl(rhyme_gpu_ctx* ctx, int level, int number, double* cells, const int dims[3], int ghost,
@@ -579,12 +591,15 @@ int rhyme_gpu_sync_to_device(rhyme_gpu_ctx* ctx, int handle) {
   // The other buffer receives the ghost cells (corners included); in FP64 by
   // a copy of everything, in mixed precision by the pass that writes the
   // mirror.
-  CK(cudaMemcpyAsync(b->state[b->cur], b->host, b->hydro_bytes, cudaMemcpyHostToDevice, ctx->stream));
   if (ctx->mixed) {
-    CK(launch_ingest_mixed(b->mp, b->state[b->cur], b->state[1 - b->cur], b->Uf[b->cur], b->Uf[1 - b->cur], b->g, 0,
-                           b->g.field, nullptr, nullptr, ctx->stream));
+    const double* mapped = mapped_host(b);
+    if (!mapped)
+      CK(cudaMemcpyAsync(b->state[b->cur], b->host, b->hydro_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    CK(launch_ingest_mixed(b->mp, mapped, b->state[b->cur], b->state[1 - b->cur], b->Uf[b->cur], b->Uf[1 - b->cur],
+                           b->g, 0, b->g.field, nullptr, nullptr, ctx->stream));
     b->mirror_valid = true;
   } else {
+    CK(cudaMemcpyAsync(b->state[b->cur], b->host, b->hydro_bytes, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(b->state[1 - b->cur], b->state[b->cur], b->hydro_bytes, cudaMemcpyDeviceToDevice,
                        ctx->stream));
   }
