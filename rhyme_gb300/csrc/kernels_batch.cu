@@ -23,7 +23,8 @@ namespace {
 template <int D>
 __global__ void __launch_bounds__(256)
     batch_cfl_kernel(Gas<double> G, double courant, const BoxDesc* __restrict__ T,
-                     const WorkItem* __restrict__ items, int n) {
+                     const WorkItem* __restrict__ items, int n, int* __restrict__ heads) {
+  if (blockIdx.x == 0 && threadIdx.x < kBatchHeads) heads[threadIdx.x] = 0;  // for this step's queues
   __shared__ double sm[8];
   __shared__ int sb[8];
   for (int it = blockIdx.x; it < n; it += gridDim.x) {
@@ -174,13 +175,12 @@ cudaError_t batch_ghosts_d(const BoxDesc* TB, const BatchLists& L, cudaStream_t 
 template <int D>
 cudaError_t batch_step_d(const DevParams& P, const MixedParams& M, bool mixed, const BoxDesc* TB,
                          const BatchLists& L, FallbackQueue q, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(L.heads, 0, kBatchHeads * sizeof(int), st);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   if (mixed) {
-    e = launch_batch_cfl_mixed(M, P.courant, TB, L, st);
+    e = launch_batch_cfl_mixed(M, P.courant, TB, L, q, st);
     if (e != cudaSuccess) return e;
   } else if (L.n_cfl) {
-    batch_cfl_kernel<D><<<std::min(L.n_cfl, 152 * 4), 256, 0, st>>>(P.G, P.courant, TB, L.cfl, L.n_cfl);
+    batch_cfl_kernel<D><<<std::min(L.n_cfl, 152 * 4), 256, 0, st>>>(P.G, P.courant, TB, L.cfl, L.n_cfl, L.heads);
   }
   if (L.fill_each) e = batch_ghosts_d<D>(TB, L, st);
   if (e != cudaSuccess) return e;

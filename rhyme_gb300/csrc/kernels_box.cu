@@ -54,6 +54,7 @@ inline int grid_for(long long total, int block) {
 template <int D, typename T>
 __global__ void __launch_bounds__(kFillBlock)
     ghost_fill_kernel(const __grid_constant__ BoxRules R, T* __restrict__ U, T* __restrict__ M, Geom g, float* __restrict__ Mf) {
+  step_begin();
   const int axis = blockIdx.y / (D + 2), c = blockIdx.y % (D + 2);
   const long long n = ghost_lines(D, g, axis);
   for (long long q = (long long)blockIdx.x * kFillBlock + threadIdx.x; q < n; q += (long long)gridDim.x * kFillBlock)
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(kFillBlock)
 template <int D>
 __global__ void __launch_bounds__(kCflBlock)
     cfl_kernel(DevParams P, const double* __restrict__ U, Geom g, double mdx, StepScratch s) {
+  step_begin();
   const long long total = (long long)g.n[0] * g.n[1] * (long long)g.n[2];
   double m = 0.0;
   int bad = 0;
@@ -128,6 +130,7 @@ template <int D>
 __global__ void __launch_bounds__(kFaceBlock)
     faces_kernel(DevParams P, BoxRules R, const double* __restrict__ U, Geom g, Dx dx,
                  const double* dtp, double* __restrict__ FS) {
+  step_begin();
   const double dt = *dtp;
   const int axis = blockIdx.y;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -178,6 +181,7 @@ __device__ __forceinline__ void flux_pass(const DevParams& P, const double* __re
 template <int D>
 __global__ void __launch_bounds__(kFluxBlock, D == 1 ? 1 : 8)
     flux_kernel(DevParams P, const double* __restrict__ FS, Geom g, double* __restrict__ FR) {
+  step_begin();
   flux_pass<D>(P, FS, g, FR);
 }
 
@@ -186,6 +190,7 @@ template <int D>
 __global__ void __launch_bounds__(kUpdBlock)
     update_kernel(DevParams P, const double* __restrict__ U, const double* __restrict__ FR,
                   Geom g, Dx dx, const double* dtp, double* __restrict__ Unew) {
+  step_begin();
   const double dt = *dtp;
   double dtdx[3];
 #pragma unroll
@@ -211,14 +216,13 @@ cudaError_t mh_solve_d(const DevParams& P, const double* U, double* Unew, const 
   }
   if (ev) cudaEventRecord(ev[0], st);
   dim3 gf(grid_for(tot_f, kFaceBlock), D);
-  faces_kernel<D><<<gf, kFaceBlock, 0, st>>>(P, rules_of(P), U, g, dx, s.dt, s.faces);
+  launch_step(faces_kernel<D>, gf, kFaceBlock, st, P, rules_of(P), U, g, dx, s.dt, s.faces);
   if (ev) cudaEventRecord(ev[1], st);
   dim3 gr(grid_for(tot_r, kFluxBlock), D);
-  flux_kernel<D><<<gr, kFluxBlock, 0, st>>>(P, s.faces, g, s.fluxes);
+  launch_step(flux_kernel<D>, gr, kFluxBlock, st, P, s.faces, g, s.fluxes);
   if (ev) cudaEventRecord(ev[2], st);
   const long long tot_u = (long long)g.n[0] * g.n[1] * g.n[2];
-  update_kernel<D><<<grid_for(tot_u, kUpdBlock), kUpdBlock, 0, st>>>(P, U, s.fluxes, g, dx, s.dt,
-                                                                     Unew);
+  launch_step(update_kernel<D>, grid_for(tot_u, kUpdBlock), kUpdBlock, st, P, U, s.fluxes, g, dx, s.dt, Unew);
   if (ev) cudaEventRecord(ev[3], st);
   return cudaGetLastError();
 }
@@ -232,7 +236,7 @@ cudaError_t ghost_fill_d(const BoxRules& R, T* U, T* U_mirror, const Geom& g, cu
   long long lines = 0;
   for (int a = 0; a < D; ++a) lines = std::max(lines, ghost_lines(D, g, a));
   const dim3 grid(grid_for(lines, kFillBlock), D * (D + 2));
-  ghost_fill_kernel<D, T><<<grid, kFillBlock, 0, st>>>(R, U, U_mirror, g, Uf);
+  launch_step((ghost_fill_kernel<D, T>), grid, kFillBlock, st, R, U, U_mirror, g, Uf);
   return cudaGetLastError();
 }
 
@@ -272,9 +276,9 @@ cudaError_t launch_cfl(const DevParams& P, const double* U, const Geom& g, const
   int grid = grid_for(total, kCflBlock);
   if (grid > 152 * 4) grid = 152 * 4;
   switch (P.ndim) {
-    case 1: cfl_kernel<1><<<grid, kCflBlock, 0, st>>>(P, U, g, dx.min, s); break;
-    case 2: cfl_kernel<2><<<grid, kCflBlock, 0, st>>>(P, U, g, dx.min, s); break;
-    case 3: cfl_kernel<3><<<grid, kCflBlock, 0, st>>>(P, U, g, dx.min, s); break;
+    case 1: launch_step(cfl_kernel<1>, grid, kCflBlock, st, P, U, g, dx.min, s); break;
+    case 2: launch_step(cfl_kernel<2>, grid, kCflBlock, st, P, U, g, dx.min, s); break;
+    case 3: launch_step(cfl_kernel<3>, grid, kCflBlock, st, P, U, g, dx.min, s); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

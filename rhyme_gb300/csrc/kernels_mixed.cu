@@ -253,7 +253,9 @@ template <int D>
 __global__ void __launch_bounds__(kThreads)
     cfl_carry_kernel(MixedParams M, const double* __restrict__ U, float* __restrict__ Uf, Geom g, double courant,
                      double mdx, StepScratch s, unsigned long long* carry_bits, int* carry_ok,
-                     const int* __restrict__ prev_fix) {
+                     const int* __restrict__ prev_fix, int* __restrict__ this_fix) {
+  step_begin();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *this_fix = 0;
   const bool use = *carry_ok != 0 && *prev_fix == 0;
   if (use) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -399,6 +401,7 @@ __global__ void __launch_bounds__(128)
     fallback_fix_kernel(MixedParams M, FallbackQueue q, Geom g, Dx dx, const double* __restrict__ dtp,
                         const double* __restrict__ U, double* __restrict__ Unew, const int* __restrict__ from,
                         const __grid_constant__ FixBC fbc) {
+  step_begin();
   const int n = min(*q.n, q.cap);
   const int lo = from ? min(*from, n) : 0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && n > lo) atomicAdd(q.total, n - lo);
@@ -429,7 +432,7 @@ cudaError_t launch_fallback(const MixedParams& M, const FallbackQueue& q, const 
     fbc.bc[i] = halo.type[i];
     for (int c = 0; c < 5; ++c) fbc.inflow[i][c] = halo.inflow64[i][c];
   }
-  fallback_fix_kernel<D><<<152, 128, 0, st>>>(M, q, g, dx, dtp, U, Unew, from, fbc);
+  launch_step(fallback_fix_kernel<D>, 152, 128, st, M, q, g, dx, dtp, U, Unew, from, fbc);
   return cudaGetLastError();
 }
 
@@ -442,7 +445,12 @@ cudaError_t launch_fallback(const MixedParams& M, const FallbackQueue& q, const 
 template <int D>
 __global__ void __launch_bounds__(256)
     batch_cfl_f32_kernel(MixedParams M, double courant, const BoxDesc* __restrict__ TB,
-                         const WorkItem* __restrict__ items, int n, const int* __restrict__ whole) {
+                         const WorkItem* __restrict__ items, int n, const int* __restrict__ whole,
+                         int* __restrict__ heads, int* __restrict__ queued) {
+  if (blockIdx.x == 0) {  // for this step's queues
+    if (threadIdx.x < kBatchHeads) heads[threadIdx.x] = 0;
+    if (threadIdx.x == 0) *queued = 0;
+  }
   __shared__ float sm[8];
   __shared__ int sb[8];
   const bool all = *whole != 0;
@@ -560,19 +568,19 @@ cudaError_t launch_cfl_mixed(const MixedParams& M, const double* U, float* Uf, c
 
 cudaError_t launch_cfl_carry(const MixedParams& M, const double* U, float* Uf, const Geom& g, double courant,
                              const Dx& dx, const StepScratch& s, unsigned long long* carry_bits, int* carry_ok,
-                             const int* prev_fix, cudaStream_t st) {
+                             const int* prev_fix, int* this_fix, cudaStream_t st) {
   const long long total = (long long)g.n[0] * g.n[1] * g.n[2];
   int grid = grid_for(total, kThreads);
   if (grid > 152 * 4) grid = 152 * 4;
   switch (M.ndim) {
     case 1:
-      cfl_carry_kernel<1><<<grid, kThreads, 0, st>>>(M, U, Uf, g, courant, dx.min, s, carry_bits, carry_ok, prev_fix);
+      launch_step(cfl_carry_kernel<1>, grid, kThreads, st, M, U, Uf, g, courant, dx.min, s, carry_bits, carry_ok, prev_fix, this_fix);
       break;
     case 2:
-      cfl_carry_kernel<2><<<grid, kThreads, 0, st>>>(M, U, Uf, g, courant, dx.min, s, carry_bits, carry_ok, prev_fix);
+      launch_step(cfl_carry_kernel<2>, grid, kThreads, st, M, U, Uf, g, courant, dx.min, s, carry_bits, carry_ok, prev_fix, this_fix);
       break;
     case 3:
-      cfl_carry_kernel<3><<<grid, kThreads, 0, st>>>(M, U, Uf, g, courant, dx.min, s, carry_bits, carry_ok, prev_fix);
+      launch_step(cfl_carry_kernel<3>, grid, kThreads, st, M, U, Uf, g, courant, dx.min, s, carry_bits, carry_ok, prev_fix, this_fix);
       break;
     default: return cudaErrorInvalidValue;
   }
@@ -583,14 +591,14 @@ cudaError_t launch_mh_solve_mixed(const MixedParams& M, const double* U, const f
                                   double* Unew, float* acc, const Geom& g,
                                   const Dx& dx, const StepScratch& s, const FallbackQueue& q,
                                   const SweepPlan& plan, cudaStream_t st, const HaloBC& halo, cudaEvent_t* ev,
-                                  const SweepCarry& carry, int* fused) {
+                                  const SweepCarry& carry, int* fused, bool queue_reset) {
   // ev (optional, 3 events): recorded after the x sweep, after the y sweep
   // and at the end (the z sweep and the FP64 fix-up); absent axes record
   // at the same point, and so do both when one kernel ran the x and y
   // sweeps (*fused, optional, is then 1).
   const int D = M.ndim;
   if (D < 1 || D > 3) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(q.n, 0, sizeof(int), st);
+  cudaError_t e = queue_reset ? cudaMemsetAsync(q.n, 0, sizeof(int), st) : cudaSuccess;
   int first = 0;
   if (fused) *fused = 0;
   if (e == cudaSuccess && D == 3 && plan.fuse_xy) {
@@ -680,13 +688,13 @@ long long sweep_tile_count(int ndim, int axis, int shape, const int* n) {
 }
 
 cudaError_t launch_batch_cfl_mixed(const MixedParams& M, double courant, const BoxDesc* TB,
-                                   const BatchLists& L, cudaStream_t st) {
+                                   const BatchLists& L, const FallbackQueue& q, cudaStream_t st) {
   if (!L.n_cfl) return cudaSuccess;
   const int grid = L.n_cfl < 152 * 8 ? L.n_cfl : 152 * 8;
   switch (M.ndim) {
-    case 1: batch_cfl_f32_kernel<1><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole); break;
-    case 2: batch_cfl_f32_kernel<2><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole); break;
-    case 3: batch_cfl_f32_kernel<3><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole); break;
+    case 1: batch_cfl_f32_kernel<1><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole, L.heads, q.n); break;
+    case 2: batch_cfl_f32_kernel<2><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole, L.heads, q.n); break;
+    case 3: batch_cfl_f32_kernel<3><<<grid, 256, 0, st>>>(M, courant, TB, L.cfl, L.n_cfl, L.whole, L.heads, q.n); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -699,7 +707,7 @@ cudaError_t launch_batch_sweeps(const MixedParams& M, const BoxDesc* TB, const B
                                 const FallbackQueue& q, cudaStream_t st) {
   const int D = M.ndim;
   if (D < 1 || D > 3) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(q.n, 0, sizeof(int), st);
+  cudaError_t e = cudaSuccess;
   for (int a = 0; a < D; ++a)
     for (int k = 0; k < kSweepShapes; ++k)
       if (e == cudaSuccess && L.n_sweep[a][k]) {

@@ -35,6 +35,10 @@ namespace {
 constexpr int kPipeSlabs = 16;
 constexpr size_t kPipeMinBytes = size_t(16) << 20;
 
+// Steps of a resident run in one graph (even, so that it ends in the buffer
+// it began with).
+constexpr int kGraphSteps = 4;
+
 struct Box {
   int level = 0, number = 0;
   double* host = nullptr;
@@ -53,7 +57,7 @@ struct Box {
   int* trace_pos = nullptr;
   bool registered_host = false;
   bool host_pinned = false;  // host array is page-locked (no wait after upload)
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  cudaGraphExec_t graph[4] = {};  // one step by parity, then kGraphSteps steps by parity
   Dx graph_dx{};
   bool graph_valid = false;
   DevParams dp{};   // the context's parameters with this box's overrides
@@ -79,6 +83,7 @@ struct Box {
   // carry_valid: nothing changed the state since the last resident run
   unsigned long long* carry_bits = nullptr;
   int* carry_ok = nullptr;
+  int* fb_other = nullptr;  // the queue length of a resident run's odd steps (fbq.n: the even ones')
   bool carry_valid = false;
   bool batch_carry = false;  // likewise since the last batch run
   bool wb = false;
@@ -278,8 +283,9 @@ void make_mixed_params(const DevParams& d, MixedParams* m) {
 // already queued there) and unpins the caller's array.
 void destroy_box(Box* b, cudaStream_t st) {
   if (!b) return;
+  for (cudaGraphExec_t g : b->graph)
+    if (g) cudaGraphExecDestroy(g);
   for (int i = 0; i < 2; ++i) {
-    if (b->graph[i]) cudaGraphExecDestroy(b->graph[i]);
     if (b->state[i]) cudaFreeAsync(b->state[i], st);
     if (b->Uf[i]) cudaFreeAsync(b->Uf[i], st);
   }
@@ -528,6 +534,7 @@ int register_box_impl(rhyme_gpu_ctx* ctx, int level, int number, double* cells, 
   b->ingest_bits = (unsigned long long*)(base + 40);
   b->carry_bits = (unsigned long long*)(base + 48);
   b->carry_ok = (int*)(base + 56);
+  b->fb_other = (int*)(base + 60);
   b->fbq.status = b->s.status;
   b->fbq.total = b->fb_count;
   b->trace_buf = (double*)(base + 64);
@@ -838,6 +845,15 @@ cudaError_t fill_after_run(rhyme_gpu_ctx* ctx, Box* b) {
   return launch_ghost_fill(b->dp, b->state[1 - b->cur], b->state[b->cur], b->g, ctx->stream);
 }
 
+// The fix-up queue of a resident step that reads buffer `cur`: one length
+// counter per parity, zeroed by the step's CFL pass while the previous step's
+// is still read.
+FallbackQueue queue_of(const Box* b, int cur) {
+  FallbackQueue q = b->fbq;
+  if (cur) q.n = b->fb_other;
+  return q;
+}
+
 // In mixed precision the step carries its CFL pass into the next one: the
 // next step's CFL pass only forms dt from the carried maximum (unless the
 // FP64 fix-up changed cells after the sweep; launch_cfl_carry).
@@ -845,44 +861,52 @@ cudaError_t enqueue_step(rhyme_gpu_ctx* ctx, Box* b, int cur, const Dx& dx, bool
   StepScratch s = scratch_of(b, trace);
   double* U = b->state[cur];
   double* V = b->state[1 - cur];
+  const FallbackQueue q = queue_of(b, cur);
   cudaError_t e = ctx->mixed ? launch_cfl_carry(b->mp, U, b->Uf[cur], b->g, b->dp.courant, dx, s, b->carry_bits,
-                                                b->carry_ok, b->fbq.n, ctx->stream)
+                                                b->carry_ok, queue_of(b, 1 - cur).n, q.n, ctx->stream)
                              : launch_cfl(b->dp, U, b->g, dx, s, ctx->stream);
   if (e == cudaSuccess && !fills_last(ctx, b))
     e = launch_ghost_fill(b->dp, U, V, b->g, ctx->stream, ctx->mixed ? b->Uf[cur] : nullptr);
   if (e != cudaSuccess) return e;
   if (ctx->mixed)
-    return launch_mh_solve_mixed(b->mp, U, b->Uf[cur], V, b->acc, b->g, dx, s, b->fbq, b->plan, ctx->stream,
-                                 box_halo(ctx, b), nullptr, carry_of(b, cur));
+    return launch_mh_solve_mixed(b->mp, U, b->Uf[cur], V, b->acc, b->g, dx, s, q, b->plan, ctx->stream,
+                                 box_halo(ctx, b), nullptr, carry_of(b, cur), nullptr, false);
   return launch_mh_solve(b->dp, U, V, b->g, dx, s, ctx->stream);
 }
 
-int ensure_graphs(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx) {
-  if (b->graph_valid && memcmp(&b->graph_dx, &dx, sizeof(Dx)) == 0) return RHYME_GPU_OK;
-  int prc = box_plan(ctx, b, dx);
-  if (prc != RHYME_GPU_OK) return prc;
-  for (int i = 0; i < 2; ++i) {
-    if (b->graph[i]) {
-      cudaGraphExecDestroy(b->graph[i]);
-      b->graph[i] = nullptr;
+// The graph of 1 or kGraphSteps steps from buffer `cur`, captured on first
+// use: kernels of one graph follow each other without the host's launch gap,
+// so runs of several steps replay longer graphs.
+int step_graph(rhyme_gpu_ctx* ctx, Box* b, int cur, bool many, const Dx& dx, cudaGraphExec_t* out) {
+  if (!b->graph_valid || memcmp(&b->graph_dx, &dx, sizeof(Dx)) != 0) {
+    int prc = box_plan(ctx, b, dx);
+    if (prc != RHYME_GPU_OK) return prc;
+    for (cudaGraphExec_t& g : b->graph) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
     }
+    b->graph_dx = dx;
+    b->graph_valid = true;
   }
-  for (int parity = 0; parity < 2; ++parity) {
+  cudaGraphExec_t& exec = b->graph[cur + (many ? 2 : 0)];
+  if (!exec) {
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = enqueue_step(ctx, b, parity, dx, true);
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < (many ? kGraphSteps : 1) && e == cudaSuccess; ++k) e = enqueue_step(ctx, b, (cur + k) & 1, dx, true);
     cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
     if (e != cudaSuccess || e2 != cudaSuccess) {
       if (e2 == cudaSuccess) cudaGraphDestroy(graph);
-      return fail(ctx, RHYME_GPU_ECUDA, "graph capture: %s",
-                  cudaGetErrorString(e != cudaSuccess ? e : e2));
+      return fail(ctx, RHYME_GPU_ECUDA, "graph capture: %s", cudaGetErrorString(e != cudaSuccess ? e : e2));
     }
-    cudaError_t e3 = cudaGraphInstantiate(&b->graph[parity], graph, 0);
+    cudaError_t e3 = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (e3 != cudaSuccess) return fail(ctx, RHYME_GPU_ECUDA, "graph instantiate: %s", cudaGetErrorString(e3));
+    if (e3 != cudaSuccess) {
+      exec = nullptr;
+      return fail(ctx, RHYME_GPU_ECUDA, "graph instantiate: %s", cudaGetErrorString(e3));
+    }
   }
-  b->graph_dx = dx;
-  b->graph_valid = true;
+  *out = exec;
   return RHYME_GPU_OK;
 }
 
@@ -1020,7 +1044,8 @@ int rhyme_gpu_run(rhyme_gpu_ctx* ctx, int handle, const double dx[3], int nsteps
   Box* b = find_box(ctx, handle);
   if (!b) return fail(ctx, RHYME_GPU_ENOTFOUND, "unknown box handle %d", handle);
   Dx d = make_dx(ctx->params.ndim, dx);
-  int rc = ensure_graphs(ctx, b, d);
+  cudaGraphExec_t exec;
+  int rc = step_graph(ctx, b, b->cur, nsteps >= kGraphSteps, d, &exec);
   if (rc != RHYME_GPU_OK) return rc;
   if (nsteps == 0) return RHYME_GPU_OK;
   // a state changed since the last resident run: its first CFL pass is whole
@@ -1031,9 +1056,13 @@ int rhyme_gpu_run(rhyme_gpu_ctx* ctx, int handle, const double dx[3], int nsteps
   while (done < nsteps) {
     const int chunk = (nsteps - done < kTraceCap) ? nsteps - done : kTraceCap;
     CK(cudaMemsetAsync(b->trace_pos, 0, sizeof(int), ctx->stream));
-    for (int s = 0; s < chunk; ++s) {
-      CK(cudaGraphLaunch(b->graph[b->cur], ctx->stream));
-      b->cur = 1 - b->cur;
+    for (int s = 0; s < chunk;) {
+      const bool many = chunk - s >= kGraphSteps;
+      rc = step_graph(ctx, b, b->cur, many, d, &exec);
+      if (rc != RHYME_GPU_OK) return rc;
+      CK(cudaGraphLaunch(exec, ctx->stream));
+      s += many ? kGraphSteps : 1;
+      if (!many) b->cur = 1 - b->cur;
     }
     if (done + chunk == nsteps) CK(fill_after_run(ctx, b));
     if (dt_trace) {
@@ -1186,14 +1215,15 @@ extern "C" int rhyme_gpu_profile_steps(rhyme_gpu_ctx* ctx, int handle, const dou
       // FP64 fix-up of the queued interfaces and the carried CFL pass)
       if (e == cudaSuccess)
         e = launch_cfl_carry(b->mp, U, b->Uf[b->cur], b->g, b->dp.courant, d, sc, b->carry_bits, b->carry_ok,
-                             b->fbq.n, ctx->stream);
+                             queue_of(b, 1 - b->cur).n, queue_of(b, b->cur).n, ctx->stream);
       if (e == cudaSuccess) e = cudaEventRecord(ev[1], ctx->stream);
       if (e == cudaSuccess && !fills_last(ctx, b))
         e = launch_ghost_fill(b->dp, U, V, b->g, ctx->stream, b->Uf[b->cur]);
       if (e == cudaSuccess) e = cudaEventRecord(ev[2], ctx->stream);
       if (e == cudaSuccess)
         e = launch_mh_solve_mixed(b->mp, U, b->Uf[b->cur], V, b->acc, b->g, d, sc,
-                                  b->fbq, b->plan, ctx->stream, box_halo(ctx, b), ev + 3, carry_of(b, b->cur), &fused);
+                                  queue_of(b, b->cur), b->plan, ctx->stream, box_halo(ctx, b), ev + 3,
+                                  carry_of(b, b->cur), &fused, false);
     } else {
       if (e == cudaSuccess) e = launch_cfl(b->dp, U, b->g, d, sc, ctx->stream);
       if (e == cudaSuccess) e = cudaEventRecord(ev[1], ctx->stream);

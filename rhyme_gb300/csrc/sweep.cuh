@@ -482,6 +482,7 @@ __global__ void __launch_bounds__(TileCfg<S, P>::threads, TileCfg<S, P>::templat
                  Dx dx, const double* __restrict__ dtp, float* __restrict__ acc,
                  double* __restrict__ Unew, FallbackQueue q, const __grid_constant__ CUtensorMap map,
                  int tma_on, int o_off, SweepCarry carry, const __grid_constant__ HaloBC halo) {
+  step_begin();
   constexpr int C = Axes<D, A>::C;
   __shared__ SweepSmem<D, S, P> sh;
   __shared__ __align__(8) unsigned long long bar;
@@ -765,6 +766,7 @@ __global__ void __launch_bounds__(XYCfg<TX, TY>::threads, XYCfg<TX, TY>::ctas)
     sweep_xy_kernel(MixedParams M, const float* __restrict__ Uf, Geom g, Dx dx, const double* __restrict__ dtp,
                     float* __restrict__ acc, FallbackQueue q, const __grid_constant__ CUtensorMap map,
                     const __grid_constant__ HaloBC halo) {
+  step_begin();
   __shared__ XYSmem<TX, TY> sh;
   __shared__ __align__(8) unsigned long long bar;
   if (threadIdx.x == 0) mbar_init(&bar);

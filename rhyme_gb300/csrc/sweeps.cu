@@ -61,9 +61,8 @@ cudaError_t launch_one(const MixedParams& M, const float* Uf, const double* U, c
   const int tma_on = encode_mirror_map(&map, Uf, g, D, A, S, P) ? 1 : 0;
   SweepCarry cs = carry;
   if (cs.Uf_next) cs.Uf_next += shift;
-  sweep_kernel<D, A, S, P, mode_of<D, A>()><<<grid, TileCfg<S, P>::threads, 0, st>>>(
+  return launch_step(sweep_kernel<D, A, S, P, mode_of<D, A>()>, grid, dim3(TileCfg<S, P>::threads), st,
       M, Uf + shift, U + shift, gs, dx, dtp, acc + shift, Unew + shift, qs, map, tma_on, lo - 1, cs, halo);
-  return cudaGetLastError();
 }
 
 template <int D, int A, int S, int P>
@@ -170,9 +169,8 @@ cudaError_t launch_sweep_xy_3(const MixedParams& M, const float* Uf, const Geom&
   CUtensorMap map;
   memset(&map, 0, sizeof map);
   if (!encode_xy_map(&map, Uf, g, TX, TY)) return cudaErrorNotSupported;
-  sweep_xy_kernel<TX, TY><<<dim3(gx, gy, (unsigned)g.n[2]), XYCfg<TX, TY>::threads, 0, st>>>(M, Uf, g, dx, dtp, acc,
-                                                                                             q, map, halo);
-  return cudaGetLastError();
+  return launch_step(sweep_xy_kernel<TX, TY>, dim3(gx, gy, (unsigned)g.n[2]), dim3(XYCfg<TX, TY>::threads), st, M, Uf, g,
+                     dx, dtp, acc, q, map, halo);
 }
 
 namespace {
