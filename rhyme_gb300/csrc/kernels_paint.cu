@@ -25,9 +25,10 @@ __device__ __forceinline__ void to_cons(const Gas<double>& G, const double* w, d
 
 template <int D>
 __global__ void __launch_bounds__(256)
-    paint_kernel(const PaintShape* __restrict__ shapes, int n, Gas<double> G, Geom g, int le0, int le1, int le2,
+    paint_kernel(const PaintShape* __restrict__ list, const __grid_constant__ PaintList few, int n, Gas<double> G, Geom g, int le0, int le1, int le2,
                  double* __restrict__ U, float* __restrict__ Uf) {
   constexpr int K = D + 2;
+  const PaintShape* shapes = list ? list : few.s;
   const double pi = 4.0 * atan(1.0);
   const long long total = (long long)g.n[0] * g.n[1] * g.n[2];
   const int le[3] = {le0, le1, le2};
@@ -143,16 +144,16 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace
 
-cudaError_t launch_paint(int ndim, const PaintShape* shapes, int n, const Gas<double>& G, const Geom& g,
+cudaError_t launch_paint(int ndim, const PaintShape* shapes, const PaintList& few, int n, const Gas<double>& G, const Geom& g,
                          const int* left_edge, double* U, float* Uf, cudaStream_t st) {
   const long long total = (long long)g.n[0] * g.n[1] * g.n[2];
   long long blocks = (total + 255) / 256;
   if (blocks > 152 * 16) blocks = 152 * 16;
   if (blocks < 1) blocks = 1;
   switch (ndim) {
-    case 1: paint_kernel<1><<<(int)blocks, 256, 0, st>>>(shapes, n, G, g, left_edge[0], left_edge[1], left_edge[2], U, Uf); break;
-    case 2: paint_kernel<2><<<(int)blocks, 256, 0, st>>>(shapes, n, G, g, left_edge[0], left_edge[1], left_edge[2], U, Uf); break;
-    case 3: paint_kernel<3><<<(int)blocks, 256, 0, st>>>(shapes, n, G, g, left_edge[0], left_edge[1], left_edge[2], U, Uf); break;
+    case 1: paint_kernel<1><<<(int)blocks, 256, 0, st>>>(shapes, few, n, G, g, left_edge[0], left_edge[1], left_edge[2], U, Uf); break;
+    case 2: paint_kernel<2><<<(int)blocks, 256, 0, st>>>(shapes, few, n, G, g, left_edge[0], left_edge[1], left_edge[2], U, Uf); break;
+    case 3: paint_kernel<3><<<(int)blocks, 256, 0, st>>>(shapes, few, n, G, g, left_edge[0], left_edge[1], left_edge[2], U, Uf); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

@@ -572,7 +572,8 @@ struct PackDesc {
 constexpr int kPackChunk = 1024;
 inline long long pack_blocks(int ndim, long long cells) { return (ndim + 2) * ((cells + kPackChunk - 1) / kPackChunk); }
 
-cudaError_t launch_pack_level(const PackDesc* desc, int n, long long blocks, int ndim, float* out,
+// desc: n boxes in device memory, or null: the one box of `one`.
+cudaError_t launch_pack_level(const PackDesc* desc, const PackDesc& one, int n, long long blocks, int ndim, float* out,
                               cudaStream_t st);
 
 // Sanity checks (kernels_sanity.cu): the properties of
@@ -618,7 +619,13 @@ struct PaintShape {
   double base[5];
 };
 
-cudaError_t launch_paint(int ndim, const PaintShape* shapes, int n, const Gas<double>& G, const Geom& g,
+// A list of shapes short enough for the kernel's parameters.
+constexpr int kPaintFew = 8;
+struct PaintList {
+  PaintShape s[kPaintFew];
+};
+// shapes: n shapes in device memory, or null: the first n of `few`.
+cudaError_t launch_paint(int ndim, const PaintShape* shapes, const PaintList& few, int n, const Gas<double>& G, const Geom& g,
                          const int* left_edge, double* U, float* Uf, cudaStream_t st);
 
 // Element-level launchers (kernels_elem.cu): device arrays in and out.

@@ -46,6 +46,8 @@ struct Box {
   int ncmp = 0;
   Geom g{};
   size_t hydro_bytes = 0;  // (NDIM+2) component blocks
+  char* mem = nullptr;     // the device memory that the arrays below share
+  size_t zero_bytes = 0;   // its first part: the states and their mirrors
   double* state[2] = {nullptr, nullptr};
   int cur = 0;
   StepScratch s{};
@@ -102,6 +104,7 @@ struct rhyme_gpu_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   std::vector<Box*> boxes;
+  cudaMemPool_t pool = nullptr;  // the boxes' and batches' device memory (device_alloc)
   double* pinned_dt = nullptr;   // pinned host scalars read back synchronously (dt, status, totals)
   void* elem_buf = nullptr;      // growable device buffer for element calls
   size_t elem_cap = 0;
@@ -143,6 +146,28 @@ int fail(rhyme_gpu_ctx* ctx, int code, const char* fmt, ...) {
       return fail(ctx, e_ == cudaErrorMemoryAllocation ? RHYME_GPU_ENOMEM : RHYME_GPU_ECUDA, \
                   "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);   \
   } while (0)
+
+// Device memory in stream order from the context's own pool, which keeps up
+// to 1 GiB of what is freed (the default pool gives everything back at each
+// synchronisation, and a server admitting boxes paid for the mapping again);
+// destroyed with the context.
+cudaError_t device_alloc(rhyme_gpu_ctx* ctx, void** p, size_t bytes) {
+  if (!ctx->pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
+    if (e != cudaSuccess) {
+      ctx->pool = nullptr;
+      return e;
+    }
+    uint64_t keep = uint64_t(1) << 30;
+    e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+}
 
 // Bounded wait on the context stream: polls an event until the deadline.
 int wait_stream(rhyme_gpu_ctx* ctx) {
@@ -285,15 +310,7 @@ void destroy_box(Box* b, cudaStream_t st) {
   if (!b) return;
   for (cudaGraphExec_t g : b->graph)
     if (g) cudaGraphExecDestroy(g);
-  for (int i = 0; i < 2; ++i) {
-    if (b->state[i]) cudaFreeAsync(b->state[i], st);
-    if (b->Uf[i]) cudaFreeAsync(b->Uf[i], st);
-  }
-  if (b->acc) cudaFreeAsync(b->acc, st);
-  if (b->fbq.e) cudaFreeAsync(b->fbq.e, st);
-  if (b->s.faces) cudaFreeAsync(b->s.faces, st);
-  if (b->s.fluxes) cudaFreeAsync(b->s.fluxes, st);
-  if (b->s.dt) cudaFreeAsync(b->s.dt, st);
+  if (b->mem) cudaFreeAsync(b->mem, st);
   if (b->registered_host) cudaHostUnregister(b->host);
   delete b;
 }
@@ -363,6 +380,7 @@ int rhyme_gpu_destroy(rhyme_gpu_ctx* ctx) {
   if (ctx->wb_done) cudaEventDestroy(ctx->wb_done);
   if (ctx->copy) cudaStreamDestroy(ctx->copy);
   cudaFreeHost(ctx->pinned_dt);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return RHYME_GPU_OK;
@@ -500,29 +518,46 @@ int register_box_impl(rhyme_gpu_ctx* ctx, int level, int number, double* cells, 
   const long long F = b->g.field;
   b->hydro_bytes = (size_t)(D + 2) * F * sizeof(double);
   cudaStream_t st = ctx->stream;
-  cudaError_t e = cudaSuccess;
-  for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMallocAsync((void**)&b->state[i], b->hydro_bytes, st);
+  // one allocation, its parts aligned to 256 bytes, the FP32 mirrors right
+  // after the states
+  size_t bytes = 0;
+  auto part = [&](size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t small = 64 + sizeof(double) * kTraceCap;  // dt, max_bits, counter, status, trace_pos, the trace
+  const size_t at_state[2] = {part(b->hydro_bytes), part(b->hydro_bytes)};
+  size_t at_mirror[2] = {0, 0}, at_acc = 0, at_queue = 0, at_faces = 0, at_fluxes = 0;
   if (ctx->mixed) {
-    for (int i = 0; i < 2 && e == cudaSuccess; ++i)
-      e = cudaMallocAsync((void**)&b->Uf[i], (size_t)(D + 2) * F * sizeof(float), st);
-    if (e == cudaSuccess && D > 1) e = cudaMallocAsync((void**)&b->acc, (size_t)(D + 2) * F * sizeof(float), st);
-    long long cells_n = (long long)b->g.n[0] * b->g.n[1] * b->g.n[2];
+    for (size_t& at : at_mirror) at = part((size_t)(D + 2) * F * sizeof(float));
+    if (D > 1) at_acc = part((size_t)(D + 2) * F * sizeof(float));
+    const long long cells_n = (long long)b->g.n[0] * b->g.n[1] * b->g.n[2];
     b->fbq.cap = (int)std::min<long long>(std::max<long long>(4096, D * cells_n / 16), 1LL << 30);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&b->fbq.e, (size_t)b->fbq.cap * sizeof(FallbackEntry), st);
+    at_queue = part((size_t)b->fbq.cap * sizeof(FallbackEntry));
   } else {
-    if (e == cudaSuccess)
-      e = cudaMallocAsync((void**)&b->s.faces, (size_t)2 * D * (D + 2) * F * sizeof(double), st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&b->s.fluxes, (size_t)D * (D + 2) * F * sizeof(double), st);
+    at_faces = part((size_t)2 * D * (D + 2) * F * sizeof(double));
+    at_fluxes = part((size_t)D * (D + 2) * F * sizeof(double));
   }
-  // small block: dt, max_bits, counter, status, trace_pos, then the trace
-  const size_t small = 64 + sizeof(double) * kTraceCap;
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&b->s.dt, small, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->s.dt, 0, small, st);
+  const size_t at_small = part(small);
+  cudaError_t e = device_alloc(ctx, (void**)&b->mem, bytes);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->mem + at_small, 0, small, st);
   if (e != cudaSuccess) {
     destroy_box(b, st);
     return fail(ctx, e == cudaErrorMemoryAllocation ? RHYME_GPU_ENOMEM : RHYME_GPU_ECUDA,
                 "box allocation: %s", cudaGetErrorString(e));
   }
+  for (int i = 0; i < 2; ++i) b->state[i] = (double*)(b->mem + at_state[i]);
+  if (ctx->mixed) {
+    for (int i = 0; i < 2; ++i) b->Uf[i] = (float*)(b->mem + at_mirror[i]);
+    if (D > 1) b->acc = (float*)(b->mem + at_acc);
+    b->fbq.e = (FallbackEntry*)(b->mem + at_queue);
+  } else {
+    b->s.faces = (double*)(b->mem + at_faces);
+    b->s.fluxes = (double*)(b->mem + at_fluxes);
+  }
+  b->zero_bytes = ctx->mixed ? at_mirror[1] + (size_t)(D + 2) * F * sizeof(float) : at_state[1] + b->hydro_bytes;
+  b->s.dt = (double*)(b->mem + at_small);
   char* base = (char*)b->s.dt;
   b->s.max_bits = (unsigned long long*)(base + 8);
   b->s.counter = (unsigned int*)(base + 16);
@@ -1320,7 +1355,7 @@ extern "C" int rhyme_gpu_output_level(rhyme_gpu_ctx* ctx, const int* handles, in
   }
   // pageable source: the copy is staged before the call returns
   CK(cudaMemcpyAsync(ctx->out_desc, desc.data(), sizeof(PackDesc) * n, cudaMemcpyHostToDevice, ctx->stream));
-  CK(launch_pack_level(ctx->out_desc, n, blocks, D, ctx->out_dev, ctx->stream));
+  CK(launch_pack_level(ctx->out_desc, PackDesc(), n, blocks, D, ctx->out_dev, ctx->stream));
   CK(cudaEventRecord(ctx->out_packed, ctx->stream));
   CK(cudaStreamWaitEvent(ctx->copy, ctx->out_packed, 0));
   if (ncmp == D + 2) {
@@ -1495,13 +1530,19 @@ extern "C" int rhyme_gpu_paint(rhyme_gpu_ctx* ctx, int handle, const int left_ed
   int rc = make_paint_shapes(ctx, b, left_edge, shapes, n, &ps);
   if (rc != RHYME_GPU_OK) return rc;
   state_changed(b);
-  PaintShape* d = nullptr;
-  CK(cudaMallocAsync((void**)&d, sizeof(PaintShape) * n, ctx->stream));
-  cudaError_t e = cudaMemcpyAsync(d, ps.data(), sizeof(PaintShape) * n, cudaMemcpyHostToDevice, ctx->stream);
+  PaintShape* d = nullptr;  // a short list goes with the launch
+  PaintList few{};
+  cudaError_t e = cudaSuccess;
+  if (n <= kPaintFew) {
+    memcpy(few.s, ps.data(), sizeof(PaintShape) * n);
+  } else {
+    CK(device_alloc(ctx, (void**)&d, sizeof(PaintShape) * n));
+    e = cudaMemcpyAsync(d, ps.data(), sizeof(PaintShape) * n, cudaMemcpyHostToDevice, ctx->stream);
+  }
   if (e == cudaSuccess)
-    e = launch_paint(ctx->params.ndim, d, n, b->dp.G, b->g, left_edge, b->state[b->cur],
+    e = launch_paint(ctx->params.ndim, d, few, n, b->dp.G, b->g, left_edge, b->state[b->cur],
                      ctx->mixed ? b->Uf[b->cur] : nullptr, ctx->stream);
-  cudaFreeAsync(d, ctx->stream);
+  if (d) cudaFreeAsync(d, ctx->stream);
   if (e != cudaSuccess) return fail(ctx, RHYME_GPU_ECUDA, "paint: %s", cudaGetErrorString(e));
   return RHYME_GPU_OK;
 }
@@ -1561,6 +1602,7 @@ struct rhyme_gpu_batch {
   std::vector<int> handles;
   std::vector<int> base_cur;  // box parity when the tables were built
   int k = 0;                  // steps taken since (mod 2)
+  char* mem = nullptr;  // the device memory that the arrays below share
   BoxDesc* table[2] = {nullptr, nullptr};
   WorkItem* items = nullptr;
   int* heads = nullptr;
@@ -1574,21 +1616,12 @@ struct rhyme_gpu_batch {
 namespace {
 
 void batch_free(rhyme_gpu_batch* B) {
-  cudaStream_t st = B->ctx->stream;
-  for (int p = 0; p < 2; ++p) {
-    if (B->graph[p]) cudaGraphExecDestroy(B->graph[p]);
-    B->graph[p] = nullptr;
-    if (B->table[p]) cudaFreeAsync(B->table[p], st);
-    B->table[p] = nullptr;
+  for (cudaGraphExec_t& g : B->graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
   }
-  if (B->items) cudaFreeAsync(B->items, st);
-  if (B->heads) cudaFreeAsync(B->heads, st);
-  if (B->q.e) cudaFreeAsync(B->q.e, st);
-  if (B->qblock) cudaFreeAsync(B->qblock, st);
-  B->items = nullptr;
-  B->heads = nullptr;
-  B->q.e = nullptr;
-  B->qblock = nullptr;
+  if (B->mem) cudaFreeAsync(B->mem, B->ctx->stream);
+  B->mem = nullptr;
 }
 
 // Builds the box tables (both parities), the work-item lists and the
@@ -1688,30 +1721,34 @@ int batch_build(rhyme_gpu_batch* B) {
       for (long long c = 0; c * kBatchChunk < cells; ++c) update.push_back({i, 0, c});
     }
   }
-  std::vector<WorkItem> all;
+  // one block: both tables, the items, the queue heads, the counters (zeroed
+  // by the copy) and, after what is copied, the fix-up queue
   constexpr int kLists = 5 + 3 * kSweepShapes;
   size_t off[kLists];
   std::vector<WorkItem>* lists[kLists] = {&cfl, &ghost, &faces, &flux, &update};
   for (int a = 0; a < 3; ++a)
     for (int k = 0; k < kSweepShapes; ++k) lists[5 + kSweepShapes * a + k] = &sweep[a][k];
+  size_t count = 0;
   for (int k = 0; k < kLists; ++k) {
-    off[k] = all.size();
-    all.insert(all.end(), lists[k]->begin(), lists[k]->end());
+    off[k] = count;
+    count += lists[k]->size();
   }
-  for (int p = 0; p < 2; ++p) {
-    CK(cudaMallocAsync((void**)&B->table[p], sizeof(BoxDesc) * std::max(n, 1), ctx->stream));
-    CK(cudaMemcpyAsync(B->table[p], tab[p].data(), sizeof(BoxDesc) * n, cudaMemcpyHostToDevice, ctx->stream));
-  }
-  CK(cudaMallocAsync((void**)&B->items, sizeof(WorkItem) * std::max<size_t>(all.size(), 1), ctx->stream));
-  CK(cudaMemcpyAsync(B->items, all.data(), sizeof(WorkItem) * all.size(), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMallocAsync((void**)&B->heads, kBatchHeads * sizeof(int), ctx->stream));
-  CK(cudaMallocAsync((void**)&B->qblock, 16 * sizeof(int), ctx->stream));
-  CK(cudaMemsetAsync(B->qblock, 0, 16 * sizeof(int), ctx->stream));
-  B->q.cap = 0;
-  if (ctx->mixed) {
-    B->q.cap = (int)std::min<long long>(std::max<long long>(65536, qcap), 1LL << 30);
-    CK(cudaMallocAsync((void**)&B->q.e, sizeof(FallbackEntry) * (size_t)B->q.cap, ctx->stream));
-  }
+  B->q.cap = ctx->mixed ? (int)std::min<long long>(std::max<long long>(65536, qcap), 1LL << 30) : 0;
+  auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+  const size_t tab_bytes = up(sizeof(BoxDesc) * n), item_bytes = up(sizeof(WorkItem) * count);
+  const size_t head_bytes = up(kBatchHeads * sizeof(int)), block_bytes = up(16 * sizeof(int));
+  std::vector<char> blob(2 * tab_bytes + item_bytes + head_bytes + block_bytes, 0);
+  for (int p = 0; p < 2; ++p) memcpy(blob.data() + p * tab_bytes, tab[p].data(), sizeof(BoxDesc) * n);
+  for (int k = 0; k < kLists; ++k)
+    if (!lists[k]->empty())
+      memcpy(blob.data() + 2 * tab_bytes + sizeof(WorkItem) * off[k], lists[k]->data(), sizeof(WorkItem) * lists[k]->size());
+  CK(device_alloc(ctx, (void**)&B->mem, blob.size() + sizeof(FallbackEntry) * (size_t)B->q.cap));
+  CK(cudaMemcpyAsync(B->mem, blob.data(), blob.size(), cudaMemcpyHostToDevice, ctx->stream));
+  for (int p = 0; p < 2; ++p) B->table[p] = (BoxDesc*)(B->mem + p * tab_bytes);
+  B->items = (WorkItem*)(B->mem + 2 * tab_bytes);
+  B->heads = (int*)(B->mem + 2 * tab_bytes + item_bytes);
+  B->qblock = (int*)(B->mem + 2 * tab_bytes + item_bytes + head_bytes);
+  if (ctx->mixed) B->q.e = (FallbackEntry*)(B->mem + blob.size());
   B->q.n = B->qblock + 0;
   B->q.status = B->qblock + 1;
   B->q.total = B->qblock + 2;
@@ -2039,11 +2076,8 @@ int rhyme_gpu_server_tick(rhyme_gpu_server* S, int* n_active, int* n_pending, in
     if (rc != RHYME_GPU_OK) return server_fail(S, rc, ctx->err.c_str());
     if (painted) {  // initial state painted on the device from zero cells: no upload
       Box* nb = ctx->boxes[h];
-      for (int i = 0; i < 2; ++i) {
-        cudaError_t e = cudaMemsetAsync(nb->state[i], 0, nb->hydro_bytes, ctx->stream);
-        if (e == cudaSuccess && nb->Uf[i]) e = cudaMemsetAsync(nb->Uf[i], 0, nb->hydro_bytes / 2, ctx->stream);
-        if (e != cudaSuccess) return server_fail(S, RHYME_GPU_ECUDA, cudaGetErrorString(e));
-      }
+      cudaError_t e = cudaMemsetAsync(nb->mem, 0, nb->zero_bytes, ctx->stream);
+      if (e != cudaSuccess) return server_fail(S, RHYME_GPU_ECUDA, cudaGetErrorString(e));
       const int le[3] = {1, 1, 1};
       rc = rhyme_gpu_paint(ctx, h, le, q.shapes.data(), (int)q.shapes.size());
       if (rc != RHYME_GPU_OK) return server_fail(S, rc, ctx->err.c_str());
@@ -2121,12 +2155,9 @@ int rhyme_gpu_server_tick(rhyme_gpu_server* S, int* n_active, int* n_pending, in
         pd.cells = q.cells;
         pd.first_block = 0;
         pd.out_off = 0;
-        PackDesc* d_pd = nullptr;
         float* d_out = nullptr;
-        cudaError_t e = cudaMallocAsync((void**)&d_pd, sizeof(PackDesc), ctx->stream);
-        if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_out, ob, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(d_pd, &pd, sizeof(PackDesc), cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess) e = launch_pack_level(d_pd, 1, pack_blocks(D, q.cells), D, d_out, ctx->stream);
+        cudaError_t e = device_alloc(ctx, (void**)&d_out, ob);
+        if (e == cudaSuccess) e = launch_pack_level(nullptr, pd, 1, pack_blocks(D, q.cells), D, d_out, ctx->stream);
         cudaEvent_t packed;
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&packed, cudaEventDisableTiming);
         if (e == cudaSuccess) {
@@ -2135,7 +2166,6 @@ int rhyme_gpu_server_tick(rhyme_gpu_server* S, int* n_active, int* n_pending, in
           cudaEventDestroy(packed);
           e = cudaMemcpyAsync(q.out_staging, d_out, ob, cudaMemcpyDeviceToHost, S->copy);
         }
-        if (d_pd) cudaFreeAsync(d_pd, S->copy);
         if (d_out) cudaFreeAsync(d_out, S->copy);
         if (e != cudaSuccess) return server_fail(S, RHYME_GPU_ECUDA, cudaGetErrorString(e));
       }

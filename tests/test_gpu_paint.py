@@ -144,3 +144,13 @@ def test_paint_errors():
             ctx.paint(b, [slab])  # a slab needs NDIM > 1
         assert e.value.code == gpu.EINVAL
         ctx.paint(b, [])  # nothing to paint
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 40])
+def test_paint_short_and_long_lists(n):
+    """Up to eight shapes go with the launch, more through device memory."""
+    shapes = [drawing.canvas([1.0, 0, 0, 0, 1.0])]
+    shapes += [drawing.sharp_cuboid([1 + k % 12, 1 + k % 7], [3, 2], [1.0 + k, 0.1 * k, 0, 0, 1.0 + 0.5 * k])
+               for k in range(1, n)]
+    dev, ref = _paint_both(2, [16, 9], shapes)
+    assert np.array_equal(dev, ref)
