@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kBlock)
                          const double* __restrict__ ur, long long n, double* __restrict__ d) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
-    d[i] = limited_slope(P.limiter, P.omega, ul[i], u[i], ur[i]);
+    d[i] = limited_slope_f64(P.limiter, P.omega, ul[i], u[i], ur[i]);
 }
 
 template <int D>

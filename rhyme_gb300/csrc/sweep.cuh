@@ -403,11 +403,6 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
     }
     bool need64 = false;
     rp_flux_f32<D, 0>(M.G, M.rp, l, r, f, &need64);  // normal-first in and out
-    if (!need64) {
-#pragma unroll
-      for (int c = 0; c < D + 2; ++c)
-        if (!isfinite(f[c])) need64 = true;
-    }
     if (need64) {
       // A non-finite cell in the interface's stencil (staged cells li .. li+3)
       // is non-finite in FP64 too, and the FP64 redo would give NaN: give it
@@ -711,11 +706,6 @@ __device__ __forceinline__ void sweep_xy_tile(const MixedParams& M, int limiter,
     }
     bool need64 = false;
     rp_flux_f32<3, 0>(M.G, M.rp, l, r, f, &need64);
-    if (!need64) {
-#pragma unroll
-      for (int k = 0; k < 5; ++k)
-        if (!isfinite(f[k])) need64 = true;
-    }
     if (need64) {
       // as the per-axis sweeps: queued once (by the tile whose left face it
       // is, or by the last tile at the box's right boundary) unless a cell
