@@ -645,9 +645,10 @@ __device__ __forceinline__ void sweep_xy_tile(const MixedParams& M, int limiter,
 
   // 2. face states: x of cells x0-1 .. x0+TX (rows y0 ..), then y of cells
   // y0-1 .. y0+TY (columns x0 ..); one loop, the axis only in the indices
-  for (int it = threadIdx.x; it < Cfg::NXF + Cfg::NYF; it += NT) {
-    const int ax = it >= Cfg::NXF;
-    const int t = ax ? it - Cfg::NXF : it;
+#pragma unroll 1
+  for (int ax = 0; ax < 2; ++ax) {
+    const int t = threadIdx.x;
+    if (t >= (ax ? Cfg::NYF : Cfg::NXF)) continue;
     int base, stride, slot;
     if (!ax) {
       const int la = t % (TX + 2), lb = t / (TX + 2);
