@@ -89,7 +89,7 @@ cudaError_t launch_kind(int kind, int blocks, int iters, double* out, cudaStream
 }
 
 // Self-check of the integer conversions of the mixed state update
-// (rgpu_internal.h widen_f32, narrow_mirror) against the hardware ones, on
+// (rgpu_internal.h widen_f32, narrow_mirror and their common forms) against the hardware ones, on
 // n pseudo-random bit patterns per thread family (splitmix64): doubles of
 // every exponent, doubles near the FP32 rounding boundaries, ties, the
 // limits of the FP32 range, and FP32 values (subnormals excluded: the FP32
@@ -142,6 +142,9 @@ __global__ void conversion_check_kernel(long long n, unsigned long long seed, un
       const double x = __longlong_as_double((long long)bits);
       const float a = rgpu::narrow_mirror(x), b = rgpu::mirror_of(x);
       if (__float_as_uint(a) != __float_as_uint(b) && !(isnan(a) && isnan(b))) ++local;
+      bool rare = false;
+      const float c = rgpu::narrow_common(x, &rare);
+      if (!rare && __float_as_uint(c) != __float_as_uint(b)) ++local;
     } else {
       const unsigned f = (unsigned)r;
       const unsigned mag = f & 0x7fffffffu;
@@ -149,6 +152,9 @@ __global__ void conversion_check_kernel(long long n, unsigned long long seed, un
       const float y = __uint_as_float(f);
       const double a = rgpu::widen_f32(y), b = (double)y;
       if (__double_as_longlong(a) != __double_as_longlong(b) && !(isnan(a) && isnan(b))) ++local;
+      bool rare = false;
+      const double c = rgpu::widen_common(y, &rare);
+      if (!rare && __double_as_longlong(c) != __double_as_longlong(b)) ++local;
     }
   }
   if (local) atomicAdd(bad, local);

@@ -262,6 +262,30 @@ __device__ __forceinline__ float narrow_mirror(double x) {
   return __uint_as_float(sign | r);
 }
 
+// The same for what a cell nearly always holds: zeros, and normal numbers
+// that stay normal in FP32. Anything else sets *rare (and returns anything):
+// the caller then redoes the cell with the two functions above. The branches
+// of those cost the last sweep a quarter of its integer instructions.
+__device__ __forceinline__ double widen_common(float f, bool* rare) {
+  const unsigned b = __float_as_uint(f);
+  const unsigned mag = b & 0x7fffffffu;
+  const bool normal = mag >= 0x00800000u;
+  const unsigned moved = (unsigned)((int)b >> 3) & 0x8fffffffu;  // the sign stays, the rest moves
+  *rare = *rare || mag >= 0x7f800000u;
+  return __hiloint2double((int)(normal ? moved + 0x38000000u : b & 0x80000000u), (int)(normal ? b << 29 : 0u));
+}
+
+__device__ __forceinline__ float narrow_common(double x, bool* rare) {
+  const unsigned long long t = (unsigned long long)__double_as_longlong(x);
+  const unsigned hi = (unsigned)(t >> 32), mag = hi & 0x7fffffffu;
+  const unsigned long long up = t + (0x0fffffffu + ((unsigned)t >> 29 & 1u));  // ties to even
+  const bool zero = mag < 0x38000000u;  // below 2^-127: flushed
+  *rare = *rare || (!zero && mag - 0x38100000u >= 0x0fe00000u);
+  // exponent rebiased by -896 modulo 2^9 at bit 23
+  const unsigned r = zero ? 0u : ((unsigned)(up >> 29) + 0x40000000u) & 0x7fffffffu;
+  return __uint_as_float(r | (hi & 0x80000000u));
+}
+
 // Signal speed |v| + cs of a cell's FP32 state (the mixed CFL's); bad is set
 // for a non-positive density or a non-finite speed, which the maximum skips.
 template <int D>

@@ -118,24 +118,19 @@ struct TileCfg {
 // The flux difference dt/dx (F_left - F_right) of one component of one cell
 // and its accumulation by mode, with explicit roundings (a fused
 // multiply-add onto the running sum) so that every sweep variant performs
-// exactly the same operations. a_prev / u_prev: the component's accumulator
-// (MID, LAST) and U^n (LAST, ONLY), prefetched.
-// Returns U^{n+1} of the component in the modes that form it (0 otherwise).
+// exactly the same operations. a_prev: the component's accumulator (MID,
+// LAST), prefetched.
+// The modes that only accumulate; LAST and ONLY form U^{n+1} from total().
 template <int MODE>
-__device__ __forceinline__ double accumulate(float dtdx, float fl, float fr, float a_prev, double u_prev,
-                                             long long oc, float* __restrict__ acc, double* __restrict__ Unew) {
+__device__ __forceinline__ void accumulate(float dtdx, float fl, float fr, float a_prev, long long oc,
+                                           float* __restrict__ acc) {
   const float d = __fsub_rn(fl, fr);
-  if (MODE == FIRST) {
-    acc[oc] = __fmul_rn(dtdx, d);
-  } else if (MODE == MID) {
-    acc[oc] = __fmaf_rn(dtdx, d, a_prev);
-  } else {
-    const float tot = (MODE == LAST) ? __fmaf_rn(dtdx, d, a_prev) : __fmul_rn(dtdx, d);
-    const double un = __dadd_rn(u_prev, widen_f32(tot));
-    Unew[oc] = un;
-    return un;
-  }
-  return 0.0;
+  acc[oc] = (MODE == FIRST) ? __fmul_rn(dtdx, d) : __fmaf_rn(dtdx, d, a_prev);
+}
+template <int MODE>
+__device__ __forceinline__ float total(float dtdx, float fl, float fr, float a_prev) {
+  const float d = __fsub_rn(fl, fr);
+  return (MODE == LAST) ? __fmaf_rn(dtdx, d, a_prev) : __fmul_rn(dtdx, d);
 }
 
 // Block-wide maximum and or of (m, bad) of a CTA of NT threads (a multiple
@@ -450,22 +445,42 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
     if (ga > NA || gb > NB) continue;
     const long long o = offset(ga, gb);
     if (PRE_ACC || PRE_U) cp_async_wait_all();  // this thread's copies (same items as phase 0)
-    double ud[D + 2];
+    auto left = [&](int c) { return sh.f[nf_slot<D, A>(c)][ix(lu, lb, S + 1)]; };
+    auto right = [&](int c) { return sh.f[nf_slot<D, A>(c)][ix(lu + 1, lb, S + 1)]; };
+    auto before = [&](int c) { return PRE_ACC ? pre_acc[c * S * P + it] : 0.f; };
+    if constexpr (!FORMS) {
 #pragma unroll
-    for (int c = 0; c < D + 2; ++c)
-      ud[c] = accumulate<MODE>(dtdx, sh.f[nf_slot<D, A>(c)][ix(lu, lb, S + 1)],
-                               sh.f[nf_slot<D, A>(c)][ix(lu + 1, lb, S + 1)],
-                               PRE_ACC ? pre_acc[c * S * P + it] : 0.f, PRE_U ? pre_u[c * S * P + it] : 0.0,
-                               (long long)c * F + o, acc, Unew);
-    if (carrying) {
+      for (int c = 0; c < D + 2; ++c) accumulate<MODE>(dtdx, left(c), right(c), before(c), (long long)c * F + o, acc);
+    } else {
       float un[D + 2];
+      bool rare = false;
 #pragma unroll
       for (int c = 0; c < D + 2; ++c) {
-        un[c] = narrow_mirror(ud[c]);
-        carry.Uf_next[(long long)c * F + o] = un[c];
+        const float tot = total<MODE>(dtdx, left(c), right(c), before(c));
+        const double ud = __dadd_rn(pre_u[c * S * P + it], widen_common(tot, &rare));
+        Unew[(long long)c * F + o] = ud;
+        if (carrying) {
+          un[c] = narrow_common(ud, &rare);
+          carry.Uf_next[(long long)c * F + o] = un[c];
+        }
       }
-      const float v = speed_f32<D>(M, un, sbad);
-      if (v > smax) smax = v;
+      if (rare) {
+#pragma unroll 1
+        for (int c = 0; c < D + 2; ++c) {
+          const float tot = total<MODE>(dtdx, left(c), right(c), before(c));
+          const double ud = __dadd_rn(pre_u[c * S * P + it], widen_f32(tot));
+          Unew[(long long)c * F + o] = ud;
+          if (carrying) carry.Uf_next[(long long)c * F + o] = narrow_mirror(ud);
+        }
+        if (carrying) {
+#pragma unroll
+          for (int c = 0; c < D + 2; ++c) un[c] = carry.Uf_next[(long long)c * F + o];
+        }
+      }
+      if (carrying) {
+        const float v = speed_f32<D>(M, un, sbad);
+        if (v > smax) smax = v;
+      }
     }
   }
   if (carrying) block_fold_max<TileCfg<S, P>::threads>(smax, sbad, carry.bits, carry.status);
