@@ -373,6 +373,9 @@ cudaError_t launch_mh_solve_mixed(const MixedParams& M, const double* U, const f
                                   const SweepPlan& plan, cudaStream_t st, const HaloBC& halo,
                                   cudaEvent_t* ev = nullptr, const SweepCarry& carry = SweepCarry(),
                                   int* fused = nullptr, bool queue_reset = true);
+// Whether the x and y sweeps of a 3-D box can run as one kernel: the mirror's
+// rows allow the plane's tensor copy.
+bool sweep_xy_runs(const float* Uf, const Geom& g);
 // The x and y sweeps of a 3-D box as one kernel (sweeps.cu, sweep_xy_kernel):
 // cudaErrorNotSupported where its tensor copy cannot be used (rows of the
 // mirror not a multiple of 16 bytes, the encoder unavailable, too many tiles);

@@ -759,11 +759,16 @@ StepScratch scratch_of(Box* b, bool trace) {
 // A box-size class is (NDIM, axis, ceil(log2) of the box's extent along the
 // axis and along the pencil axis, each clamped to [3, 10]). The first box of
 // a class met by a context has its sweep along that axis timed with every
-// candidate tile shape (one warm-up and three timed launches each, CUDA
-// events on the context's stream) on its current state; the fastest shape is
-// kept for the class. A sweep only reads U^n and its FP32 mirror, so the
-// timing launches leave the state alone (they write the next-step buffers,
-// which the step itself overwrites).
+// candidate tile shape on its current state (one warm-up launch on a few
+// rows, then one launch of a box of a million cells or more, whose sweep
+// takes 50 us or longer, or three of a smaller box, between CUDA events on
+// the context's stream; one synchronisation per axis); the fastest shape is
+// kept for the class. Where the x and y sweeps run as one kernel, only z is
+// tuned. A sweep only reads U^n and its FP32 mirror, so the timing launches
+// leave the state alone (they write the next-step buffers, which the step
+// itself overwrites). With four full launches and a synchronisation each on
+// every axis the first run of a 3-D 256^3 box took 26 ms longer than the
+// next, of 64^3 2.1 ms; so it takes 7 and 1.0.
 
 int size_bucket(int n) {
   int b = 3;
@@ -777,55 +782,66 @@ int class_key(int D, int axis, const Geom& g) {
   return D | (axis << 2) | (size_bucket(g.n[axis]) << 4) | (size_bucket(nB) << 8);
 }
 
+// Before a box's first tune_axis: the mirror, its ghosts, dt and, where one
+// kernel runs the x and y sweeps, what it leaves for the z sweep.
+int tune_begin(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, bool fused) {
+  const int c = b->cur;
+  StepScratch sc = scratch_of(b, false);
+  CK(launch_cfl_mixed(b->mp, b->state[c], b->Uf[c], b->g, b->dp.courant, dx, sc, ctx->stream));
+  CK(launch_ghost_fill_f32(b->dp, b->Uf[c], b->g, ctx->stream));
+  b->mirror_valid = false;  // the FP32 ghosts were filled without the FP64 ones
+  if (!fused) return RHYME_GPU_OK;
+  CK(cudaMemsetAsync(b->fbq.n, 0, sizeof(int), ctx->stream));
+  CK(launch_sweep_xy_3(b->mp, b->Uf[c], b->g, dx, sc.dt, b->acc, b->fbq, no_halo(), ctx->stream));
+  return RHYME_GPU_OK;
+}
+
 int tune_axis(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, int axis, int* best) {
   const int D = ctx->params.ndim;
   const int c = b->cur;
   StepScratch sc = scratch_of(b, false);
   *best = default_sweep_shape(D, axis, b->g.n[axis]);
-  CK(launch_cfl_mixed(b->mp, b->state[c], b->Uf[c], b->g, b->dp.courant, dx, sc, ctx->stream));
-  CK(launch_ghost_fill_f32(b->dp, b->Uf[c], b->g, ctx->stream));
-  b->mirror_valid = false;  // the FP32 ghosts were filled without the FP64 ones
-  cudaEvent_t ev[2];
-  CK(cudaEventCreate(&ev[0]));
-  if (cudaEventCreate(&ev[1]) != cudaSuccess) {
-    cudaEventDestroy(ev[0]);
-    return fail(ctx, RHYME_GPU_ECUDA, "event create failed");
+  const int nO = b->g.n[D - 1];
+  const int rows = std::min(nO, D == 1 ? 512 : 64);  // whole tiles of every shape
+  const int reps = (long long)b->g.n[0] * b->g.n[1] * b->g.n[2] >= 1000000 ? 1 : 3;
+  cudaEvent_t ev[kSweepShapes][2] = {};
+  bool ok[kSweepShapes];
+  cudaError_t e = cudaSuccess;
+  auto sweep = [&](int k, int hi) {
+    cudaError_t r = cudaMemsetAsync(b->fbq.n, 0, sizeof(int), ctx->stream);
+    if (r == cudaSuccess)
+      r = launch_sweep_slab(D, axis, k, b->mp, b->Uf[c], b->state[c], b->g, dx, sc.dt, b->acc, b->state[1 - c], b->fbq,
+                            1, hi, ctx->stream);
+    if (r == cudaErrorInvalidConfiguration) {  // grid too large for this shape
+      ok[k] = false;
+      r = cudaSuccess;
+    }
+    return r;
+  };
+  for (int k = 0; k < kSweepShapes && e == cudaSuccess; ++k) {
+    ok[k] = true;
+    for (cudaEvent_t& v : ev[k])
+      if (e == cudaSuccess) e = cudaEventCreate(&v);
+    if (e == cudaSuccess) e = sweep(k, rows);
+    if (e == cudaSuccess) e = cudaEventRecord(ev[k][0], ctx->stream);
+    for (int rep = 0; rep < reps && ok[k] && e == cudaSuccess; ++rep) e = sweep(k, nO);
+    if (e == cudaSuccess) e = cudaEventRecord(ev[k][1], ctx->stream);
   }
-  int rc = RHYME_GPU_OK;
+  int rc = e == cudaSuccess ? wait_stream(ctx)
+                            : fail(ctx, RHYME_GPU_ECUDA, "autotune launch: %s", cudaGetErrorString(e));
   float best_ms = 0.f;
   bool have = false;
-  for (int k = 0; k < kSweepShapes && rc == RHYME_GPU_OK; ++k) {
-    float total = 0.f;
-    bool ok = true;
-    for (int rep = 0; rep < 4 && ok; ++rep) {
-      cudaError_t e = cudaMemsetAsync(b->fbq.n, 0, sizeof(int), ctx->stream);
-      if (e == cudaSuccess) e = cudaEventRecord(ev[0], ctx->stream);
-      if (e == cudaSuccess)
-        e = launch_sweep_axis(D, axis, k, b->mp, b->Uf[c], b->state[c], b->g, dx, sc.dt, b->acc,
-                              b->state[1 - c], b->fbq, ctx->stream);
-      if (e == cudaErrorInvalidConfiguration) {  // grid too large for this shape
-        ok = false;
-        break;
-      }
-      if (e == cudaSuccess) e = cudaEventRecord(ev[1], ctx->stream);
-      if (e != cudaSuccess) {
-        rc = fail(ctx, RHYME_GPU_ECUDA, "autotune launch: %s", cudaGetErrorString(e));
-        break;
-      }
-      rc = wait_stream(ctx);
-      if (rc != RHYME_GPU_OK) break;
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, ev[0], ev[1]);
-      if (rep > 0) total += ms;
-    }
-    if (rc == RHYME_GPU_OK && ok && (!have || total < best_ms)) {
+  for (int k = 0; k < kSweepShapes; ++k) {
+    float ms = 0.f;
+    if (rc == RHYME_GPU_OK && ok[k] && cudaEventElapsedTime(&ms, ev[k][0], ev[k][1]) == cudaSuccess &&
+        (!have || ms < best_ms)) {
       have = true;
-      best_ms = total;
+      best_ms = ms;
       *best = k;
     }
+    for (cudaEvent_t v : ev[k])
+      if (v) cudaEventDestroy(v);
   }
-  cudaEventDestroy(ev[0]);
-  cudaEventDestroy(ev[1]);
   if (rc == RHYME_GPU_OK) CK(cudaMemsetAsync(b->fbq.n, 0, sizeof(int), ctx->stream));
   return rc;
 }
@@ -837,20 +853,25 @@ int box_plan(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx) {
   if (!ctx->mixed || b->plan_valid) return RHYME_GPU_OK;
   const int D = ctx->params.ndim;
   for (int a = 0; a < 3; ++a) b->plan.shape[a] = default_sweep_shape(D, a < D ? a : 0, b->g.n[a < D ? a : 0]);
+  b->plan.fuse_xy = (D == 3 && ctx->fuse_xy) ? 1 : 0;
   if (ctx->params.sweep_tuning == RHYME_GPU_TUNE_AUTO) {
-    for (int a = 0; a < D; ++a) {
+    const bool fused = b->plan.fuse_xy && sweep_xy_runs(b->Uf[0], b->g) && sweep_xy_runs(b->Uf[1], b->g);
+    bool begun = false;
+    for (int a = fused ? 2 : 0; a < D; ++a) {
       const int key = class_key(D, a, b->g);
       auto it = ctx->tuned.find(key);
       if (it == ctx->tuned.end()) {
+        int rc = RHYME_GPU_OK;
+        if (!begun) rc = tune_begin(ctx, b, dx, fused);
+        begun = true;
         int best = 0;
-        int rc = tune_axis(ctx, b, dx, a, &best);
+        if (rc == RHYME_GPU_OK) rc = tune_axis(ctx, b, dx, a, &best);
         if (rc != RHYME_GPU_OK) return rc;
         it = ctx->tuned.emplace(key, best).first;
       }
       b->plan.shape[a] = it->second;
     }
   }
-  b->plan.fuse_xy = (D == 3 && ctx->fuse_xy) ? 1 : 0;
   b->plan_valid = true;
   return RHYME_GPU_OK;
 }

@@ -160,15 +160,25 @@ cudaError_t RGPU_CAT(launch_batch_sweep_axis_, SWEEP_D)(int axis, int shape, con
 }
 
 #if SWEEP_D == 3
+namespace {
+constexpr int TX = 16, TY = 16;
+bool xy_map(CUtensorMap* map, const float* Uf, const Geom& g) {
+  memset(map, 0, sizeof *map);
+  return (g.n[1] + TY - 1) / TY <= 65535 && g.n[2] <= 65535 && encode_xy_map(map, Uf, g, TX, TY);
+}
+}  // namespace
+
+bool sweep_xy_runs(const float* Uf, const Geom& g) {
+  CUtensorMap map;
+  return xy_map(&map, Uf, g);
+}
+
 cudaError_t launch_sweep_xy_3(const MixedParams& M, const float* Uf, const Geom& g, const Dx& dx,
                               const double* dtp, float* acc, const FallbackQueue& q, const HaloBC& halo,
                               cudaStream_t st) {
-  constexpr int TX = 16, TY = 16;
   const unsigned gx = (unsigned)((g.n[0] + TX - 1) / TX), gy = (unsigned)((g.n[1] + TY - 1) / TY);
-  if (gy > 65535 || g.n[2] > 65535) return cudaErrorNotSupported;
   CUtensorMap map;
-  memset(&map, 0, sizeof map);
-  if (!encode_xy_map(&map, Uf, g, TX, TY)) return cudaErrorNotSupported;
+  if (!xy_map(&map, Uf, g)) return cudaErrorNotSupported;
   return launch_step(sweep_xy_kernel<TX, TY>, dim3(gx, gy, (unsigned)g.n[2]), dim3(XYCfg<TX, TY>::threads), st, M, Uf, g,
                      dx, dtp, acc, q, map, halo);
 }
