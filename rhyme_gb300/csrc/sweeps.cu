@@ -29,6 +29,15 @@ constexpr int mode_of() {
 // (O = A, or O = B across the pencils) the slab must start on a tile
 // boundary and end on one or at the box's edge, so that every cell belongs
 // to exactly one slab.
+// From this many threads on (columns x segments of S cells) the last sweep
+// marches along its columns (march_kernel); below, too few threads wait for
+// their chains of dependent instructions and tiles are faster. Tiles against
+// march at the best S of each: 3-D 64^3 19 / 29 us, 96^3 44.2 / 43.7 (110
+// thousand threads), 250x130x61 88 / 82 (260), 128^3 91.9 / 90.7 (262), 192^3
+// 270 / 247, 256^3 613 / 543; 2-D 1024^2 40 / 45 (131), 2047x2048 145 / 125
+// (524), 4096^2 518 / 421.
+constexpr long long kMarchThreads = 152 * 1024;
+
 template <int D, int A, int S, int P>
 cudaError_t launch_one(const MixedParams& M, const float* Uf, const double* U, const Geom& g, const Dx& dx,
                        const double* dtp, float* acc, double* Unew, const FallbackQueue& q, int lo, int hi,
@@ -40,6 +49,13 @@ cudaError_t launch_one(const MixedParams& M, const float* Uf, const double* U, c
   if (O == A || O == B) {
     constexpr int T = (O == A) ? S : P;
     if ((lo - 1) % T != 0 || (hi != NO && (hi - lo + 1) % T != 0)) return cudaErrorInvalidValue;
+  }
+  if constexpr (D > 1 && A == D - 1) {
+    const long long columns = (D == 3) ? (long long)g.n[0] * g.n[1] : g.n[0];
+    const int segments = (NO + S - 1) / S;
+    if (lo == 1 && hi == NO && columns * segments >= kMarchThreads && columns < (1LL << 31) && segments <= 65535)
+      return launch_step(march_kernel<D>, dim3((unsigned)((columns + kMarchBlock - 1) / kMarchBlock), (unsigned)segments),
+                         dim3(kMarchBlock), st, M, Uf, U, g, dx, dtp, acc, Unew, q, S, carry, halo);
   }
   Geom gs = g;
   FallbackQueue qs = q;
