@@ -247,9 +247,9 @@ def allsum(x, world):
 def launches_per_step(prec, ndim, fused_xy=False):
     """Kernels of this library launched per single-box step: FP64 cfl, ghost
     fill, faces, fluxes, update; mixed cfl (carried, or the whole pass that
-    also writes the FP32 mirror), ghost fill (of the FP64 state and of the
-    mirror, in one kernel), one sweep per axis (one kernel for x and y of a
-    3-D box where fused_xy) and the FP64 fix-up of the queued interfaces."""
+    also writes the FP32 mirror), one sweep per axis (one kernel for x and y
+    of a 3-D box where fused_xy), the FP64 fix-up of the queued interfaces and
+    the ghost fill that ends a run (every timed step is a run of its own)."""
     if prec == "fp64":
         return 5
     return 3 + ndim - (1 if fused_xy else 0)

@@ -1,17 +1,21 @@
 // kernels_mixed.cu -- mixed-precision MUSCL-Hancock step.
 //
-// The conserved state stays FP64 in HBM (U) and is mirrored once per step as
-// FP32 (Uf) by the step's first pass, the FP32 CFL, which reads U anyway.
-// Each axis is one fused sweep kernel: a CTA stages a slab of Uf (S cells
-// along the sweep axis plus the 2-cell ghost/halo layer, for P pencils) in
-// shared memory with coalesced loads, computes FP32 limited slopes and
-// half-step face states for S+2 cells, solves the S+1 exact Riemann problems
-// of the slab in FP32 and forms the flux difference of its S cells. The flux
+// The conserved state stays FP64 in HBM (U) with an FP32 mirror (Uf), which
+// the last sweep of each step writes along with U^{n+1} and its FP32 signal
+// speeds, so that the next step's CFL pass only forms dt; after an upload or
+// a change from outside the CFL pass writes the mirror itself.
+// Each axis is one fused sweep kernel (the x and y axes of a 3-D box one
+// kernel together): a CTA stages a slab of Uf (S cells along the sweep axis
+// plus the 2-cell ghost/halo layer, for P pencils) in shared memory, computes
+// FP32 limited slopes and half-step face states for S+2 cells, solves the S+1
+// exact Riemann problems of the slab in FP32 and forms the flux difference of
+// its S cells; the last sweep of a large box marches along its columns
+// instead (sweep.cuh). Ghost cells come from the interior while a tile is
+// staged, so a resident run fills them in memory only at its end. The flux
 // differences of the axes are summed in FP32 in the reference's association
 // ((X + Y) + Z), and the last sweep adds the sum to U in FP64 and writes
 // U^{n+1}: one FP64 add per conserved component and cell, since on GB300 even
-// FP64 adds are scarce (the next step's CFL makes the new mirror, where the
-// conversions cost nothing but bandwidth).
+// FP64 adds are scarce (the conversions around it are integer operations).
 //
 // Interfaces that near vacuum, or whose FP32 iteration does not reach the
 // tolerance on its first guess, or whose FP32 face states or flux are not
@@ -21,7 +25,7 @@
 // (limited slopes and half-step face states of its two cells, exact Riemann
 // problem, flux: the device code of the plain path instantiated for double),
 // and applies -+ dt/dx * F to the two adjacent interior cells of U^{n+1}.
-// Keeping the FP64 code out of the sweeps keeps them at 50-52 registers (it
+// Keeping the FP64 code out of the sweeps keeps them at 40-51 registers (it
 // tripled their register count inline).
 //
 // The CFL maximum of the mixed path is taken in FP32 over the mirror; dt

@@ -877,9 +877,8 @@ int box_plan(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx) {
 }
 
 // One captured step: CFL pass (dt; in mixed precision also the FP32
-// mirror's interior), ghost fill (the FP64 state, the other buffer and the
-// mirror's ghosts), solve. Running the ghost fill on a second stream beside
-// the CFL pass made the captured step 2.8 % slower at 256^3.
+// mirror's interior where the last sweep has not carried it), ghost fill
+// (where the sweeps do not take the ghost cells from the interior), solve.
 // The mixed step's carry: the last sweep writes U^{n+1}'s FP32 mirror into
 // the other buffer's mirror and folds its signal speeds.
 SweepCarry carry_of(Box* b, int cur) {

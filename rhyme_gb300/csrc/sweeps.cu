@@ -177,6 +177,8 @@ cudaError_t RGPU_CAT(launch_batch_sweep_axis_, SWEEP_D)(int axis, int shape, con
 
 #if SWEEP_D == 3
 namespace {
+// The tile of a single box, at 256^3 (64^3): 16x16 741 us (20.5), 8x16 795
+// (22.1), 16x8 812 (22.3), 32x8 832 (21.9), 8x8 912 (24.8).
 constexpr int TX = 16, TY = 16;
 bool xy_map(CUtensorMap* map, const float* Uf, const Geom& g) {
   memset(map, 0, sizeof *map);
