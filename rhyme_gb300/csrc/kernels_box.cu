@@ -17,7 +17,7 @@
 // the limiters' spared divisions and the two sides' waves run in common
 // passes, and the solve calls those functions instead of inlining them (its
 // warps waited for instructions half of the time): a step of the 2-D 256^2
-// slab 348 -> 118 us, of 3-D 128^3 17.5 -> 6.0 ms, of 16 boxes of 8..64^3 5.5
+// slab 348 -> 114 us, of 3-D 128^3 17.5 -> 5.5 ms, of 16 boxes of 8..64^3 5.5
 // -> 2.0 ms. A third of the FP64 warp instructions of the flux pass that are
 // left run with part of their lanes.
 //
@@ -126,8 +126,9 @@ __global__ void __launch_bounds__(kCflBlock)
 
 // ------------------------------------------------------------------ K3 ---
 // Pass 1: face states of every cell with i_AX in [0, N+1] (box_elems.cuh).
+// At least 8 CTAs per SM, as for the fluxes below: 128^3 1.44 ms unbounded, 1.40 at 8, 1.45 at 12.
 template <int D>
-__global__ void __launch_bounds__(kFaceBlock)
+__global__ void __launch_bounds__(kFaceBlock, 8)
     faces_kernel(DevParams P, BoxRules R, const double* __restrict__ U, Geom g, Dx dx,
                  const double* dtp, double* __restrict__ FS) {
   step_begin();
@@ -172,14 +173,14 @@ __device__ __forceinline__ void flux_pass(const DevParams& P, const double* __re
   }
 }
 
-// At least 8 CTAs per SM in 2-D and 3-D (64 registers, some spilled): the
-// solve's chains of dependent FP64 and integer instructions need the warps
-// more than the registers (128^3: 4.96 ms at 3 CTAs, 4.32 at 5, 3.97 at 8,
-// 3.86 at 12; 2-D 256^2: 97 us at 3, 75 at 8). A 1-D box rarely fills the SMs
-// once; there the unbounded kernel is the faster one (512 cells: 31 against
-// 33 us).
+// At least 8 CTAs per SM in 2-D, 16 in 3-D (64 and 32 registers, some
+// spilled): the solve's chains of dependent FP64 and integer instructions need
+// the warps more than the registers (128^3: 4.96 ms at 3 CTAs, 4.32 at 5, 3.97
+// at 8, 3.82 at 12, 3.54 at 16; 2-D 256^2: 97 us at 3, 73 at 8, 76 at 16). A
+// 1-D box rarely fills the SMs once; there the unbounded kernel is the faster
+// one (512 cells: 31 against 33 us).
 template <int D>
-__global__ void __launch_bounds__(kFluxBlock, D == 1 ? 1 : 8)
+__global__ void __launch_bounds__(kFluxBlock, D == 1 ? 1 : D == 2 ? 8 : 16)
     flux_kernel(DevParams P, const double* __restrict__ FS, Geom g, double* __restrict__ FR) {
   step_begin();
   flux_pass<D>(P, FS, g, FR);
