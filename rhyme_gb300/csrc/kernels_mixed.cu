@@ -395,13 +395,24 @@ struct FixBC {
   double inflow[6][5];
 };
 
+// The fix-up kernels: one CTA per SM, few enough for an early launch (the
+// queue is nearly always empty), of 8 warps, since a redo is a chain of
+// dependent FP64 and integer instructions: a step of 512 boxes, some of them
+// unphysical and queued whole, takes 11.1 ms with 4 warps, 9.5 with 8 or 16
+// (6.6 of them the fix-up, bound by its longest Newton iterations). A short
+// queue is spread over the SMs, a warp of entries each.
+constexpr int kFixGrid = 152, kFixBlock = 256;
+__device__ __forceinline__ int fix_first() {
+  return ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+}
+
 // FP64 redo of the queued interfaces; -+ dt/dx * F applied to the adjacent
 // interior cells of U^{n+1} (atomically: a cell can border two queued
 // interfaces).
 // Entries from *from (0 when from is null) to the queue's end: a solve in
 // slabs fixes the entries of each slab after its sweeps.
 template <int D>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kFixBlock)
     fallback_fix_kernel(MixedParams M, FallbackQueue q, Geom g, Dx dx, const double* __restrict__ dtp,
                         const double* __restrict__ U, double* __restrict__ Unew, const int* __restrict__ from,
                         const __grid_constant__ FixBC fbc) {
@@ -411,7 +422,7 @@ __global__ void __launch_bounds__(128)
   if (blockIdx.x == 0 && threadIdx.x == 0 && n > lo) atomicAdd(q.total, n - lo);
   const double dt = *dtp;
   const long long F = g.field;
-  for (int i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = lo + fix_first(); i < n; i += gridDim.x * kFixBlock) {
     const FallbackEntry e = q.e[i];
     double f[D + 2];
     redo_any_axis<D>(M, M.limiter, M.omega64, U, g, e, fbc.bc, fbc.inflow, 0.5 * dt / dx.v[e.axis], f);
@@ -436,7 +447,7 @@ cudaError_t launch_fallback(const MixedParams& M, const FallbackQueue& q, const 
     fbc.bc[i] = halo.type[i];
     for (int c = 0; c < 5; ++c) fbc.inflow[i][c] = halo.inflow64[i][c];
   }
-  launch_step(fallback_fix_kernel<D>, 152, 128, st, M, q, g, dx, dtp, U, Unew, from, fbc);
+  launch_step(fallback_fix_kernel<D>, kFixGrid, kFixBlock, st, M, q, g, dx, dtp, U, Unew, from, fbc);
   return cudaGetLastError();
 }
 
@@ -519,11 +530,11 @@ __global__ void __launch_bounds__(256)
 
 // Batched FP64 fix-up: as fallback_fix_kernel, with the box of each entry.
 template <int D>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kFixBlock)
     batch_fallback_fix_kernel(MixedParams M, FallbackQueue q, const BoxDesc* __restrict__ TB) {
   const int n = min(*q.n, q.cap);
   if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(q.total, n);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = fix_first(); i < n; i += gridDim.x * kFixBlock) {
     const FallbackEntry e = q.e[i];
     const BoxDesc& b = TB[e.box];
     *carry_ok_of(b) = 0;  // the box's cells change after its last sweep: its next CFL pass is whole
@@ -545,7 +556,7 @@ __global__ void __launch_bounds__(128)
 template <int D>
 cudaError_t launch_batch_fallback(const MixedParams& M, const BoxDesc* TB, const FallbackQueue& q,
                                   cudaStream_t st) {
-  batch_fallback_fix_kernel<D><<<152, 128, 0, st>>>(M, q, TB);
+  batch_fallback_fix_kernel<D><<<kFixGrid, kFixBlock, 0, st>>>(M, q, TB);
   return cudaGetLastError();
 }
 
