@@ -20,6 +20,7 @@
 #include <string>
 #include <thread>
 #include <map>
+#include <memory>
 #include <vector>
 
 #include "../../include/rhyme_gpu.h"
@@ -1760,18 +1761,20 @@ int batch_build(rhyme_gpu_batch* B) {
   auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
   const size_t tab_bytes = up(sizeof(BoxDesc) * n), item_bytes = up(sizeof(WorkItem) * count);
   const size_t head_bytes = up(kBatchHeads * sizeof(int)), block_bytes = up(16 * sizeof(int));
-  std::vector<char> blob(2 * tab_bytes + item_bytes + head_bytes + block_bytes, 0);
-  for (int p = 0; p < 2; ++p) memcpy(blob.data() + p * tab_bytes, tab[p].data(), sizeof(BoxDesc) * n);
+  const size_t blob_bytes = 2 * tab_bytes + item_bytes + head_bytes + block_bytes;
+  std::unique_ptr<char[]> blob(new char[blob_bytes]);
+  memset(blob.get() + blob_bytes - head_bytes - block_bytes, 0, head_bytes + block_bytes);
+  for (int p = 0; p < 2; ++p) memcpy(blob.get() + p * tab_bytes, tab[p].data(), sizeof(BoxDesc) * n);
   for (int k = 0; k < kLists; ++k)
     if (!lists[k]->empty())
-      memcpy(blob.data() + 2 * tab_bytes + sizeof(WorkItem) * off[k], lists[k]->data(), sizeof(WorkItem) * lists[k]->size());
-  CK(device_alloc(ctx, (void**)&B->mem, blob.size() + sizeof(FallbackEntry) * (size_t)B->q.cap));
-  CK(cudaMemcpyAsync(B->mem, blob.data(), blob.size(), cudaMemcpyHostToDevice, ctx->stream));
+      memcpy(blob.get() + 2 * tab_bytes + sizeof(WorkItem) * off[k], lists[k]->data(), sizeof(WorkItem) * lists[k]->size());
+  CK(device_alloc(ctx, (void**)&B->mem, blob_bytes + sizeof(FallbackEntry) * (size_t)B->q.cap));
+  CK(cudaMemcpyAsync(B->mem, blob.get(), blob_bytes, cudaMemcpyHostToDevice, ctx->stream));
   for (int p = 0; p < 2; ++p) B->table[p] = (BoxDesc*)(B->mem + p * tab_bytes);
   B->items = (WorkItem*)(B->mem + 2 * tab_bytes);
   B->heads = (int*)(B->mem + 2 * tab_bytes + item_bytes);
   B->qblock = (int*)(B->mem + 2 * tab_bytes + item_bytes + head_bytes);
-  if (ctx->mixed) B->q.e = (FallbackEntry*)(B->mem + blob.size());
+  if (ctx->mixed) B->q.e = (FallbackEntry*)(B->mem + blob_bytes);
   B->q.n = B->qblock + 0;
   B->q.status = B->qblock + 1;
   B->q.total = B->qblock + 2;
