@@ -222,6 +222,8 @@ RGPU_HD bool f64_gt(double a, double b) {
   }
   return hw_gt(a, b);
 }
+RGPU_HD bool f64_nan(double x) { return (f64_bits(x) << 1) > 0xffe0000000000000ull; }
+
 // x > c for a positive constant c or zero: x in (c, infinity].
 RGPU_HD bool f64_above(double x, double c) {
   const uint64_t uc = f64_bits(c);

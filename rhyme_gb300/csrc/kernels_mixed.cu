@@ -397,10 +397,9 @@ struct FixBC {
 
 // The fix-up kernels: one CTA per SM, few enough for an early launch (the
 // queue is nearly always empty), of 8 warps, since a redo is a chain of
-// dependent FP64 and integer instructions: a step of 512 boxes, some of them
-// unphysical and queued whole, takes 11.1 ms with 4 warps, 9.5 with 8 or 16
-// (6.6 of them the fix-up, bound by its longest Newton iterations). A short
-// queue is spread over the SMs, a warp of entries each.
+// dependent FP64 and integer instructions: where 512 boxes queued interfaces
+// that iterated long, a step took 11.1 ms with 4 warps, 9.5 with 8 or 16. A
+// short queue is spread over the SMs, a warp of entries each.
 constexpr int kFixGrid = 152, kFixBlock = 256;
 __device__ __forceinline__ int fix_first() {
   return ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
