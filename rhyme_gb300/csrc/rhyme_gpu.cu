@@ -297,9 +297,17 @@ void make_mixed_params(const DevParams& d, MixedParams* m) {
   m->rp.tol = (float)d.rp.tol;
   m->rp.n_iter = d.rp.n_iter;
   // third order: a last step of cbrt(tol) leaves less than tol, one of 5e-3
-  // less than 1.3e-8; with few iterations allowed the FP64 form may stop
-  // short of the root, and only steps below tol agree with it
-  m->rp.last = d.rp.n_iter < 8 ? (float)d.rp.tol : (float)std::min(5e-3, std::cbrt(d.rp.tol));
+  // less than 1.6e-8. Only steps below tol count where few iterations are
+  // allowed (the FP64 form may stop short of the root) and where tol is below
+  // FP32's resolution of p: there the interfaces whose p does not settle go
+  // to FP64. The line at 2^-22 is where the Newton steps to tol that this
+  // iteration replaced sent so many that the mean flux error over all
+  // interfaces was as low (10^6 between states of ratios up to e^12, host
+  // build, redone / error in 1e-9: tol 2.5e-7 Newton 6.5 % / 8.4, cbrt 1.5 %
+  // / 8.4; 1.5e-7 8.2 % / 7.9, cbrt 1.5 % / 8.4, steps to tol 4.6 % / 7.8;
+  // 1e-10 28.8 % / 5.2, cbrt 1.5 % / 8.4, steps to tol 26.0 % / 5.3).
+  const bool to_tol = d.rp.n_iter < 8 || d.rp.tol < 0x1p-22;
+  m->rp.last = (float)(to_tol ? d.rp.tol : std::min(5e-3, std::cbrt(d.rp.tol)));
   m->G64 = d.G;
   m->rp64 = d.rp;
   m->ndim = d.ndim;
