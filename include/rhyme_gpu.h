@@ -180,7 +180,8 @@ int rhyme_gpu_set_rows(rhyme_gpu_ctx* ctx, int handle, int row0, int nrows, cons
  * Reads and clears the box's status word (no reference counterpart: the
  * reference only logs, rhyme_sanity_check_perform.f90:34-63). Bit 0 is set
  * when a CFL pass met a cell with non-positive density or a non-finite
- * signal speed; such cells are skipped by the dt maximum exactly as the
+ * signal speed (in mixed precision the state that the last run ended in is
+ * looked at too); such cells are skipped by the dt maximum exactly as the
  * reference's `if (u > max_u)` skips them, and the run goes on. Returns
  * RHYME_GPU_ENANSTATE when a bit is set, RHYME_GPU_OK otherwise.
  */

@@ -263,7 +263,9 @@ __global__ void __launch_bounds__(kThreads)
   const bool use = *carry_ok != 0 && *prev_fix == 0;
   if (use) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-      const float mu = __uint_as_float((unsigned int)*carry_bits);
+      const unsigned long long carried = *carry_bits;
+      const float mu = __uint_as_float((unsigned int)carried);
+      if (carried >> 32) atomicOr(s.status, 1);
       const double dt = courant * mdx / (double)mu;
       *s.dt = dt;
       if (s.dt_trace) {
@@ -328,6 +330,28 @@ __global__ void __launch_bounds__(kThreads)
       }
     }
   }
+}
+
+// launch_carry_status: see rgpu_internal.h. The speeds' mirror is written as
+// the next whole CFL pass would.
+template <int D>
+__global__ void __launch_bounds__(kThreads)
+    carry_status_kernel(MixedParams M, const double* __restrict__ U, float* __restrict__ Uf, Geom g,
+                        unsigned long long* carry_bits, const int* __restrict__ carry_ok,
+                        const int* __restrict__ prev_fix, int* status) {
+  if (*carry_ok != 0 && (!prev_fix || *prev_fix == 0)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (*carry_bits >> 32) atomicOr(status, 1);
+      *carry_bits &= 0xffffffffull;
+    }
+    return;
+  }
+  const long long total = (long long)g.n[0] * g.n[1] * (long long)g.n[2];
+  int bad = 0;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x)
+    signal_speed_f32<D>(M, U, Uf, g, t, bad);
+  if (bad) atomicOr(status, 1);
 }
 
 // FP64 flux of the interface between cell o (index ga along AX) and cell
@@ -476,7 +500,9 @@ __global__ void __launch_bounds__(256)
     const bool carried = !all && *(volatile int*)carry_ok_of(b) != 0;
     if (carried) {
       if (w.chunk == 0 && threadIdx.x == 0) {
-        const float mu = __uint_as_float((unsigned int)*carry_bits_of(b));
+        const unsigned long long folded = *carry_bits_of(b);
+        const float mu = __uint_as_float((unsigned int)folded);
+        if (folded >> 32) atomicOr((int*)(b.ctl + 2) + 1, 1);
         b.ctl[0] = courant * b.dx.min / (double)mu;
         *carry_bits_of(b) = 0ull;
       }
@@ -596,6 +622,20 @@ cudaError_t launch_cfl_carry(const MixedParams& M, const double* U, float* Uf, c
     case 3:
       launch_step(cfl_carry_kernel<3>, grid, kThreads, st, M, U, Uf, g, courant, dx.min, s, carry_bits, carry_ok, prev_fix, this_fix);
       break;
+    default: return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_carry_status(const MixedParams& M, const double* U, float* Uf, const Geom& g,
+                                unsigned long long* carry_bits, const int* carry_ok, const int* prev_fix, int* status,
+                                cudaStream_t st) {
+  int grid = grid_for((long long)g.n[0] * g.n[1] * g.n[2], kThreads);
+  if (grid > 152 * 4) grid = 152 * 4;
+  switch (M.ndim) {
+    case 1: carry_status_kernel<1><<<grid, kThreads, 0, st>>>(M, U, Uf, g, carry_bits, carry_ok, prev_fix, status); break;
+    case 2: carry_status_kernel<2><<<grid, kThreads, 0, st>>>(M, U, Uf, g, carry_bits, carry_ok, prev_fix, status); break;
+    case 3: carry_status_kernel<3><<<grid, kThreads, 0, st>>>(M, U, Uf, g, carry_bits, carry_ok, prev_fix, status); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

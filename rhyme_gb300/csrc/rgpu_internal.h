@@ -300,12 +300,15 @@ __device__ __forceinline__ float speed_f32(const MixedParams& M, const float* u,
 
 // The CFL pass carried by the last sweep of the mixed step: besides U^{n+1}
 // it writes the interior of U^{n+1}'s FP32 mirror (Uf_next) and folds the
-// FP32 signal speeds of U^{n+1} into *bits, so the next step's CFL pass
-// only forms dt (launch_cfl_carry). Null members: no carry.
+// FP32 signal speeds of U^{n+1} into *bits (low half: the maximum's bits; high
+// half: 1 if a cell is bad), so the next step's CFL pass only forms dt and
+// passes the flag on to the status word (launch_cfl_carry). The flag waits
+// for that pass because the FP64 fix-up may still change the cells: a cell
+// that lacks the flux of a queued interface can look unphysical and not be
+// it. Null members: no carry.
 struct SweepCarry {
   float* Uf_next = nullptr;
   unsigned long long* bits = nullptr;
-  int* status = nullptr;
 };
 
 // The boundary rules as the mixed sweeps apply them: a face of type 1..4
@@ -363,6 +366,13 @@ cudaError_t launch_to_f32(const double* U, float* Uf, long long n, cudaStream_t 
 cudaError_t launch_cfl_carry(const MixedParams& M, const double* U, float* Uf, const Geom& g, double courant,
                              const Dx& dx, const StepScratch& s, unsigned long long* carry_bits, int* carry_ok,
                              const int* prev_fix, int* this_fix, cudaStream_t st);
+// The status bit of the state that a run of carrying steps ended in, which no
+// CFL pass has looked at: the carried flag (then taken off), or, where the
+// FP64 fix-up changed cells after the carry (*carry_ok == 0 or, if given,
+// *prev_fix != 0), the speeds of all cells.
+cudaError_t launch_carry_status(const MixedParams& M, const double* U, float* Uf, const Geom& g,
+                                unsigned long long* carry_bits, const int* carry_ok, const int* prev_fix, int* status,
+                                cudaStream_t st);
 // FP32 CFL of the mixed form: also writes the interior of the FP32 mirror Uf
 // from U (the sweeps read the mirror; the step that wrote U left it stale).
 cudaError_t launch_cfl_mixed(const MixedParams& M, const double* U, float* Uf, const Geom& g, double courant,

@@ -89,6 +89,7 @@ struct Box {
   int* fb_other = nullptr;  // the queue length of a resident run's odd steps (fbq.n: the even ones')
   bool carry_valid = false;
   bool batch_carry = false;  // likewise since the last batch run
+  bool status_current = false;  // mixed: the status word tells of the state that a run ended in
   bool wb = false;
   bool wb_pending = false;
 };
@@ -448,7 +449,17 @@ void state_changed(Box* b) {
   b->maxu_valid = false;
   b->carry_valid = false;
   b->batch_carry = false;
+  b->status_current = false;
   b->wb_pending = false;
+}
+
+// The fix-up queue of a resident step that reads buffer `cur`: one length
+// counter per parity, zeroed by the step's CFL pass while the previous step's
+// is still read.
+FallbackQueue queue_of(const Box* b, int cur) {
+  FallbackQueue q = b->fbq;
+  if (cur) q.n = b->fb_other;
+  return q;
 }
 
 // Whether the box's copies overlap its kernels: mixed precision, 2-D or 3-D,
@@ -733,6 +744,12 @@ int rhyme_gpu_box_status(rhyme_gpu_ctx* ctx, int handle, int* flags) {
   if (!ctx || !flags) return fail(ctx, RHYME_GPU_EINVAL, "null argument");
   Box* b = find_box(ctx, handle);
   if (!b) return fail(ctx, RHYME_GPU_ENOTFOUND, "unknown box handle %d", handle);
+  // the state that a mixed run ended in has had no CFL pass of its own yet
+  if (ctx->mixed && (b->carry_valid || b->batch_carry) && !b->status_current) {
+    CK(launch_carry_status(b->mp, b->state[b->cur], b->Uf[b->cur], b->g, b->carry_bits, b->carry_ok,
+                           b->carry_valid ? queue_of(b, 1 - b->cur).n : nullptr, b->s.status, ctx->stream));
+    b->status_current = true;
+  }
   int* st = (int*)(ctx->pinned_dt + 1);
   CK(cudaMemcpyAsync(st, b->s.status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaMemsetAsync(b->s.status, 0, sizeof(int), ctx->stream));
@@ -894,7 +911,6 @@ SweepCarry carry_of(Box* b, int cur) {
   SweepCarry c;
   c.Uf_next = b->Uf[1 - cur];
   c.bits = b->carry_bits;
-  c.status = b->s.status;
   return c;
 }
 
@@ -910,15 +926,6 @@ HaloBC box_halo(const rhyme_gpu_ctx* ctx, const Box* b) {
 cudaError_t fill_after_run(rhyme_gpu_ctx* ctx, Box* b) {
   if (!fills_last(ctx, b)) return cudaSuccess;
   return launch_ghost_fill(b->dp, b->state[1 - b->cur], b->state[b->cur], b->g, ctx->stream);
-}
-
-// The fix-up queue of a resident step that reads buffer `cur`: one length
-// counter per parity, zeroed by the step's CFL pass while the previous step's
-// is still read.
-FallbackQueue queue_of(const Box* b, int cur) {
-  FallbackQueue q = b->fbq;
-  if (cur) q.n = b->fb_other;
-  return q;
 }
 
 // In mixed precision the step carries its CFL pass into the next one: the

@@ -136,9 +136,9 @@ __device__ __forceinline__ float total(float dtdx, float fl, float fr, float a_p
 }
 
 // Block-wide maximum and or of (m, bad) of a CTA of NT threads (a multiple
-// of 32), folded into *bits and *status by one thread.
+// of 32), folded into the halves of *bits by one thread (SweepCarry).
 template <int NT>
-__device__ __forceinline__ void block_fold_max(float m, int bad, unsigned long long* bits, int* status) {
+__device__ __forceinline__ void block_fold_max(float m, int bad, unsigned long long* bits) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     const float o = __shfl_down_sync(0xffffffffu, m, off);
@@ -158,8 +158,8 @@ __device__ __forceinline__ void block_fold_max(float m, int bad, unsigned long l
       if (sm[k] > m) m = sm[k];
       bad |= sb[k];
     }
-    atomicMax(bits, (unsigned long long)__float_as_uint(m));
-    if (bad) atomicOr(status, 1);
+    atomicMax((unsigned*)bits, __float_as_uint(m));
+    if (bad) atomicOr((unsigned*)bits + 1, 1u);
   }
 }
 
@@ -485,7 +485,7 @@ __device__ __forceinline__ void sweep_tile(const MixedParams& M, int limiter, fl
       }
     }
   }
-  if (carrying) block_fold_max<TileCfg<S, P>::threads>(smax, sbad, carry.bits, carry.status);
+  if (carrying) block_fold_max<TileCfg<S, P>::threads>(smax, sbad, carry.bits);
 }
 
 template <int D, int A, int S, int P, int MODE>
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(kMarchBlock, 6)
       for (int s = 0; s < D + 2; ++s) rp[s] = r[s];
     }
   }
-  if (carrying) block_fold_max<kMarchBlock>(smax, sbad, carry.bits, carry.status);
+  if (carrying) block_fold_max<kMarchBlock>(smax, sbad, carry.bits);
 }
 
 // The same sweep over the tiles of a batch of boxes, taken from a work queue
@@ -708,7 +708,6 @@ __global__ void __launch_bounds__(TileCfg<S, P>::threads, TileCfg<S, P>::templat
     if (MODE == LAST || MODE == ONLY) {
       carry.Uf_next = b.Uf_next;
       carry.bits = carry_bits_of(b);
-      carry.status = (int*)(b.ctl + 2) + 1;
     }
     sweep_tile<D, A, S, P, MODE>(M, b.limiter, b.omega_f, b.Uf, b.U, b.g, b.dx, b.ctl, b.acc, b.V,
                                  q, w.box, tA, tB, cC, sh, tma, nullptr, parity, carry, b.halo);
