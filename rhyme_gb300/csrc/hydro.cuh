@@ -65,12 +65,6 @@ __device__ __forceinline__ float m_div(float a, const Inv<float>& i) { return __
 __device__ __forceinline__ double m_div(double a, const Inv<double>& i) { return div_by(a, i.d); }
 __device__ __forceinline__ float m_div(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double m_div(double a, double b) { return div_rn(a, b); }
-// a / (2 b): the significand of 2 b is that of b
-__device__ __forceinline__ double div_half(double a, const Inv<double>& i) {
-  Divisor d = i.d;
-  d.b = f64_scale<1>(d.b);
-  return div_by(a, d);
-}
 __device__ __forceinline__ bool m_gt(float a, float b) { return a > b; }
 __device__ __forceinline__ bool m_gt(double a, double b) { return f64_gt(a, b); }
 __device__ __forceinline__ bool m_neg(float a) { return a < 0.f; }
@@ -465,7 +459,7 @@ __device__ __forceinline__ void nonlinear_waves(const Gas<double>& G, const Wave
       const double factor = m_sqrt(m_div(l ? L.Ak : R.Ak, ibp));
       const double f = dp * factor;
       // (p - pk)/(2 bp): half of the quotient by bp
-      const double fp = factor * (1.0 - div_half(dp, ibp));
+      const double fp = factor * (1.0 - div_by_twice(dp, ibp.d));
       l_f = l ? f : l_f;
       l_fp = l ? fp : l_fp;
       r_f = l ? r_f : f;
