@@ -497,7 +497,9 @@ typedef struct rhyme_gpu_request {
 typedef struct rhyme_gpu_server rhyme_gpu_server;
 
 /* base: gas, Riemann, precision (ndim, limiter, bc ignored); courant[k] is
- * the Courant number of (k+1)-D requests. */
+ * the Courant number of (k+1)-D requests. The budget bounds the boxes of the
+ * active requests together; of what finished ones leave, the server keeps up
+ * to a quarter of the budget (1 GiB at most) for the next. */
 int rhyme_gpu_server_create(const rhyme_gpu_params* base, const double courant[3],
                             long long hbm_budget_bytes, int max_active,
                             rhyme_gpu_server** server);

@@ -94,6 +94,13 @@ struct Box {
   bool wb_pending = false;
 };
 
+// A pool of device memory, made on first use, that keeps up to `keep` bytes of
+// what is freed (0: not used).
+struct DevicePool {
+  cudaMemPool_t pool = nullptr;
+  uint64_t keep = 0;
+};
+
 }  // namespace
 
 struct rhyme_gpu_ctx {
@@ -106,8 +113,7 @@ struct rhyme_gpu_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   std::vector<Box*> boxes;
-  cudaMemPool_t pool = nullptr;  // a server's: its boxes' and batches' device memory (device_alloc)
-  uint64_t pool_keep = 0;        // what the pool keeps of freed memory; 0: no pool
+  DevicePool* pool = nullptr;    // a server's (it owns it): boxes' and batches' device memory (device_alloc)
   double* pinned_dt = nullptr;   // pinned host scalars read back synchronously (dt, status, totals)
   void* elem_buf = nullptr;      // growable device buffer for element calls
   size_t elem_cap = 0;
@@ -150,28 +156,37 @@ int fail(rhyme_gpu_ctx* ctx, int code, const char* fmt, ...) {
                   "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);   \
   } while (0)
 
-// Device memory in stream order. A server's contexts have a pool of their
-// own, which keeps up to pool_keep bytes of what is freed and goes with the
-// context: the default pool gives everything back at each synchronisation,
+// Device memory in stream order. A server's contexts share a pool, which
+// keeps up to DevicePool::keep bytes of what is freed and goes with the
+// server: the default pool gives everything back at each synchronisation,
 // and admitting a box paid for the mapping again (32 painted requests: 6.8
-// against 7.6 ms). A context whose boxes stay has no use for one, and making
-// it takes 0.25 ms.
+// against 7.6 ms). One pool, so that what requests of one dimensionality left
+// serves the next ones and the server's HBM budget bounds what it holds: with
+// a pool each the contexts of an idle server kept 1.4 GB of a 2 GB budget. A
+// context whose boxes stay has no use for one, and making it takes 0.25 ms.
 cudaError_t device_alloc(rhyme_gpu_ctx* ctx, void** p, size_t bytes) {
-  if (!ctx->pool_keep) return cudaMallocAsync(p, bytes, ctx->stream);
-  if (!ctx->pool) {
+  DevicePool* P = ctx->pool;
+  if (!P || !P->keep) return cudaMallocAsync(p, bytes, ctx->stream);
+  if (!P->pool) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = ctx->device;
-    cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
+    cudaError_t e = cudaMemPoolCreate(&P->pool, &props);
     if (e != cudaSuccess) {
-      ctx->pool = nullptr;
+      P->pool = nullptr;
       return e;
     }
-    e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &ctx->pool_keep);
+    e = cudaMemPoolSetAttribute(P->pool, cudaMemPoolAttrReleaseThreshold, &P->keep);
     if (e != cudaSuccess) return e;
   }
-  return cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, P->pool, ctx->stream);
+  if (e == cudaErrorMemoryAllocation) {  // what the pool keeps in pieces too small
+    cudaGetLastError();
+    cudaMemPoolTrimTo(P->pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, P->pool, ctx->stream);
+  }
+  return e;
 }
 
 // Bounded wait on the context stream: polls an event until the deadline.
@@ -393,7 +408,6 @@ int rhyme_gpu_destroy(rhyme_gpu_ctx* ctx) {
   if (ctx->wb_done) cudaEventDestroy(ctx->wb_done);
   if (ctx->copy) cudaStreamDestroy(ctx->copy);
   cudaFreeHost(ctx->pinned_dt);
-  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return RHYME_GPU_OK;
@@ -1969,6 +1983,7 @@ struct rhyme_gpu_server {
   cudaStream_t copy = nullptr;
   std::chrono::steady_clock::time_point t0;
   std::vector<std::pair<size_t, void*>> pinned_free;  // page-locked staging pool
+  DevicePool pool;  // of the three contexts
   std::string err;
   long long cell_updates = 0;
 };
@@ -2024,6 +2039,7 @@ int rhyme_gpu_server_create(const rhyme_gpu_params* base, const double courant[3
   rhyme_gpu_server* S = new rhyme_gpu_server();
   S->budget = hbm_budget_bytes;
   S->max_active = max_active;
+  S->pool.keep = (uint64_t)std::min<long long>(1LL << 30, hbm_budget_bytes / 4);
   S->t0 = std::chrono::steady_clock::now();
   for (int k = 0; k < 3; ++k) {
     rhyme_gpu_params p = *base;
@@ -2037,7 +2053,7 @@ int rhyme_gpu_server_create(const rhyme_gpu_params* base, const double courant[3
       delete S;
       return rc;
     }
-    S->ctx[k]->pool_keep = (uint64_t)std::min<long long>(1LL << 30, hbm_budget_bytes / 4);
+    S->ctx[k]->pool = &S->pool;
   }
   if (cudaStreamCreateWithFlags(&S->copy, cudaStreamNonBlocking) != cudaSuccess) {
     for (int k = 0; k < 3; ++k) rhyme_gpu_destroy(S->ctx[k]);
@@ -2264,6 +2280,7 @@ int rhyme_gpu_server_destroy(rhyme_gpu_server* S) {
   }
   for (auto& f : S->pinned_free) cudaFreeHost(f.second);
   for (int k = 0; k < 3; ++k) rhyme_gpu_destroy(S->ctx[k]);
+  if (S->pool.pool) cudaMemPoolDestroy(S->pool.pool);
   if (S->copy) cudaStreamDestroy(S->copy);
   delete S;
   return RHYME_GPU_OK;
