@@ -367,6 +367,14 @@ int rhyme_gpu_paint(rhyme_gpu_ctx* ctx, int handle, const int left_edge[3], cons
  */
 int rhyme_gpu_sweep_plan(rhyme_gpu_ctx* ctx, int handle, const double dx[3], int tile_cells[3],
                          int tile_pencils[3]);
+/*
+ * Instrumentation (no reference counterpart): how many (box-size class, axis)
+ * pairs the context's autotuner has timed so far. The sweeps of a 1- or 2-D
+ * batch run as tiles whatever the box's size and are timed as such, apart
+ * from those of a box by itself; the solve with overlapped write-back takes
+ * the size rule's shapes.
+ */
+int rhyme_gpu_tuned_classes(rhyme_gpu_ctx* ctx, int* n);
 
 /*
  * Instrumentation (no reference counterpart): how many single-box sweep

@@ -695,7 +695,8 @@ cudaError_t launch_mh_solve_mixed_slab(const MixedParams& M, const double* U, co
   if (D < 1 || D > 3) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
   for (int a = 0; a < D && e == cudaSuccess; ++a)
-    e = launch_sweep_slab(D, a, plan.shape[a], M, Uf, U, g, dx, s.dt, acc, Unew, q, lo, hi, st);
+    e = launch_sweep_slab(D, a, plan.shape[a], M, Uf, U, g, dx, s.dt, acc, Unew, q, lo, hi, st, SweepCarry(), no_halo(),
+                          true);
   if (e == cudaSuccess) {
     switch (D) {
       case 1: e = launch_fallback<1>(M, q, g, dx, s.dt, U, Unew, st, no_halo(), done); break;

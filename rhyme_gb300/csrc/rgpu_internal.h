@@ -117,7 +117,8 @@ inline int default_sweep_shape(int ndim, int axis, int nA) {
   return k;
 }
 
-// Tile shape per axis of one box's mixed sweeps.
+// Tile shape per axis of one box's mixed sweeps (the last axis of a large box:
+// the march's segment length, sweep_marches).
 struct SweepPlan {
   int shape[3];
   int fuse_xy = 0;  // 3-D: the x and y sweeps as one kernel (sweep_xy_kernel) where it can run
@@ -150,6 +151,23 @@ inline Geom make_geom(int D, const int* dims) {
   g.s[2] = (long long)ext[0] * ext[1];
   g.field = g.s[2] * ext[2];
   return g;
+}
+
+// The last sweep of a whole 2-D or 3-D box marches along its columns
+// (march_kernel) from this many threads on (columns x segments of S cells);
+// below, too few threads wait for their chains of dependent instructions and
+// tiles are faster. Tiles against march at the best S of each: 3-D 64^3 19 /
+// 29 us, 96^3 44.2 / 43.7 (110 thousand threads), 250x130x61 88 / 82 (260),
+// 128^3 91.9 / 90.7 (262), 192^3 270 / 247, 256^3 613 / 543; 2-D 1024^2 40 /
+// 45 (131), 2047x2048 145 / 125 (524), 4096^2 518 / 421.
+constexpr long long kMarchThreads = 152 * 1024;
+inline bool sweep_marches(int ndim, int axis, int shape, const Geom& g) {
+  if (ndim < 2 || axis != ndim - 1) return false;
+  int S, P;
+  sweep_shape(ndim, shape, &S, &P);
+  const long long columns = (ndim == 3) ? (long long)g.n[0] * g.n[1] : g.n[0];
+  const int segments = (g.n[axis] + S - 1) / S;
+  return columns * segments >= kMarchThreads && columns < (1LL << 31) && segments <= 65535;
 }
 
 // Device scratch of one box for the plain FP64 solver.
@@ -520,12 +538,13 @@ long long sweep_tile_count(int ndim, int axis, int shape, const int* n);
 
 // One mixed sweep along `axis` with tile shape `shape` of the slab of a box
 // holding interior cells [lo, hi] of its outermost axis (sweeps.cu, compiled
-// once per dimensionality).
+// once per dimensionality). tiles: by tiles also where it could march.
 #define RGPU_SWEEP_DECL(D)                                                                              \
   cudaError_t launch_sweep_axis_##D(int axis, int shape, const MixedParams& M, const float* Uf,         \
                                     const double* U, const Geom& g, const Dx& dx, const double* dtp,    \
                                     float* acc, double* Unew, const FallbackQueue& q, int lo, int hi,   \
-                                    cudaStream_t st, const SweepCarry& carry, const HaloBC& halo);      \
+                                    cudaStream_t st, const SweepCarry& carry, const HaloBC& halo,       \
+                                    bool tiles);                                                        \
   cudaError_t launch_batch_sweep_axis_##D(int axis, int shape, const MixedParams& M, const BoxDesc* TB, \
                                           const WorkItem* items, int n, int* head, const FallbackQueue& q, \
                                           cudaStream_t st);
@@ -538,11 +557,11 @@ inline cudaError_t launch_sweep_slab(int ndim, int axis, int shape, const MixedP
                                      const double* U, const Geom& g, const Dx& dx, const double* dtp,
                                      float* acc, double* Unew, const FallbackQueue& q, int lo, int hi,
                                      cudaStream_t st, const SweepCarry& carry = SweepCarry(),
-                                     const HaloBC& halo = no_halo()) {
+                                     const HaloBC& halo = no_halo(), bool tiles = false) {
   switch (ndim) {
-    case 1: return launch_sweep_axis_1(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
-    case 2: return launch_sweep_axis_2(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
-    case 3: return launch_sweep_axis_3(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+    case 1: return launch_sweep_axis_1(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
+    case 2: return launch_sweep_axis_2(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
+    case 3: return launch_sweep_axis_3(axis, shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -66,8 +66,9 @@ struct Box {
   DevParams dp{};   // the context's parameters with this box's overrides
   MixedParams mp{};
   Dx dx{};          // cell size for batched steps (rhyme_gpu_batch_create)
-  SweepPlan plan{};  // tile shape per axis of the mixed sweeps
-  bool plan_valid = false;
+  SweepPlan plan{};   // tile shape per axis of the mixed sweeps (box_plan)
+  SweepPlan tiles{};  // and in a batch, as tiles of each axis by itself (tile_plan)
+  bool plan_valid = false, tiles_valid = false;
   // Copies overlapped with kernels (2-/3-D mixed boxes with a page-locked
   // host array): an upload writes the FP32 mirror of the arriving rows
   // (mirror_valid: Uf[cur] is the FP32 image of the current state, as long
@@ -797,14 +798,16 @@ StepScratch scratch_of(Box* b, bool trace) {
 // ---- autotuner of the mixed sweeps ------------------------------------------
 //
 // A box-size class is (NDIM, axis, ceil(log2) of the box's extent along the
-// axis and along the pencil axis, each clamped to [3, 10]). The first box of
+// axis and along the pencil axis, each clamped to [3, 10], and which shapes the
+// sweep would march with). The first box of
 // a class met by a context has its sweep along that axis timed with every
 // candidate tile shape on its current state (one warm-up launch on a few
 // rows, then one launch of a box of a million cells or more, whose sweep
 // takes 50 us or longer, or three of a smaller box, between CUDA events on
 // the context's stream; one synchronisation per axis); the fastest shape is
 // kept for the class. Where the x and y sweeps run as one kernel, only z is
-// tuned. A sweep only reads U^n and its FP32 mirror, so the timing launches
+// tuned; the sweeps of a batch, tiles whatever the box's size, have classes of
+// their own where another solve would march. A sweep only reads U^n and its FP32 mirror, so the timing launches
 // leave the state alone (they write the next-step buffers, which the step
 // itself overwrites). With four full launches and a synchronisation each on
 // every axis the first run of a 3-D 256^3 box took 26 ms longer than the
@@ -816,27 +819,35 @@ int size_bucket(int n) {
   return b;
 }
 
-int class_key(int D, int axis, const Geom& g) {
+int class_key(int D, int axis, const Geom& g, bool tiles) {
   const int bax = (D == 1) ? 1 : (axis == 0 ? 1 : 0);
   const int nB = (bax < D) ? g.n[bax] : 1;
-  return D | (axis << 2) | (size_bucket(g.n[axis]) << 4) | (size_bucket(nB) << 8);
+  int key = D | (axis << 2) | (size_bucket(g.n[axis]) << 4) | (size_bucket(nB) << 8);
+  for (int k = 0; k < kSweepShapes; ++k)
+    if (!tiles && sweep_marches(D, axis, k, g)) key |= 1 << (12 + k);
+  return key;
 }
 
-// Before a box's first tune_axis: the mirror, its ghosts, dt and, where one
-// kernel runs the x and y sweeps, what it leaves for the z sweep.
-int tune_begin(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, bool fused) {
+// Before a box's first tune_axis: the mirror, its ghosts, dt and what the
+// sweeps before `axis` leave for it.
+int tune_begin(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, const SweepPlan& plan, int axis, bool fused) {
   const int c = b->cur;
   StepScratch sc = scratch_of(b, false);
   CK(launch_cfl_mixed(b->mp, b->state[c], b->Uf[c], b->g, b->dp.courant, dx, sc, ctx->stream));
   CK(launch_ghost_fill_f32(b->dp, b->Uf[c], b->g, ctx->stream));
   b->mirror_valid = false;  // the FP32 ghosts were filled without the FP64 ones
-  if (!fused) return RHYME_GPU_OK;
   CK(cudaMemsetAsync(b->fbq.n, 0, sizeof(int), ctx->stream));
-  CK(launch_sweep_xy_3(b->mp, b->Uf[c], b->g, dx, sc.dt, b->acc, b->fbq, no_halo(), ctx->stream));
+  if (fused) {
+    CK(launch_sweep_xy_3(b->mp, b->Uf[c], b->g, dx, sc.dt, b->acc, b->fbq, no_halo(), ctx->stream));
+    return RHYME_GPU_OK;
+  }
+  for (int a = 0; a < axis; ++a)
+    CK(launch_sweep_axis(ctx->params.ndim, a, plan.shape[a], b->mp, b->Uf[c], b->state[c], b->g, dx, sc.dt, b->acc,
+                         b->state[1 - c], b->fbq, ctx->stream));
   return RHYME_GPU_OK;
 }
 
-int tune_axis(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, int axis, int* best) {
+int tune_axis(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, int axis, bool tiles, int* best) {
   const int D = ctx->params.ndim;
   const int c = b->cur;
   StepScratch sc = scratch_of(b, false);
@@ -851,7 +862,7 @@ int tune_axis(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, int axis, int* best) {
     cudaError_t r = cudaMemsetAsync(b->fbq.n, 0, sizeof(int), ctx->stream);
     if (r == cudaSuccess)
       r = launch_sweep_slab(D, axis, k, b->mp, b->Uf[c], b->state[c], b->g, dx, sc.dt, b->acc, b->state[1 - c], b->fbq,
-                            1, hi, ctx->stream);
+                            1, hi, ctx->stream, SweepCarry(), no_halo(), tiles);
     if (r == cudaErrorInvalidConfiguration) {  // grid too large for this shape
       ok[k] = false;
       r = cudaSuccess;
@@ -886,34 +897,53 @@ int tune_axis(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, int axis, int* best) {
   return rc;
 }
 
-// The box's tile shapes (mixed mode): from the class table, tuning the
-// classes not seen yet (RHYME_GPU_TUNE_AUTO), or by the size rule. Must run
-// outside stream capture.
+// A box's tile shapes by the size rule.
+SweepPlan rule_plan(int D, const Geom& g) {
+  SweepPlan plan;
+  for (int a = 0; a < 3; ++a) plan.shape[a] = default_sweep_shape(D, a < D ? a : 0, g.n[a < D ? a : 0]);
+  return plan;
+}
+
+// A box's tile shapes (mixed mode): from the class table, tuning the classes
+// not seen yet (RHYME_GPU_TUNE_AUTO), or by the size rule. tiles: of sweeps
+// that run as tiles of each axis by itself. Must run outside stream capture.
+int make_plan(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, bool tiles, SweepPlan* plan) {
+  const int D = ctx->params.ndim;
+  *plan = rule_plan(D, b->g);
+  plan->fuse_xy = (!tiles && D == 3 && ctx->fuse_xy) ? 1 : 0;
+  if (ctx->params.sweep_tuning != RHYME_GPU_TUNE_AUTO) return RHYME_GPU_OK;
+  const bool fused = plan->fuse_xy && sweep_xy_runs(b->Uf[0], b->g) && sweep_xy_runs(b->Uf[1], b->g);
+  bool begun = false;
+  for (int a = fused ? 2 : 0; a < D; ++a) {
+    const int key = class_key(D, a, b->g, tiles);
+    auto it = ctx->tuned.find(key);
+    if (it == ctx->tuned.end()) {
+      int rc = RHYME_GPU_OK;
+      if (!begun) rc = tune_begin(ctx, b, dx, *plan, a, fused);
+      begun = true;
+      int best = 0;
+      if (rc == RHYME_GPU_OK) rc = tune_axis(ctx, b, dx, a, tiles, &best);
+      if (rc != RHYME_GPU_OK) return rc;
+      it = ctx->tuned.emplace(key, best).first;
+    }
+    plan->shape[a] = it->second;
+  }
+  return RHYME_GPU_OK;
+}
+
+// The plan of the solves of the whole box, and the one of a batch's unfused
+// sweeps, which are tiles whatever the box's size.
 int box_plan(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx) {
   if (!ctx->mixed || b->plan_valid) return RHYME_GPU_OK;
-  const int D = ctx->params.ndim;
-  for (int a = 0; a < 3; ++a) b->plan.shape[a] = default_sweep_shape(D, a < D ? a : 0, b->g.n[a < D ? a : 0]);
-  b->plan.fuse_xy = (D == 3 && ctx->fuse_xy) ? 1 : 0;
-  if (ctx->params.sweep_tuning == RHYME_GPU_TUNE_AUTO) {
-    const bool fused = b->plan.fuse_xy && sweep_xy_runs(b->Uf[0], b->g) && sweep_xy_runs(b->Uf[1], b->g);
-    bool begun = false;
-    for (int a = fused ? 2 : 0; a < D; ++a) {
-      const int key = class_key(D, a, b->g);
-      auto it = ctx->tuned.find(key);
-      if (it == ctx->tuned.end()) {
-        int rc = RHYME_GPU_OK;
-        if (!begun) rc = tune_begin(ctx, b, dx, fused);
-        begun = true;
-        int best = 0;
-        if (rc == RHYME_GPU_OK) rc = tune_axis(ctx, b, dx, a, &best);
-        if (rc != RHYME_GPU_OK) return rc;
-        it = ctx->tuned.emplace(key, best).first;
-      }
-      b->plan.shape[a] = it->second;
-    }
-  }
-  b->plan_valid = true;
-  return RHYME_GPU_OK;
+  const int rc = make_plan(ctx, b, dx, false, &b->plan);
+  b->plan_valid = rc == RHYME_GPU_OK;
+  return rc;
+}
+int tile_plan(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx) {
+  if (!ctx->mixed || b->tiles_valid) return RHYME_GPU_OK;
+  const int rc = make_plan(ctx, b, dx, true, &b->tiles);
+  b->tiles_valid = rc == RHYME_GPU_OK;
+  return rc;
 }
 
 // One captured step: CFL pass (dt; in mixed precision also the FP32
@@ -1002,16 +1032,22 @@ int step_graph(rhyme_gpu_ctx* ctx, Box* b, int cur, bool many, const Dx& dx, cud
 // every sweep's tile extent along it), each slab's finished rows copied to
 // the host array on the copy stream while the next slab is solved. A slab's
 // last row waits for the next slab, which may queue the FP64 fix-up of the
-// interface between them. The context stream waits for the copies.
+// interface between them. The context stream waits for the copies. The tile
+// shapes are the size rule's: its 16 rows along the outermost axis keep the
+// slabs small, and timing all three axes' tiles would give 1 % of the sweeps
+// (256^3: x, y, z 409, 435, 540 us by the rule, 409, 433, 540 the fastest of
+// the four; 160^3 106, 112, 138 and 105, 112, 138; 72^3 19.0, 17.7, 21.2 and
+// 16.9, 17.7, 21.2) for 8.6 ms at 256^3 and 2.7 at 160^3 in the first solve.
 int solve_slabs_write_back(rhyme_gpu_ctx* ctx, Box* b, const Dx& d) {
   int rc = ensure_copy_stream(ctx);
   if (rc != RHYME_GPU_OK) return rc;
   const int D = ctx->params.ndim, O = D - 1;
   const int N = b->g.n[O];
+  const SweepPlan plan = rule_plan(D, b->g);
   int align = 1;
   for (int a = 0; a < D; ++a) {
     int S = 1, P = 1;
-    sweep_shape(D, b->plan.shape[a], &S, &P);
+    sweep_shape(D, plan.shape[a], &S, &P);
     const int bax = (a == 0) ? 1 : 0;
     const int t = (a == O) ? S : (bax == O ? P : 1);
     if (t > align) align = t;
@@ -1029,7 +1065,7 @@ int solve_slabs_write_back(rhyme_gpu_ctx* ctx, Box* b, const Dx& d) {
   int j = 0;
   for (int lo = 1; lo <= N; lo += rows, ++j) {
     const int hi = std::min(N, lo + rows - 1);
-    CK(launch_mh_solve_mixed_slab(b->mp, U, b->Uf[b->cur], V, b->acc, b->g, d, sc, b->fbq, b->fb_done, b->plan,
+    CK(launch_mh_solve_mixed_slab(b->mp, U, b->Uf[b->cur], V, b->acc, b->g, d, sc, b->fbq, b->fb_done, plan,
                                   lo, hi, ctx->stream));
     // final: array rows up to the one of cell hi - 1 (cell i is array row
     // i + 1), or all of them after the last slab
@@ -1089,7 +1125,8 @@ int rhyme_gpu_mh_solve(rhyme_gpu_ctx* ctx, int handle, const double dx[3], doubl
   if (!b) return fail(ctx, RHYME_GPU_ENOTFOUND, "unknown box handle %d", handle);
   if (!(dt > 0.0) || !std::isfinite(dt)) return fail(ctx, RHYME_GPU_EINVAL, "dt must be positive and finite");
   Dx d = make_dx(ctx->params.ndim, dx);
-  int rc = box_plan(ctx, b, d);
+  const bool slabs = b->wb && pipelined(ctx, b);
+  int rc = slabs ? RHYME_GPU_OK : box_plan(ctx, b, d);
   if (rc != RHYME_GPU_OK) return rc;
   // dt by value through a one-thread kernel: no host staging buffer, so no
   // wait for the stream (the host enqueues the solve while the ghost fill
@@ -1104,7 +1141,7 @@ int rhyme_gpu_mh_solve(rhyme_gpu_ctx* ctx, int handle, const double dx[3], doubl
     if (!b->mirror_valid)
       CK(launch_to_f32(b->state[b->cur], b->Uf[b->cur], (long long)(ctx->params.ndim + 2) * b->g.field,
                        ctx->stream));
-    if (b->wb && pipelined(ctx, b)) {
+    if (slabs) {
       rc = solve_slabs_write_back(ctx, b, d);
       if (rc != RHYME_GPU_OK) return rc;
       written_back = true;
@@ -1613,6 +1650,12 @@ extern "C" int rhyme_gpu_sweep_plan(rhyme_gpu_ctx* ctx, int handle, const double
   return RHYME_GPU_OK;
 }
 
+extern "C" int rhyme_gpu_tuned_classes(rhyme_gpu_ctx* ctx, int* n) {
+  if (!ctx || !n) return fail(ctx, RHYME_GPU_EINVAL, "null argument");
+  *n = (int)ctx->tuned.size();
+  return RHYME_GPU_OK;
+}
+
 extern "C" int rhyme_gpu_fallback_count(rhyme_gpu_ctx* ctx, int handle, long long* count) {
   if (!ctx || !count) return fail(ctx, RHYME_GPU_EINVAL, "null argument");
   Box* b = find_box(ctx, handle);
@@ -1707,7 +1750,7 @@ int batch_build(rhyme_gpu_batch* B) {
   for (int i = 0; i < n; ++i) {
     Box* b = ctx->boxes[B->handles[i]];
     if (!fuse) {  // (a fused batch's shapes follow from its boxes' sizes)
-      int rc = box_plan(ctx, b, b->dx);
+      int rc = tile_plan(ctx, b, b->dx);
       if (rc != RHYME_GPU_OK) return rc;
     }
     B->base_cur[i] = b->cur;
@@ -1757,7 +1800,7 @@ int batch_build(rhyme_gpu_batch* B) {
         for (long long t = 0; t < nt; ++t) sweep[0][k].push_back({i, 0, t});
       }
       for (int a = fuse ? 2 : 0; a < D; ++a) {
-        const int k = fuse ? batch_z_shape(g.n[0], g.n[2]) : b->plan.shape[a];
+        const int k = fuse ? batch_z_shape(g.n[0], g.n[2]) : b->tiles.shape[a];
         const long long nt = sweep_tile_count(D, a, k, g.n);
         for (long long t = 0; t < nt; ++t) sweep[a][k].push_back({i, a, t});
       }

@@ -29,19 +29,10 @@ constexpr int mode_of() {
 // (O = A, or O = B across the pencils) the slab must start on a tile
 // boundary and end on one or at the box's edge, so that every cell belongs
 // to exactly one slab.
-// From this many threads on (columns x segments of S cells) the last sweep
-// marches along its columns (march_kernel); below, too few threads wait for
-// their chains of dependent instructions and tiles are faster. Tiles against
-// march at the best S of each: 3-D 64^3 19 / 29 us, 96^3 44.2 / 43.7 (110
-// thousand threads), 250x130x61 88 / 82 (260), 128^3 91.9 / 90.7 (262), 192^3
-// 270 / 247, 256^3 613 / 543; 2-D 1024^2 40 / 45 (131), 2047x2048 145 / 125
-// (524), 4096^2 518 / 421.
-constexpr long long kMarchThreads = 152 * 1024;
-
 template <int D, int A, int S, int P>
 cudaError_t launch_one(const MixedParams& M, const float* Uf, const double* U, const Geom& g, const Dx& dx,
                        const double* dtp, float* acc, double* Unew, const FallbackQueue& q, int lo, int hi,
-                       cudaStream_t st, const SweepCarry& carry, const HaloBC& halo) {
+                       cudaStream_t st, const SweepCarry& carry, const HaloBC& halo, bool tiles) {
   constexpr int B = Axes<D, A>::B, C = Axes<D, A>::C;
   constexpr int O = D - 1;
   const int NO = g.n[O];
@@ -51,11 +42,13 @@ cudaError_t launch_one(const MixedParams& M, const float* Uf, const double* U, c
     if ((lo - 1) % T != 0 || (hi != NO && (hi - lo + 1) % T != 0)) return cudaErrorInvalidValue;
   }
   if constexpr (D > 1 && A == D - 1) {
-    const long long columns = (D == 3) ? (long long)g.n[0] * g.n[1] : g.n[0];
-    const int segments = (NO + S - 1) / S;
-    if (lo == 1 && hi == NO && columns * segments >= kMarchThreads && columns < (1LL << 31) && segments <= 65535)
-      return launch_step(march_kernel<D>, dim3((unsigned)((columns + kMarchBlock - 1) / kMarchBlock), (unsigned)segments),
+    constexpr int shape = S == 8 ? 0 : S == 16 ? 1 : S == 32 ? 2 : 3;
+    if (!tiles && lo == 1 && hi == NO && sweep_marches(D, A, shape, g)) {
+      const long long columns = (D == 3) ? (long long)g.n[0] * g.n[1] : g.n[0];
+      return launch_step(march_kernel<D>,
+                         dim3((unsigned)((columns + kMarchBlock - 1) / kMarchBlock), (unsigned)((NO + S - 1) / S)),
                          dim3(kMarchBlock), st, M, Uf, U, g, dx, dtp, acc, Unew, q, S, carry, halo);
+    }
   }
   Geom gs = g;
   FallbackQueue qs = q;
@@ -96,20 +89,20 @@ template <int D, int A>
 cudaError_t by_shape(int shape, const MixedParams& M, const float* Uf, const double* U, const Geom& g,
                      const Dx& dx, const double* dtp, float* acc, double* Unew,
                      const FallbackQueue& q, int lo, int hi, cudaStream_t st, const SweepCarry& carry,
-                     const HaloBC& halo) {
+                     const HaloBC& halo, bool tiles) {
   if constexpr (D == 1) {
     switch (shape) {
-      case 0: return launch_one<D, A, 64, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
-      case 1: return launch_one<D, A, 128, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
-      case 2: return launch_one<D, A, 256, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
-      case 3: return launch_one<D, A, 512, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      case 0: return launch_one<D, A, 64, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
+      case 1: return launch_one<D, A, 128, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
+      case 2: return launch_one<D, A, 256, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
+      case 3: return launch_one<D, A, 512, 1>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
     }
   } else {
     switch (shape) {
-      case 0: return launch_one<D, A, 8, 32>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
-      case 1: return launch_one<D, A, 16, 16>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
-      case 2: return launch_one<D, A, 32, 8>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
-      case 3: return launch_one<D, A, 64, 4>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      case 0: return launch_one<D, A, 8, 32>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
+      case 1: return launch_one<D, A, 16, 16>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
+      case 2: return launch_one<D, A, 32, 8>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
+      case 3: return launch_one<D, A, 64, 4>(M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
     }
   }
   return cudaErrorInvalidValue;
@@ -145,15 +138,15 @@ cudaError_t RGPU_CAT(launch_sweep_axis_, SWEEP_D)(int axis, int shape, const Mix
                                                  const double* U, const Geom& g, const Dx& dx,
                                                  const double* dtp, float* acc, double* Unew,
                                                  const FallbackQueue& q, int lo, int hi, cudaStream_t st,
-                                                 const SweepCarry& carry, const HaloBC& halo) {
+                                                 const SweepCarry& carry, const HaloBC& halo, bool tiles) {
   constexpr int D = SWEEP_D;
   switch (axis) {
-    case 0: return by_shape<D, 0>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+    case 0: return by_shape<D, 0>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
     case 1:
-      if constexpr (D > 1) return by_shape<D, 1>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      if constexpr (D > 1) return by_shape<D, 1>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
       break;
     case 2:
-      if constexpr (D > 2) return by_shape<D, 2>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo);
+      if constexpr (D > 2) return by_shape<D, 2>(shape, M, Uf, U, g, dx, dtp, acc, Unew, q, lo, hi, st, carry, halo, tiles);
       break;
   }
   return cudaErrorInvalidValue;

@@ -38,7 +38,7 @@ EXPORTS = ["rhyme_gpu_abi_version", "rhyme_gpu_create", "rhyme_gpu_destroy", "rh
            "rhyme_gpu_batch_create", "rhyme_gpu_batch_run", "rhyme_gpu_batch_dt", "rhyme_gpu_batch_destroy",
            "rhyme_gpu_server_create", "rhyme_gpu_server_submit", "rhyme_gpu_server_tick",
            "rhyme_gpu_server_request", "rhyme_gpu_server_stats", "rhyme_gpu_server_last_error",
-           "rhyme_gpu_server_destroy", "rhyme_gpu_sweep_plan",
+           "rhyme_gpu_server_destroy", "rhyme_gpu_sweep_plan", "rhyme_gpu_tuned_classes",
            "rhyme_gpu_output_level", "rhyme_gpu_output_wait", "rhyme_gpu_box_totals",
            "rhyme_gpu_sanity_check", "rhyme_gpu_paint"]
 REQ_PENDING, REQ_ACTIVE, REQ_DRAINING, REQ_DONE = 0, 1, 2, 3
@@ -165,6 +165,7 @@ def load():
     L.rhyme_gpu_rate_probe.argtypes = [C.c_int, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]
     L.rhyme_gpu_check_conversions.argtypes = [C.c_longlong, C.c_ulonglong, C.POINTER(C.c_ulonglong)]
     L.rhyme_gpu_sweep_plan.argtypes = [vp, C.c_int, dp, ip, ip]
+    L.rhyme_gpu_tuned_classes.argtypes = [vp, ip]
     L.rhyme_gpu_output_level.argtypes = [vp, ip, C.c_int, C.c_int, C.POINTER(C.c_float), C.c_longlong]
     L.rhyme_gpu_output_wait.argtypes = [vp]
     L.rhyme_gpu_box_totals.argtypes = [vp, C.c_int, dp]
@@ -368,6 +369,12 @@ class Context:
                                                   s.ctypes.data_as(C.POINTER(C.c_int)),
                                                   p.ctypes.data_as(C.POINTER(C.c_int))))
         return [(int(a), int(b)) for a, b in zip(s, p) if a]
+
+    def tuned_classes(self):
+        """(box-size class, axis) pairs the autotuner has timed so far."""
+        n = C.c_int()
+        self._check(self.lib.rhyme_gpu_tuned_classes(self.h, C.byref(n)))
+        return n.value
 
     def output_level(self, boxes, ncmp=None, out=None):
         """Start the level output of `boxes` (the Chombo "data:datatype=0"
