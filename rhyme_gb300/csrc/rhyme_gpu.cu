@@ -802,7 +802,8 @@ StepScratch scratch_of(Box* b, bool trace) {
 // sweep would march with). The first box of
 // a class met by a context has its sweep along that axis timed with every
 // candidate tile shape on its current state (one warm-up launch on a few
-// rows, then one launch of a box of a million cells or more, whose sweep
+// rows, the march once on the whole box since S is an argument of its only
+// kernel: without it the first S was charged 8 to 11 us for loading it; then one launch of a box of a million cells or more, whose sweep
 // takes 50 us or longer, or three of a smaller box, between CUDA events on
 // the context's stream; one synchronisation per axis); the fastest shape is
 // kept for the class. Where the x and y sweeps run as one kernel, only z is
@@ -856,7 +857,7 @@ int tune_axis(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, int axis, bool tiles, in
   const int rows = std::min(nO, D == 1 ? 512 : 64);  // whole tiles of every shape
   const int reps = (long long)b->g.n[0] * b->g.n[1] * b->g.n[2] >= 1000000 ? 1 : 3;
   cudaEvent_t ev[kSweepShapes][2] = {};
-  bool ok[kSweepShapes];
+  bool ok[kSweepShapes], marched = false;
   cudaError_t e = cudaSuccess;
   auto sweep = [&](int k, int hi) {
     cudaError_t r = cudaMemsetAsync(b->fbq.n, 0, sizeof(int), ctx->stream);
@@ -873,7 +874,9 @@ int tune_axis(rhyme_gpu_ctx* ctx, Box* b, const Dx& dx, int axis, bool tiles, in
     ok[k] = true;
     for (cudaEvent_t& v : ev[k])
       if (e == cudaSuccess) e = cudaEventCreate(&v);
-    if (e == cudaSuccess) e = sweep(k, rows);
+    const bool marches = !tiles && sweep_marches(D, axis, k, b->g);
+    if (e == cudaSuccess && !(marches && marched)) e = sweep(k, marches ? nO : rows);
+    marched = marched || marches;
     if (e == cudaSuccess) e = cudaEventRecord(ev[k][0], ctx->stream);
     for (int rep = 0; rep < reps && ok[k] && e == cudaSuccess; ++rep) e = sweep(k, nO);
     if (e == cudaSuccess) e = cudaEventRecord(ev[k][1], ctx->stream);
