@@ -317,18 +317,29 @@ __device__ __forceinline__ void limited_slopes(int type, double w, const double*
 #pragma unroll
   for (int c = 0; c < N; ++c) delta[c] = limited_slope_f64(type, w, ul[c], u[c], ur[c]);
 }
+// The FP32 quotients by d_R are 0 where it is beyond 2^126 (__fdividef): such
+// a cell's density slope becomes a NaN, which makes its face states none that
+// the FP32 solve takes, and FP64 redoes both interfaces. The sum of all |d_R|
+// tells (four times it is infinite then, and a product with 0 a NaN): six
+// instructions of the FP32 pipe where the limiter divides (256^3 superbee, x+y
+// 768 -> 774 us; with the largest |d_R|, a comparison and a selection 777).
 template <int N>
 __device__ __forceinline__ void limited_slopes(int type, float w, const float* ul, const float* u, const float* ur,
                                                float* delta) {
-  auto each = [&](auto slope) {
+  auto each = [&](auto slope, bool divides) {
+    float sum = 0.f;
 #pragma unroll
-    for (int c = 0; c < N; ++c) delta[c] = slope(ul[c], u[c], ur[c]);
+    for (int c = 0; c < N; ++c) {
+      delta[c] = slope(ul[c], u[c], ur[c]);
+      sum = sum + fabsf(ur[c] - u[c]);
+    }
+    if (divides) delta[0] = __fmaf_rn(__fmul_rn(4.f, sum), 0.f, delta[0]);
   };
-  if (w != 0.f) each([&](float a, float b, float c) { return limited_slope_w_f32(type, w, a, b, c); });
-  else if (type == 1) each(limited_slope_w0_f32<1>);
-  else if (type == 2) each(limited_slope_w0_f32<2>);
-  else if (type == 3) each(limited_slope_w0_f32<3>);
-  else each(limited_slope_w0_f32<4>);
+  if (w != 0.f) each([&](float a, float b, float c) { return limited_slope_w_f32(type, w, a, b, c); }, true);
+  else if (type == 1) each(limited_slope_w0_f32<1>, false);
+  else if (type == 2) each(limited_slope_w0_f32<2>, true);
+  else if (type == 3) each(limited_slope_w0_f32<3>, true);
+  else each(limited_slope_w0_f32<4>, true);
 }
 
 // The difference of the FP32 fluxes of l and r (rhyme_ideal_gas_flux.f90:
