@@ -234,7 +234,7 @@ __device__ __forceinline__ double signal_speed_elem(const Gas<double>& G, const 
   double ss = 0.0;
 #pragma unroll
   for (int a = 0; a < D; ++a) ss = ss + u[1 + a] * u[1 + a];
-  const Inv<double> i0 = m_inv(u[0]);
+  const Divisor i0 = divisor(u[0]);
   const double v = m_div(m_sqrt(ss), i0) + sound_speed<D>(G, u, i0);
   if (!(u[0] > 0.0) || !isfinite(v)) bad = 1;
   return v;

@@ -1,9 +1,10 @@
 // hydro.cuh -- device functions of the MUSCL-Hancock step: ideal-gas EOS,
 // slope limiters, half-step extrapolation and the exact Riemann solver.
 //
-// Templated on NDIM (D), on the normal axis (AX, compile-time so no state
-// vector is indexed dynamically) and on the arithmetic type T (double for the
-// plain path, float for the FP32 stages of the mixed path). Each routine keeps
+// Templated on NDIM (D) and on the normal axis (AX, compile-time so no state
+// vector is indexed dynamically); double for the plain path and the mixed
+// path's redone interfaces, float for the FP32 stages of the mixed path. Each
+// FP64 routine keeps
 // the floating-point evaluation order of the Fortran routine it restates
 // (operators of equal precedence left to right), so that with FMA contraction
 // disabled the double instantiation performs the same IEEE operations as the
@@ -29,7 +30,6 @@ namespace rgpu {
 // FP64 path returns the reference's bits even in flows that amplify a one-ulp
 // difference; libm_pow_int.h forms them mostly in integers.
 __device__ __forceinline__ double m_sqrt(double x) { return sqrt_rn(x); }
-__device__ __forceinline__ float m_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double m_pow(double x, double y) { return libm_pow_int::pow(x, y); }
 // Float powers as 2^(y log2 x) with CUDA's log2f and exp2f: the rounding of
 // the product adds a relative error of about 2^-24 |y log2 x| to the result
@@ -47,46 +47,20 @@ __device__ __forceinline__ void m_pow2(float x, float y1, float y2, float& r1, f
   r1 = exp2f(y1 * l);
   r2 = exp2f(y2 * l);
 }
-__device__ __forceinline__ double m_abs(double x) { return fabs(x); }
-__device__ __forceinline__ float m_abs(float x) { return fabsf(x); }
 
-// Divisions, comparisons and powers of two: FP64 through the integer forms
-// of fp64_int.h (the same bits; a division or a comparison on the FP64 pipe
-// costs 550 or 64 cycles a warp), FP32 as written. Inv is a divisor used
-// several times.
-template <typename T> struct Inv;
-template <> struct Inv<float> { float b; };
-template <> struct Inv<double> { Divisor d; };
-__host__ __device__ __forceinline__ Inv<float> m_inv(float b) { return {b}; }
-__host__ __device__ __forceinline__ Inv<double> m_inv(double b) { return {divisor(b)}; }
-// a/b as a times the approximate reciprocal of b (2 ulp for |b| <= 2^126),
-// without the scaling that the division operator adds for larger divisors.
-__device__ __forceinline__ float m_div(float a, const Inv<float>& i) { return __fdividef(a, i.b); }
-__device__ __forceinline__ double m_div(double a, const Inv<double>& i) { return div_by(a, i.d); }
-__device__ __forceinline__ float m_div(float a, float b) { return __fdividef(a, b); }
+// FP64 divisions, comparisons and powers of two through the integer forms of
+// fp64_int.h (the same bits; a division or a comparison on the FP64 pipe costs
+// 550 or 64 cycles a warp). A Divisor is a divisor used several times.
+__device__ __forceinline__ double m_div(double a, const Divisor& d) { return div_by(a, d); }
 __device__ __forceinline__ double m_div(double a, double b) { return div_rn(a, b); }
-__device__ __forceinline__ bool m_gt(float a, float b) { return a > b; }
 __device__ __forceinline__ bool m_gt(double a, double b) { return f64_gt(a, b); }
-__device__ __forceinline__ bool m_neg(float a) { return a < 0.f; }
 __device__ __forceinline__ bool m_neg(double a) { return f64_negative(a); }
-__device__ __forceinline__ float m_half(float a) { return 0.5f * a; }
 __device__ __forceinline__ double m_half(double a) { return f64_scale<-1>(a); }
-__device__ __forceinline__ float m_twice(float a) { return 2.f * a; }
 __device__ __forceinline__ double m_twice(double a) { return f64_scale<1>(a); }
-__device__ __forceinline__ bool m_tiny(float a) { return fabsf(a) < FLT_MIN; }
-__device__ __forceinline__ bool m_tiny(double a) { return f64_tiny(a); }
-
-template <typename T> struct Limits;
-template <> struct Limits<double> {
-  __device__ static constexpr double tiny() { return DBL_MIN; }
-};
-template <> struct Limits<float> {
-  __device__ static constexpr float tiny() { return FLT_MIN; }
-};
 
 // Fortran MAX/MIN of two reals (same ternary as the CPU oracle).
-template <typename T> __device__ __forceinline__ T fmax_ref(T a, T b) { return m_gt(b, a) ? b : a; }
-template <typename T> __device__ __forceinline__ T fmin_ref(T a, T b) { return m_gt(a, b) ? b : a; }
+__device__ __forceinline__ double fmax_ref(double a, double b) { return m_gt(b, a) ? b : a; }
+__device__ __forceinline__ double fmin_ref(double a, double b) { return m_gt(a, b) ? b : a; }
 // FP32: one instruction, which like the selections above keeps a NaN in a.
 __device__ __forceinline__ float fmax_ref(float a, float b) {
   float r;
@@ -103,90 +77,92 @@ __device__ __forceinline__ float fmin_ref(float a, float b) {
 // rhyme_irs_init.f90:21-27) plus the literal quotients the reference
 // recomputes at each use (2/gp1, 2/gm1, 1/gm1_2g, gm1/2): the same values.
 template <typename T>
-struct Gas {
+struct GasOnly;  // what one of the two forms needs besides
+template <>
+struct GasOnly<double> {
+  Divisor by_gm1, by_gp1, by_kb_amu;
+};
+template <>
+struct GasOnly<float> {
+  float gm1_lo, g_gm1;  // what rounding gm1 to FP32 lost; gamma/(gamma-1)
+};
+template <typename T>
+struct Gas : GasOnly<T> {
   T g, gm1, gp1, gm1_gp1, gm1_2g, gp1_2g, g_inv, kb_amu;
   T two_gp1, two_gm1, inv_gm1_2g, gm1_half, half_gm1, g_kb_amu;
-  Inv<T> by_gm1, by_gp1, by_kb_amu;  // divisors
-  T gm1_lo, g_gm1;  // FP32: what rounding gm1 to FP32 lost; gamma/(gamma-1)
 };
 
 // Run parameters used inside kernels.
 template <typename T>
 struct Rp {
   T vac_rho, vac_p, vac_rho_next;  // w_vacuum(rho), w_vacuum(p), nearest(w_vac_rho, +1)
-  T tol;
-  T last;  // FP32: relative size of a step of rp_flux_f32's iteration that ends it
+  T tol;  // FP64: the tolerance; FP32: the relative size of a step that ends rp_flux_f32's iteration
   int n_iter;
-};
-
-struct Limiter {
-  int type;
-  double w;
 };
 
 // ---- EOS: rhyme_hydro_base / rhyme_ideal_gas ------------------------------
 
-// rhyme_hydro_base_specific_kinetic_energy.f90:9; i0: the density as a divisor
-template <int D, typename T>
-__device__ __forceinline__ T sp_kin_e(const T* u) {
-  T s = T(0);
+// rhyme_hydro_base_specific_kinetic_energy.f90:9
+template <int D>
+__device__ __forceinline__ double sp_kin_e(const double* u) {
+  double s = 0.0;
 #pragma unroll
   for (int a = 0; a < D; ++a) s = s + u[1 + a] * u[1 + a];
   return m_div(m_half(s), u[0] * u[0]);
 }
 
-// rhyme_hydro_base_specific_internal_energy.f90:9
-template <int D, typename T>
-__device__ __forceinline__ T sp_int_e(const T* u, const Inv<T>& i0) {
+// rhyme_hydro_base_specific_internal_energy.f90:9; i0: the density as a divisor
+template <int D>
+__device__ __forceinline__ double sp_int_e(const double* u, const Divisor& i0) {
   return m_div(u[D + 1], i0) - sp_kin_e<D>(u);
 }
 
-// The FP32 forms of the mixed sweeps (pressure, sound speed, flux) are the
-// same quantities with fewer divisions: p = (E - |m|^2 / (2 rho)) (gamma-1)
-// for rho e_int (gamma-1), cs = sqrt(gamma p / rho) for
-// sqrt(gamma kB/amu T/mu), and the flux from one reciprocal of rho. FP32
-// division is a reciprocal and a multiply plus range handling; the sweeps
-// divide a lot (256^3 mixed step 2.43 -> 2.20 ms, L1(rho) against FP64 a
-// little lower). The double forms keep the reference's operations.
-
 // rhyme_ideal_gas_pressure.f90:9
-template <int D, typename T>
-__device__ __forceinline__ T pressure(const Gas<T>& G, const T* u, const Inv<T>& i0) {
-  if constexpr (sizeof(T) == sizeof(float)) {
-    T s = T(0);
-#pragma unroll
-    for (int a = 0; a < D; ++a) s = s + u[1 + a] * u[1 + a];
-    return (u[D + 1] - T(0.5) * s / u[0]) * G.gm1;
-  }
+template <int D>
+__device__ __forceinline__ double pressure(const Gas<double>& G, const double* u, const Divisor& i0) {
   return u[0] * sp_int_e<D>(u, i0) * G.gm1;
 }
-template <int D, typename T>
-__device__ __forceinline__ T pressure(const Gas<T>& G, const T* u) {
-  return pressure<D>(G, u, m_inv(u[0]));
+template <int D>
+__device__ __forceinline__ double pressure(const Gas<double>& G, const double* u) {
+  return pressure<D>(G, u, divisor(u[0]));
 }
 
 // rhyme_ideal_gas_temperature_per_mu.f90:9-10, _speed_of_sound.f90:9
-template <int D, typename T>
-__device__ __forceinline__ T sound_speed(const Gas<T>& G, const T* u, const Inv<T>& i0) {
-  if constexpr (sizeof(T) == sizeof(float)) return m_sqrt(G.g * pressure<D>(G, u) / u[0]);
-  T t_mu = m_div(sp_int_e<D>(u, i0) * G.gm1, G.by_kb_amu);
+template <int D>
+__device__ __forceinline__ double sound_speed(const Gas<double>& G, const double* u, const Divisor& i0) {
+  const double t_mu = m_div(sp_int_e<D>(u, i0) * G.gm1, G.by_kb_amu);
   return m_sqrt(G.g_kb_amu * t_mu);
 }
-template <int D, typename T>
-__device__ __forceinline__ T sound_speed(const Gas<T>& G, const T* u) {
-  return sound_speed<D>(G, u, m_inv(u[0]));
+template <int D>
+__device__ __forceinline__ double sound_speed(const Gas<double>& G, const double* u) {
+  return sound_speed<D>(G, u, divisor(u[0]));
+}
+
+// The FP32 form of the mixed CFL is the same quantity with fewer divisions:
+// p = (E - |m|^2 / (2 rho)) (gamma-1) for rho e_int (gamma-1), cs =
+// sqrt(gamma p / rho) for sqrt(gamma kB/amu T/mu). The sweeps' flux and
+// interface solve form p so too, from one reciprocal of rho: FP32 division is
+// a reciprocal and a multiply plus range handling, and the sweeps divide a lot
+// (256^3 mixed step 2.43 -> 2.20 ms, L1(rho) against FP64 a little lower).
+template <int D>
+__device__ __forceinline__ float sound_speed(const Gas<float>& G, const float* u) {
+  float s = 0.f;
+#pragma unroll
+  for (int a = 0; a < D; ++a) s = s + u[1 + a] * u[1 + a];
+  const float p = (u[D + 1] - 0.5f * s / u[0]) * G.gm1;
+  return sqrtf(G.g * p / u[0]);
 }
 
 // rhyme_ideal_gas_flux.f90:12-23 along axis AX
-template <int D, int AX, typename T>
-__device__ __forceinline__ void flux(const Gas<T>& G, const T* u, T* f) {
-  if (m_tiny(u[0])) {
+template <int D, int AX>
+__device__ __forceinline__ void flux(const Gas<double>& G, const double* u, double* f) {
+  if (f64_tiny(u[0])) {
 #pragma unroll
-    for (int c = 0; c < D + 2; ++c) f[c] = T(0);
+    for (int c = 0; c < D + 2; ++c) f[c] = 0.0;
     return;
   }
-  const Inv<T> i0 = m_inv(u[0]);
-  T p = pressure<D>(G, u, i0);
+  const Divisor i0 = divisor(u[0]);
+  const double p = pressure<D>(G, u, i0);
   f[0] = u[1 + AX];
 #pragma unroll
   for (int a = 0; a < D; ++a) f[1 + a] = m_div(u[1 + a] * f[0], i0);
@@ -195,10 +171,11 @@ __device__ __forceinline__ void flux(const Gas<T>& G, const T* u, T* f) {
 }
 
 // rhyme_ideal_gas_primitive_vars_to_conserved.f90:9-11
-template <int D, typename T>
-__device__ __forceinline__ void prim_vars_to_cons(const Gas<T>& G, T rho, const T* v, T p, T* u) {
+template <int D>
+__device__ __forceinline__ void prim_vars_to_cons(const Gas<double>& G, double rho, const double* v, double p,
+                                                  double* u) {
   u[0] = rho;
-  T s = T(0);
+  double s = 0.0;
 #pragma unroll
   for (int a = 0; a < D; ++a) {
     u[1 + a] = rho * v[a];
@@ -370,31 +347,38 @@ __device__ __forceinline__ void flux_difference_f32(const Gas<float>& G, const f
 }
 
 // rhyme_muscl_hancock_half_step_extrapolation.f90:15-21; hdtdx = (.5*dt)/dx
-template <int D, int AX, typename T>
-__device__ __forceinline__ void half_step(const Gas<T>& G, const T* u, const T* delta, T hdtdx,
-                                          T* l, T* r) {
-  T fl[D + 2], fr[D + 2];
+template <int D, int AX>
+__device__ __forceinline__ void half_step(const Gas<double>& G, const double* u, const double* delta, double hdtdx,
+                                          double* l, double* r) {
+  double fl[D + 2], fr[D + 2];
 #pragma unroll
   for (int c = 0; c < D + 2; ++c) {
     l[c] = u[c] - m_half(delta[c]);
     r[c] = u[c] + m_half(delta[c]);
   }
-  if constexpr (sizeof(T) == sizeof(float)) {
-    flux_difference_f32<D, AX>(G, l, r, fl);
-#pragma unroll
-    for (int c = 0; c < D + 2; ++c) {
-      l[c] = l[c] + hdtdx * fl[c];
-      r[c] = r[c] + hdtdx * fl[c];
-    }
-    return;
-  }
   flux<D, AX>(G, l, fl);
   flux<D, AX>(G, r, fr);
 #pragma unroll
   for (int c = 0; c < D + 2; ++c) {
-    T df = fl[c] - fr[c];
+    const double df = fl[c] - fr[c];
     l[c] = l[c] + hdtdx * df;
     r[c] = r[c] + hdtdx * df;
+  }
+}
+template <int D, int AX>
+__device__ __forceinline__ void half_step(const Gas<float>& G, const float* u, const float* delta, float hdtdx,
+                                          float* l, float* r) {
+  float df[D + 2];
+#pragma unroll
+  for (int c = 0; c < D + 2; ++c) {
+    l[c] = u[c] - 0.5f * delta[c];
+    r[c] = u[c] + 0.5f * delta[c];
+  }
+  flux_difference_f32<D, AX>(G, l, r, df);
+#pragma unroll
+  for (int c = 0; c < D + 2; ++c) {
+    l[c] = l[c] + hdtdx * df[c];
+    r[c] = r[c] + hdtdx * df[c];
   }
 }
 
@@ -416,7 +400,7 @@ __device__ __forceinline__ void face_states(const Gas<T>& G, int lim, T w, const
 // pass on the side each has picked (a selection of registers is a few
 // integer instructions, a pass of the rarefaction's two powers 57 FP64
 // ones). Divisors used more than once (a side's density, pressure and sound
-// speed) are kept with their reciprocal (Inv).
+// speed) are kept with their reciprocal (Divisor).
 
 // One side's loop-invariant terms of
 // rhyme_irs_nonlinear_wave_function.f90:15-23 (Ak, Bk, 2cs/gm1, 1/(rho cs)):
@@ -424,13 +408,13 @@ __device__ __forceinline__ void face_states(const Gas<T>& G, int lim, T w, const
 // operations, so computing them once gives the same values.
 struct WaveSide {
   double p, Ak, Bk, c2g, irc;
-  Inv<double> ip;
+  Divisor ip;
 };
 
 __device__ __forceinline__ WaveSide wave_side(const Gas<double>& G, double s_rho, double s_p, double s_cs) {
   WaveSide w;
   w.p = s_p;
-  w.ip = m_inv(s_p);
+  w.ip = divisor(s_p);
   w.Ak = m_div(2.0, G.gp1 * s_rho);
   w.Bk = m_div(G.gm1 * s_p, G.by_gp1);
   w.c2g = m_div(m_twice(s_cs), G.by_gm1);
@@ -449,7 +433,7 @@ __device__ __forceinline__ void nonlinear_waves(const Gas<double>& G, const Wave
     const bool l = pass == 0 && !l_shock;
     if (l || (!r_shock && (pass == 0 || !l_shock))) {
       double y, z;
-      const Inv<double> ip = l ? L.ip : R.ip;
+      const Divisor ip = l ? L.ip : R.ip;
       m_pow2(m_div(p, ip), G.gm1_2g, -G.gp1_2g, y, z);
       const double f = (l ? L.c2g : R.c2g) * (y - 1.0);
       const double fp = (l ? L.irc : R.irc) * z;
@@ -465,12 +449,12 @@ __device__ __forceinline__ void nonlinear_waves(const Gas<double>& G, const Wave
     if (l || (r_shock && (pass == 0 || l_shock))) {
       const double pk = l ? L.p : R.p;
       const double bp = (l ? L.Bk : R.Bk) + p;
-      const Inv<double> ibp = m_inv(bp);
+      const Divisor ibp = divisor(bp);
       const double dp = p - pk;
       const double factor = m_sqrt(m_div(l ? L.Ak : R.Ak, ibp));
       const double f = dp * factor;
       // (p - pk)/(2 bp): half of the quotient by bp
-      const double fp = factor * (1.0 - div_by_twice(dp, ibp.d));
+      const double fp = factor * (1.0 - div_by_twice(dp, ibp));
       l_f = l ? f : l_f;
       l_fp = l ? fp : l_fp;
       r_f = l ? r_f : f;
@@ -490,12 +474,12 @@ __device__ __forceinline__ double guess_p_star_adaptive(const Gas<double>& G, do
   const double p_max = fmax_ref(l_p, r_p);
   // q_max = p_max/p_min <= q_user = 2: for normal numbers the quotient
   // rounds to at most 2 exactly where p_max <= 2 p_min
-  const bool near2 = (!m_tiny(p_min) && f64_hi(p_min) < 0x7fe00000u && f64_hi(p_max) < 0x7ff00000u)
+  const bool near2 = (!f64_tiny(p_min) && f64_hi(p_min) < 0x7fe00000u && f64_hi(p_max) < 0x7ff00000u)
                          ? !m_gt(p_max, m_twice(p_min))
                          : p_max / p_min <= 2.0;
   if (near2 && (m_gt(ppv, p_min) && m_gt(p_max, ppv))) return ppv;  // PVRS
   if (m_gt(p_min, ppv)) {                                          // two-rarefaction
-    const Inv<double> icl = m_inv(l_cs), icr = m_inv(r_cs);
+    const Divisor icl = divisor(l_cs), icr = divisor(r_cs);
     const double pq = m_pow(m_div(l_p, r_p), G.gm1_2g);
     const double um = m_div(m_div(pq * vl, icl) + m_div(vr, icr) + G.two_gm1 * (pq - 1.0),
                             m_div(pq, icl) + m_div(1.0, icr));
@@ -531,7 +515,7 @@ static __device__ __noinline__ double guess_p_star(const Gas<double>& G, int k, 
   } else {  // arithmetic mean
     p = 0.5 * (l_p + r_p);
   }
-  return fmax_ref(p, Limits<double>::tiny());
+  return fmax_ref(p, DBL_MIN);
 }
 
 // rhyme_irs_exec.f90:19-44 with lazily evaluated guesses. l_f / r_f are the
@@ -555,7 +539,7 @@ __device__ __forceinline__ double irs_exec(const Gas<double>& G, double tol, int
       p_star = p_prev - m_div(l_f + r_f + du, l_fp + r_fp);
       if (m_neg(p_star)) break;
       if (f64_nan(p_prev)) break;
-      if (m_gt(tol, m_div(m_twice(m_abs(p_star - p_prev)), p_star + p_prev))) break;
+      if (m_gt(tol, m_div(m_twice(fabs(p_star - p_prev)), p_star + p_prev))) break;
       p_prev = p_star;
     }
     if (f64_above(p_star, 0.0)) break;
@@ -568,7 +552,7 @@ __device__ __forceinline__ double irs_exec(const Gas<double>& G, double tol, int
 template <int D>
 struct Side {
   double rho, v[D], p, cs;
-  Inv<double> ip;
+  Divisor ip;
 };
 
 // rhyme_riemann_problem_w_kfan.f90:14-31
@@ -630,7 +614,7 @@ __device__ __forceinline__ void rp_sample_side(const Gas<double>& G, const Side<
 // The velocities across AX of the side that is sampled, from its conserved
 // state q.
 template <int D, int AX>
-__device__ __forceinline__ void side_transverse(Side<D>& S, const double* q, const Inv<double>& i0) {
+__device__ __forceinline__ void side_transverse(Side<D>& S, const double* q, const Divisor& i0) {
 #pragma unroll
   for (int a = 0; a < D; ++a)
     if (a != AX) S.v[a] = m_div(q[1 + a], i0);
@@ -659,7 +643,7 @@ __device__ __forceinline__ void rp_solve(const Gas<double>& G, const Rp<double>&
   const bool vacuum_right = r_below && L.rho > e_rho;
   const bool vacuum_left = l_below && R.rho > e_rho;
   const bool vacuum_both = l_below && r_below;
-  const double tiny = Limits<double>::tiny();
+  const double tiny = DBL_MIN;
 
   if (vacuum_right) {
 #pragma unroll
@@ -683,7 +667,7 @@ __device__ __forceinline__ void rp_solve(const Gas<double>& G, const Rp<double>&
     vacuum_state<D>(G, rp, u);
   } else {
     // velocities across AX: only for the side sampled (side_transverse)
-    const Inv<double> il = m_inv(l[0]), ir = m_inv(r[0]);
+    const Divisor il = divisor(l[0]), ir = divisor(r[0]);
     L.v[AX] = m_div(l[1 + AX], il);
     L.p = fmax_ref(pressure<D>(G, l, il), rp.vac_p);
     L.cs = fmax_ref(sound_speed<D>(G, l, il), tiny);
@@ -854,11 +838,11 @@ __device__ __forceinline__ void rp_flux_f32(const Gas<float>& G, const Rp<float>
   // Halley's iteration from it: the wave functions' second derivatives cost
   // a few products and make it of third order, with the error of a step
   // below 0.12 of its cube (relative to p; 0.097 for gamma = 5/3, 0.103 for
-  // 7/5, 0.116 for 1.1). A step below rp.last therefore leaves an error below
+  // 7/5, 0.116 for 1.1). A step below rp.tol therefore leaves an error below
   // the FP32 rounding, and the wave functions at the new p follow from their
   // Taylor series: no evaluation is spent on confirming the root. The step is
   // taken as p has it, rounded, so that under a tolerance below FP32's
-  // resolution (rp.last is then the tolerance) only a p that stays counts.
+  // resolution (rp.tol is then the tolerance) only a p that stays counts.
   const float Akl = G.two_gp1 * il, Bkl = __fmul_rn(G.gm1_gp1, pl), c2gl = G.two_gm1 * cl;
   const float Akr = G.two_gp1 * ir, Bkr = __fmul_rn(G.gm1_gp1, pr), c2gr = G.two_gm1 * cr;
   float fl = 0.f, fr = 0.f;
@@ -874,7 +858,7 @@ __device__ __forceinline__ void rp_flux_f32(const Gas<float>& G, const Rp<float>
     const float before = p;
     p = p + d;
     if (!(p > 0.f)) break;
-    if (fabsf(p - before) < rp.last * p) {
+    if (fabsf(p - before) < rp.tol * p) {
       fl = __fmaf_rn(d, __fmaf_rn(0.5f * d, fppl, fpl), fl);
       fr = __fmaf_rn(d, __fmaf_rn(0.5f * d, fppr, fpr), fr);
       conv = true;

@@ -264,9 +264,9 @@ void rgpu::make_dev_params(const rhyme_gpu_params* p, DevParams* d) {
   G.gm1_half = 0.5 * G.gm1;
   G.half_gm1 = G.gm1 / 2.0;
   G.g_kb_amu = g * p->kb_amu;
-  G.by_gm1 = m_inv(G.gm1);
-  G.by_gp1 = m_inv(G.gp1);
-  G.by_kb_amu = m_inv(G.kb_amu);
+  G.by_gm1 = divisor(G.gm1);
+  G.by_gp1 = divisor(G.gp1);
+  G.by_kb_amu = divisor(G.kb_amu);
   d->rp.vac_rho = p->vacuum_density;
   d->rp.vac_p = p->vacuum_pressure;
   d->rp.vac_rho_next = std::nextafter(p->vacuum_density, 1.0);
@@ -303,15 +303,11 @@ void make_mixed_params(const DevParams& d, MixedParams* m) {
   F.gm1_half = (float)G.gm1_half;
   F.half_gm1 = (float)G.half_gm1;
   F.g_kb_amu = (float)G.g_kb_amu;
-  F.by_gm1 = m_inv(F.gm1);
-  F.by_gp1 = m_inv(F.gp1);
-  F.by_kb_amu = m_inv(F.kb_amu);
   F.gm1_lo = (float)(G.gm1 - (double)F.gm1);
   F.g_gm1 = (float)(G.g / G.gm1);
   m->rp.vac_rho = (float)d.rp.vac_rho;
   m->rp.vac_p = (float)d.rp.vac_p;
   m->rp.vac_rho_next = std::nextafter((float)d.rp.vac_rho, 1.0f);
-  m->rp.tol = (float)d.rp.tol;
   m->rp.n_iter = d.rp.n_iter;
   // third order: a last step of cbrt(tol) leaves less than tol, one of 5e-3
   // less than 1.6e-8. Only steps below tol count where few iterations are
@@ -324,7 +320,7 @@ void make_mixed_params(const DevParams& d, MixedParams* m) {
   // / 8.4; 1.5e-7 8.2 % / 7.9, cbrt 1.5 % / 8.4, steps to tol 4.6 % / 7.8;
   // 1e-10 28.8 % / 5.2, cbrt 1.5 % / 8.4, steps to tol 26.0 % / 5.3).
   const bool to_tol = d.rp.n_iter < 8 || d.rp.tol < 0x1p-22;
-  m->rp.last = (float)(to_tol ? d.rp.tol : std::min(5e-3, std::cbrt(d.rp.tol)));
+  m->rp.tol = (float)(to_tol ? d.rp.tol : std::min(5e-3, std::cbrt(d.rp.tol)));
   m->G64 = d.G;
   m->rp64 = d.rp;
   m->ndim = d.ndim;
