@@ -249,12 +249,13 @@ RGPU_HD double f64_scale(double x) {
   return hw_mul(x, K < 0 ? 1.0 / (double)(1 << (K < 0 ? -K : 0)) : (double)(1 << (K > 0 ? K : 0)));
 }
 
-// a / (2 b), b given with its reciprocal: the significand of 2 b is b's, unless
+// a / (2 b), b given with its reciprocal: the significand of 2 b is b's unless
 // b is subnormal (its leading zeros differ from 2 b's).
 RGPU_HD double div_by_twice(double a, const Divisor& d) {
-  const double b2 = f64_scale<1>(d.b);
-  if (f64_tiny(d.b)) return div_rn(a, b2);
-  return div_with(a, b2, d.R);
+  const uint32_t h = f64_hi(d.b) & 0x7fffffffu;
+  if (h - 0x00100000u < 0x7fe00000u - 0x00100000u)  // b and 2 b normal
+    return div_with(a, f64_from(f64_bits(d.b) + (1ull << 52)), d.R);
+  return div_rn(a, hw_mul(2.0, d.b));
 }
 
 }  // namespace rgpu
