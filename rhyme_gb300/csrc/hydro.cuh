@@ -97,6 +97,7 @@ template <typename T>
 struct Rp {
   T vac_rho, vac_p, vac_rho_next;  // w_vacuum(rho), w_vacuum(p), nearest(w_vac_rho, +1)
   T tol;  // FP64: the tolerance; FP32: the relative size of a step that ends rp_flux_f32's iteration
+  T settle;  // FP32: what the rounded p may move in that step
   int n_iter;
 };
 
@@ -840,9 +841,9 @@ __device__ __forceinline__ void rp_flux_f32(const Gas<float>& G, const Rp<float>
   // below 0.12 of its cube (relative to p; 0.097 for gamma = 5/3, 0.103 for
   // 7/5, 0.116 for 1.1). A step below rp.tol therefore leaves an error below
   // the FP32 rounding, and the wave functions at the new p follow from their
-  // Taylor series: no evaluation is spent on confirming the root. The step is
-  // taken as p has it, rounded, so that under a tolerance below FP32's
-  // resolution (rp.tol is then the tolerance) only a p that stays counts.
+  // Taylor series: no evaluation is spent on confirming the root. Under a
+  // tolerance below FP32's resolution rp.settle asks besides that p, rounded,
+  // has moved by less than the tolerance (1 otherwise: always so).
   const float Akl = G.two_gp1 * il, Bkl = __fmul_rn(G.gm1_gp1, pl), c2gl = G.two_gm1 * cl;
   const float Akr = G.two_gp1 * ir, Bkr = __fmul_rn(G.gm1_gp1, pr), c2gr = G.two_gm1 * cr;
   float fl = 0.f, fr = 0.f;
@@ -858,7 +859,8 @@ __device__ __forceinline__ void rp_flux_f32(const Gas<float>& G, const Rp<float>
     const float before = p;
     p = p + d;
     if (!(p > 0.f)) break;
-    if (fabsf(p - before) < rp.tol * p) {
+    if (fabsf(d) < rp.tol * p) {
+      if (!(fabsf(p - before) < rp.settle * p)) continue;
       fl = __fmaf_rn(d, __fmaf_rn(0.5f * d, fppl, fpl), fl);
       fr = __fmaf_rn(d, __fmaf_rn(0.5f * d, fppr, fpr), fr);
       conv = true;

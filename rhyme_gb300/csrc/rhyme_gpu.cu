@@ -319,8 +319,11 @@ void make_mixed_params(const DevParams& d, MixedParams* m) {
   // build, redone / error in 1e-9: tol 2.5e-7 Newton 6.5 % / 8.4, cbrt 1.5 %
   // / 8.4; 1.5e-7 8.2 % / 7.9, cbrt 1.5 % / 8.4, steps to tol 4.6 % / 7.8;
   // 1e-10 28.8 % / 5.2, cbrt 1.5 % / 8.4, steps to tol 26.0 % / 5.3).
-  const bool to_tol = d.rp.n_iter < 8 || d.rp.tol < 0x1p-22;
-  m->rp.tol = (float)(to_tol ? d.rp.tol : std::min(5e-3, std::cbrt(d.rp.tol)));
+  // A p that settles may still be half a unit of its last place, 2^-24, off its step.
+  const bool fine = d.rp.tol < 0x1p-22;
+  const double last = (fine || d.rp.n_iter < 8) ? d.rp.tol : std::min(5e-3, std::cbrt(d.rp.tol));
+  m->rp.tol = (float)(fine ? last + 0x1p-24 : last);
+  m->rp.settle = fine ? (float)last : 1.f;
   m->G64 = d.G;
   m->rp64 = d.rp;
   m->ndim = d.ndim;
