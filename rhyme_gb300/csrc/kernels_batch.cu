@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// 8 CTAs per SM: 512 boxes of 8..64^3, a step 83.2 ms at 8, 85.7 at 12, 84.8
+// 8 CTAs per SM: 512 boxes of 8..64^3, a step 55.9 ms at 8, 57.3 at 12, 56.8
 // at 16 (its items are too uneven for the gain that one 3-D box has there).
 template <int D>
 __global__ void __launch_bounds__(128, 8)

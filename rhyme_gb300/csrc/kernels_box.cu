@@ -6,20 +6,19 @@
 //                         loops 1-3 (and the cpu-intensive update order)
 //
 // The plain path on GB300 is bound by the FP64 pipe (a warp instruction per
-// SM sub-partition every 64 cycles), not by HBM: one interface solve costs
-// about a thousand FP64 warp instructions against 80 bytes of state per 3-D
-// cell. So K3 does every face state and every interface solve exactly once
-// with full parallelism (one thread per cell-axis, then one thread per
-// interface-axis) and keeps face states and fluxes in device scratch (that
-// traffic is well under 1% of HBM bandwidth at the FP64 rate), and whatever
-// integers compute exactly is kept off the pipe (fp64_int.h: divisions,
-// roots, comparisons, powers of two; libm_pow_int.h: most of a power), with
-// the limiters' spared divisions and the two sides' waves run in common
-// passes, and the solve calls those functions instead of inlining them (its
-// warps waited for instructions half of the time): a step of the 2-D 256^2
-// slab 348 -> 114 us, of 3-D 128^3 17.5 -> 5.5 ms, of 16 boxes of 8..64^3 5.5
-// -> 2.0 ms. A third of the FP64 warp instructions of the flux pass that are
-// left run with part of their lanes.
+// SM sub-partition every 64 cycles) and by instruction issue, not by HBM. So K3
+// does every face state and every interface solve exactly once with full
+// parallelism (one thread per cell-axis, then one thread per interface-axis)
+// and keeps face states and fluxes in device scratch, and whatever integers
+// compute exactly is kept off the pipe (fp64_int.h: divisions, roots,
+// comparisons, powers of two; libm_pow_int.h: most of a power), with the
+// limiters' spared divisions and the two sides' waves run in common passes,
+// and the solve calls those functions instead of inlining them: about a
+// thousand FP64 warp instructions of an interface solve became 180 (of 7300 in
+// all; 3-D 128^3 spheres), a step of the 2-D 256^2 slab took 348 us and takes
+// 114, of 3-D 128^3 17.5 and 5.5 ms, of 16 boxes of 8..64^3 5.5 and 2.0 ms. What
+// is left of the flux pass waits for instructions first (18 of 33 warp cycles
+// per issue) and keeps the FP64 pipe 68 % busy.
 //
 // This file is compiled with --fmad=false so the double arithmetic performs
 // the same IEEE operations, in the same order, as the reference.

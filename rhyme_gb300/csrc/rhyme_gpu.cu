@@ -798,20 +798,21 @@ StepScratch scratch_of(Box* b, bool trace) {
 //
 // A box-size class is (NDIM, axis, ceil(log2) of the box's extent along the
 // axis and along the pencil axis, each clamped to [3, 10], and which shapes the
-// sweep would march with). The first box of
-// a class met by a context has its sweep along that axis timed with every
-// candidate tile shape on its current state (one warm-up launch on a few
-// rows, the march once on the whole box since S is an argument of its only
-// kernel: without it the first S was charged 8 to 11 us for loading it; then one launch of a box of a million cells or more, whose sweep
-// takes 50 us or longer, or three of a smaller box, between CUDA events on
-// the context's stream; one synchronisation per axis); the fastest shape is
-// kept for the class. Where the x and y sweeps run as one kernel, only z is
-// tuned; the sweeps of a batch, tiles whatever the box's size, have classes of
-// their own where another solve would march. A sweep only reads U^n and its FP32 mirror, so the timing launches
+// sweep would march with). The first box of a class met by a context has its
+// sweep along that axis timed with every candidate tile shape on its current
+// state, between CUDA events on the context's stream and with one
+// synchronisation per axis: one warm-up launch on a few rows (the march once on
+// the whole box, since S is an argument of its only kernel: without it the
+// first S was charged 8 to 11 us for loading it), then one launch of a box of a
+// million cells or more, whose sweep takes 50 us or longer, or three of a
+// smaller box. The fastest shape is kept for the class. Where the x and y
+// sweeps run as one kernel, only z is tuned; the sweeps of a batch, tiles
+// whatever the box's size, have classes of their own where another solve would
+// march. A sweep only reads U^n and its FP32 mirror, so the timing launches
 // leave the state alone (they write the next-step buffers, which the step
 // itself overwrites). With four full launches and a synchronisation each on
-// every axis the first run of a 3-D 256^3 box took 26 ms longer than the
-// next, of 64^3 2.1 ms; so it takes 7 and 1.0.
+// every axis the first run of a 3-D 256^3 box took 26 ms longer than the next,
+// of 64^3 2.1 ms; so it takes 8 and 1.0.
 
 int size_bucket(int n) {
   int b = 3;
